@@ -302,6 +302,42 @@ __device__ __forceinline__ double widen_f32(float f) {
   }
   return __hiloint2double((int)hi, (int)lo);
 }
+// A running sum as an unevaluated pair of floats, hi + lo (Knuth's TwoSum with
+// the rounding errors collected in lo).  The terms below enter exactly, so the
+// sum carries about 2^-45 relative error: FP64 sums of FP32 data without an
+// FP64 instruction per term (GB300 issues those at 1/64 of the FP32 rate).
+struct PairSum {
+  float hi, lo;
+};
+__device__ __forceinline__ void pair_add(PairSum& s, float x) {
+  const float t = __fadd_rn(s.hi, x);
+  const float b = __fadd_rn(t, -s.hi);
+  const float e = __fadd_rn(__fadd_rn(s.hi, -__fadd_rn(t, -b)), __fadd_rn(x, -b));
+  s.hi = t;
+  s.lo = __fadd_rn(s.lo, e);
+}
+// s += x^2, exact.
+__device__ __forceinline__ void pair_add_square(PairSum& s, float x) {
+  const float p = __fmul_rn(x, x);
+  pair_add(s, p);
+  s.lo = __fadd_rn(s.lo, __fmaf_rn(x, x, -p));
+}
+// s += (wh + wl) * (xh + xl), with the product of the leading parts exact.
+__device__ __forceinline__ void pair_add_prod(PairSum& s, float wh, float wl, float xh, float xl) {
+  const float p = __fmul_rn(wh, xh);
+  const float e = __fmaf_rn(wh, xh, -p);
+  pair_add(s, p);
+  s.lo = __fadd_rn(s.lo, __fmaf_rn(wh, xl, __fmaf_rn(wl, xh, e)));
+}
+__device__ __forceinline__ void pair_merge(PairSum& s, float hi, float lo) {
+  pair_add(s, hi);
+  s.lo = __fadd_rn(s.lo, lo);
+}
+__device__ __forceinline__ double pair_value(const PairSum& s) {
+  // an infinity or NaN stands in hi; lo is then meaningless
+  return isfinite(s.hi) ? widen_f32(s.hi) + widen_f32(s.lo) : widen_f32(s.hi);
+}
+
 __device__ __forceinline__ double to_f64(float f) { return widen_f32(f); }
 __device__ __forceinline__ double to_f64(double f) { return f; }
 
