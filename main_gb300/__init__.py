@@ -363,9 +363,9 @@ class Engine:
         prm = MpcmdConcParams(x_slab, y_slab, z_slab, half_width, x_width, y_width, z_width)
         L = (self.cfg["lx"], self.cfg["ly"], self.cfg["lz"])
         nx, ny, nz = (int(L[c] / w) if w > 0 else 0 for c, w in enumerate((x_width, y_width, z_width)))
-        out = {"totals": np.zeros(4), "c1d_a": np.zeros(nx), "c1d_b": np.zeros(nx),
-               "xy_a": np.zeros(nx * ny), "xy_b": np.zeros(nx * ny), "xz_a": np.zeros(nx * nz),
-               "xz_b": np.zeros(nx * nz), "yz_a": np.zeros(ny * nz), "yz_b": np.zeros(ny * nz)}
+        size = {"totals": 4, "c1d_a": nx, "c1d_b": nx, "xy_a": nx * ny, "xy_b": nx * ny, "xz_a": nx * nz,
+                "xz_b": nx * nz, "yz_a": ny * nz, "yz_b": ny * nz}
+        out = {k: np.empty(m) for k, m in size.items()}   # (the call fills every element)
         keys = ("totals", "c1d_a", "c1d_b", "xy_a", "xy_b", "xz_a", "xz_b", "yz_a", "yz_b")
         self._c(lib().mpcmd_concentration(self.h, C.byref(prm), *[_ptr(out[k], C.c_double) for k in keys]),
                 "concentration")

@@ -252,6 +252,7 @@ struct Engine : EngineBase {
     for (cudaEvent_t e : marks) if (e) cudaEventDestroy(e);
     if (cst) cudaStreamSynchronize(cst);
     for (cudaEvent_t e : xev) if (e) cudaEventDestroy(e);
+    conc_release();
     for (void* p : allocs) cudaFree(p);
     if (cst) cudaStreamDestroy(cst);
     if (st) cudaStreamDestroy(st);
@@ -1158,9 +1159,44 @@ struct Engine : EngineBase {
     return dev_status_to_api(h.status);
   }
 
+  // Scratch of concentration(): the totals, a block of densities and the
+  // counts in one device buffer, and a page-locked copy of the totals and the
+  // block, kept between calls while small (an allocation and a free per call
+  // cost 170 us, as much as the counting).
+  void* conc_dev = nullptr;
+  void* conc_host = nullptr;
+  size_t conc_cap = 0, conc_host_cap = 0;
+  static constexpr size_t CONC_KEEP = (size_t)64 << 20;
+  static constexpr int64_t CONC_BLOCK = (int64_t)1 << 21;   // densities per copy
+
+  void conc_release() {
+    if (conc_dev) { cudaFree(conc_dev); bytes -= (int64_t)conc_cap; }
+    if (conc_host) cudaFreeHost(conc_host);
+    conc_dev = conc_host = nullptr;
+    conc_cap = conc_host_cap = 0;
+  }
+  int conc_reserve(size_t dev_bytes, size_t host_bytes) {
+    if (dev_bytes <= conc_cap && host_bytes <= conc_host_cap) return MPCMD_OK;
+    conc_release();
+    if (cudaMalloc(&conc_dev, dev_bytes) == cudaSuccess) {
+      conc_cap = dev_bytes;
+      bytes += (int64_t)dev_bytes;
+      if (cudaHostAlloc(&conc_host, host_bytes, cudaHostAllocDefault) == cudaSuccess) {
+        conc_host_cap = host_bytes;
+        return MPCMD_OK;
+      }
+      conc_host = nullptr;
+    } else {
+      conc_dev = nullptr;
+    }
+    cudaGetLastError();
+    conc_release();
+    return MPCMD_ERR_CUDA;
+  }
+
   // output_mod.f95:482-575 on the device: a flush of the shell, one counting
-  // pass over the particles, normalisation on the host.  Allocates its count
-  // arrays per call (an output-cadence call, not part of the step).
+  // pass over the particles, the row sums of the 1D field and the
+  // normalisation.
   int concentration(const mpcmd_conc_params* p, double* totals, double* const* fields) override {
     if (!(p->x_width > 0 && p->y_width > 0 && p->z_width > 0 && p->half_width >= 0)) return MPCMD_ERR_CONFIG;
     const double L[3] = {(double)cfg.lx, (double)cfg.ly, (double)cfg.lz};
@@ -1170,53 +1206,79 @@ struct Engine : EngineBase {
     if (advanced) return MPCMD_ERR_STATE;
     flush_shell();
     const int64_t sz[8] = {nx, nx, nx * ny, nx * ny, nx * nz, nx * nz, ny * nz, ny * nz};
-    int64_t off[9];
-    off[0] = 0;
-    for (int q = 0; q < 8; ++q) off[q + 1] = off[q] + sz[q];
-    uint32_t* cnt = nullptr;
-    unsigned long long* tot = nullptr;
-    if (cudaMalloc(&cnt, sizeof(uint32_t) * (size_t)off[8]) != cudaSuccess) return MPCMD_ERR_CUDA;
-    if (cudaMalloc(&tot, 2 * sizeof(unsigned long long)) != cudaSuccess) { cudaFree(cnt); return MPCMD_ERR_CUDA; }
-    int r = MPCMD_OK;
-    std::vector<uint32_t> h((size_t)off[8]);
-    unsigned long long ht[2] = {0, 0};
-    ConcArgs c;
-    c.xs = p->x_slab; c.ys = p->y_slab; c.zs = p->z_slab; c.hw = p->half_width;
-    c.xw = p->x_width; c.yw = p->y_width; c.zw = p->z_width;
-    c.nx = (int)nx; c.ny = (int)ny; c.nz = (int)nz;
-    uint32_t* ptrs[8];
-    for (int q = 0; q < 8; ++q) ptrs[q] = cnt + off[q];
-    c.c1a = ptrs[0]; c.c1b = ptrs[1]; c.xya = ptrs[2]; c.xyb = ptrs[3];
-    c.xza = ptrs[4]; c.xzb = ptrs[5]; c.yza = ptrs[6]; c.yzb = ptrs[7];
-    c.tot = tot;
-    if (cudaMemsetAsync(cnt, 0, sizeof(uint32_t) * (size_t)off[8], st) != cudaSuccess ||
-        cudaMemsetAsync(tot, 0, 2 * sizeof(unsigned long long), st) != cudaSuccess) {
-      r = MPCMD_ERR_CUDA;
-    } else {
-      Launch<T>::concentration(d, kp, time_count, (int)(last_rebuild - last_full), c, st);
-      if (cudaMemcpyAsync(h.data(), cnt, sizeof(uint32_t) * h.size(), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-          cudaMemcpyAsync(ht, tot, sizeof(ht), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-          cudaStreamSynchronize(st) != cudaSuccess)
-        r = MPCMD_ERR_CUDA;
-    }
-    cudaFree(cnt);
-    cudaFree(tot);
-    if (r) return r;
     const double hw2 = 2.0 * p->half_width;
-    const double vol = (double)(int64_t)(L[0] * L[1] * L[2]);
     const double v[8] = {p->x_width * L[1] * hw2, p->x_width * L[1] * hw2,
                          p->x_width * p->y_width * hw2, p->x_width * p->y_width * hw2,
                          p->x_width * p->z_width * hw2, p->x_width * p->z_width * hw2,
                          p->y_width * p->z_width * hw2, p->y_width * p->z_width * hw2};
-    if (totals) {
-      totals[0] = (double)ht[0]; totals[1] = (double)ht[1];
-      totals[2] = (double)ht[0] / vol; totals[3] = (double)ht[1] / vol;
+    ConcScale sc;
+    sc.off[0] = 0;
+    for (int q = 0; q < 8; ++q) { sc.off[q + 1] = sc.off[q] + sz[q]; sc.vol[q] = v[q]; }
+    const int64_t m = sc.off[8];
+    const int64_t blk = std::min(m, CONC_BLOCK);
+    const size_t head = sizeof(double) * (size_t)(2 + blk);   // two totals and a block of densities
+    int r = conc_reserve(head + sizeof(uint32_t) * (size_t)m, head);
+    if (r) return r;
+    unsigned long long* tot = static_cast<unsigned long long*>(conc_dev);
+    double* out = static_cast<double*>(conc_dev) + 2;
+    uint32_t* cnt = reinterpret_cast<uint32_t*>(out + blk);
+    ConcArgs c;
+    const double slab[3] = {p->x_slab, p->y_slab, p->z_slab}, w[3] = {p->x_width, p->y_width, p->z_width};
+    for (int q = 0; q < 3; ++q) {
+      c.lo[q] = slab[q] - p->half_width;
+      c.hi[q] = slab[q] + p->half_width;
+      c.w[q] = w[q];
+      c.iwf[q] = (float)(1.0 / w[q]);
+      // the cells whose particles (in [k, k + 1]) can be in the slab; none for
+      // a slab that is not a number
+      c.clo[q] = 0; c.chi[q] = -1;
+      if (c.lo[q] <= c.hi[q]) {
+        c.clo[q] = (int)std::floor(std::min(std::max(c.lo[q], -4.0), 4096.0)) - 1;
+        c.chi[q] = (int)std::floor(std::min(std::max(c.hi[q], -4.0), 4096.0)) + 1;
+      }
     }
-    for (int q = 0; q < 8; ++q) {
-      if (!fields[q]) continue;
-      for (int64_t j = 0; j < sz[q]; ++j) fields[q][j] = (double)h[(size_t)(off[q] + j)] / v[q];
+    c.nx = (int)nx; c.ny = (int)ny; c.nz = (int)nz;
+    for (int s = 0; s < 2; ++s) {
+      c.c1[s] = cnt + sc.off[s]; c.xy[s] = cnt + sc.off[2 + s];
+      c.xz[s] = cnt + sc.off[4 + s]; c.yz[s] = cnt + sc.off[6 + s];
     }
-    return check_device_status();
+    c.tot = tot;
+    Counters h;
+    if (cudaMemsetAsync(tot, 0, 2 * sizeof(unsigned long long), st) != cudaSuccess ||
+        cudaMemsetAsync(cnt, 0, sizeof(uint32_t) * (size_t)m, st) != cudaSuccess)
+      r = MPCMD_ERR_CUDA;
+    else
+      Launch<T>::concentration(d, kp, time_count, (int)(last_rebuild - last_full), c, st);
+    const double* ho = static_cast<const double*>(conc_host) + 2;
+    for (int64_t a = 0; a < m && r == MPCMD_OK; a += blk) {
+      const int64_t b = std::min(a + blk, m);
+      Launch<T>::conc_scale(cnt, out, sc, a, b, st);
+      if (cudaMemcpyAsync(conc_host, conc_dev, sizeof(double) * (size_t)(2 + b - a), cudaMemcpyDeviceToHost, st) !=
+          cudaSuccess) {
+        r = MPCMD_ERR_CUDA;
+        break;
+      }
+      if ((r = read_counters(h))) break;   // (waits for the copy)
+      for (int q = 0; q < 8; ++q) {
+        const int64_t lo = std::max(a, sc.off[q]), hi = std::min(b, sc.off[q + 1]);
+        if (fields[q] && lo < hi)
+          std::memcpy(fields[q] + (lo - sc.off[q]), ho + (lo - a), sizeof(double) * (size_t)(hi - lo));
+      }
+    }
+    if (r == MPCMD_OK) {
+      const unsigned long long* ht = static_cast<const unsigned long long*>(conc_host);
+      const double vol = (double)(int64_t)(L[0] * L[1] * L[2]);
+      if (totals) {
+        totals[0] = (double)ht[0]; totals[1] = (double)ht[1];
+        totals[2] = (double)ht[0] / vol; totals[3] = (double)ht[1] / vol;
+      }
+      n_inside = h.n_inside;
+      r = dev_status_to_api(h.status);
+    } else {
+      cudaStreamSynchronize(st);
+    }
+    if (conc_cap > CONC_KEEP) conc_release();
+    return r;
   }
 
   // Dimer axes from the FP64 sphere state: output_mod.f95:826-846 (d / Dcn)

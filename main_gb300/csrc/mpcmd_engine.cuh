@@ -83,13 +83,21 @@ struct Particles {
   uint8_t* flag;
 };
 
-// Concentration-field counting (mpcmd_concentration): slab centres, half
-// thickness, bin widths, bin counts per axis and the device count arrays.
+// Concentration-field counting (mpcmd_concentration): per axis the slab's
+// bounds, the cells that can reach into it, and the bin width; bin counts per
+// axis and the device count arrays per species.
 struct ConcArgs {
-  double xs, ys, zs, hw, xw, yw, zw;
+  double lo[3], hi[3], w[3];
+  float iwf[3];
+  int clo[3], chi[3];
   int nx, ny, nz;
-  uint32_t *c1a, *c1b, *xya, *xyb, *xza, *xzb, *yza, *yzb;
+  uint32_t *c1[2], *xy[2], *xz[2], *yz[2];
   unsigned long long* tot;   // [2] particles of species 0 and 1
+};
+// Ends of the eight count arrays in one buffer and the volume of their bins.
+struct ConcScale {
+  int64_t off[9];
+  double vol[8];
 };
 
 template <typename T>
@@ -212,8 +220,12 @@ struct Launch {
   // caller provides lid2 and lpos and swaps nothing
   static void resort(Dev<T>& d, const KParams<T>& kp, int tc, int tc_full, cudaStream_t st);
   static void observables(const Dev<T>& d, const KParams<T>& kp, const double* mass, int grid, cudaStream_t st);
+  // counts into c's arrays (zeroed by the caller)
   static void concentration(const Dev<T>& d, const KParams<T>& kp, int tc, int tc_defer, const ConcArgs& c,
                             cudaStream_t st);
+  // out[0, hi - lo) = the counts [lo, hi) over their bins' volumes
+  static void conc_scale(const uint32_t* cnt, double* out, const ConcScale& s, int64_t lo, int64_t hi,
+                         cudaStream_t st);
   // resident blocks per SM of the persistent kernels (rebuild, force, rotate)
   static void occupancy(int* blocks);
   static void init_solvent(const Dev<T>& d, const KParams<T>& kp, const int64_t* bounds, double kT,
