@@ -278,7 +278,7 @@ int mpcmd_profile_read(mpcmd_ctx* ctx, double* ms, int64_t* count, int n);
  * +1 (Rodrigues form) or -1 (projection form), contract seed.  Launches on
  * `stream` (a cudaStream_t; NULL = legacy default stream) and does not wait.
  * Allocates nothing: its only scratch is a static device array of
- * MPCMD_STATIC_MAX_CELLS x 4 doubles (16 MiB) that every GPU loading this
+ * MPCMD_STATIC_MAX_CELLS x 12 doubles (48 MiB) that every GPU loading this
  * library holds until exit; boxes with more shifted cells (lx*ly*lz, or
  * lx*ly*(lz+1) with walls) return MPCMD_ERR_CONFIG.  The first call on a
  * device resolves the array's address (cudaGetSymbolAddress) and must come
