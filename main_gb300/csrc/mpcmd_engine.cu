@@ -205,6 +205,9 @@ struct Engine : EngineBase {
   // index -> slot table
   int64_t resort_every = 0, resorts = 0;
   uint32_t *lid_a = nullptr, *lid_b = nullptr, *lpos_buf = nullptr;
+  // particles per shifted cell of the last mpc_rotation stage call (k_cells
+  // clears the sums they come from), for mpcmd_get_cell_rotation
+  uint32_t* cnt_snap = nullptr;
   double w3 = 1.0;
   unsigned int n_inside = 0;
 
@@ -253,6 +256,7 @@ struct Engine : EngineBase {
     if (cst) cudaStreamSynchronize(cst);
     for (cudaEvent_t e : xev) if (e) cudaEventDestroy(e);
     conc_release();
+    if (hctr) cudaFreeHost(hctr);
     for (void* p : allocs) cudaFree(p);
     if (cst) cudaStreamDestroy(cst);
     if (st) cudaStreamDestroy(st);
@@ -325,6 +329,7 @@ struct Engine : EngineBase {
     CK(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
     CK(cudaStreamCreateWithFlags(&cst, cudaStreamNonBlocking));
     for (cudaEvent_t& e : xev) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    CK(cudaHostAlloc(reinterpret_cast<void**>(&hctr), sizeof(Counters), cudaHostAllocDefault));
 
     const int64_t n = c.n_solvent, ns = 2 * (int64_t)c.n_dimers;
     kp.lx = c.lx; kp.ly = c.ly; kp.lz = c.lz;
@@ -429,6 +434,7 @@ struct Engine : EngineBase {
     if (c.owner_tags) { r |= alloc(d.owner, n); r |= alloc(d.owner2, n); }
     if (c.catalysis == MPCMD_CAT_ON_EXIT) { r |= alloc(d.inc, n); r |= alloc(d.inc2, n); }
     r |= alloc(lid_a, n); r |= alloc(lid_b, n); r |= alloc(lpos_buf, n);
+    r |= alloc(cnt_snap, kp.ncell_shift);
     if (r) return MPCMD_ERR_ALLOC;
     d.lid = d.lid2 = d.lpos = nullptr;
     // a re-sort every ten collision periods (the cell order of a diffusing
@@ -439,6 +445,7 @@ struct Engine : EngineBase {
     CK(cudaMemsetAsync(d.dcnt, 0, 4 * (size_t)kp.ncell, st));
     CK(cudaMemsetAsync(d.dfirst, 0xFF, 16 * (size_t)kp.ncell, st));
     CK(cudaMemsetAsync(d.affected, 0, (size_t)kp.ncell, st));
+    CK(cudaMemsetAsync(cnt_snap, 0, 4 * (size_t)kp.ncell_shift, st));
     CK(cudaMemsetAsync(d.ctr, 0, sizeof(Counters), st));
     CK(cudaMemsetAsync(d.facc, 0, sizeof(double) * 4 * std::max<int64_t>(ns, 1), st));
     CK(cudaMemsetAsync(d.fmot, 0, sizeof(double) * 4 * std::max<int64_t>(ns, 1), st));
@@ -533,10 +540,14 @@ struct Engine : EngineBase {
     return MPCMD_OK;
   }
 
+  // (through page-locked memory: a copy to pageable memory is staged by the
+  // driver and costs several times as much)
+  Counters* hctr = nullptr;
   int read_counters(Counters& h) {
     CK(cudaGetLastError());   // launch-configuration errors of the kernels queued so far
-    CK(cudaMemcpyAsync(&h, d.ctr, sizeof(Counters), cudaMemcpyDeviceToHost, st));
+    CK(cudaMemcpyAsync(hctr, d.ctr, sizeof(Counters), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
+    h = *hctr;
     return MPCMD_OK;
   }
 
@@ -971,7 +982,6 @@ struct Engine : EngineBase {
     StepArgs a = args(cstep);
     Launch<T>::accumulate_main(d, kp, a, 2, st);
     if (kp.exclusion == MPCMD_EXCL_CELLS) Launch<T>::affected(d, kp, a, st);
-    CK(cudaStreamSynchronize(st));
     return check_device_status();
   }
 
@@ -981,27 +991,10 @@ struct Engine : EngineBase {
     draw_shift(cstep);
     StepArgs a = args(cstep);
     Launch<T>::accumulate_main(d, kp, a, 1, st);
-    snapshot_counts();
+    Launch<T>::cell_counts(d, kp, cnt_snap, st);
     Launch<T>::cells(d, kp, a, 1, st);
     Launch<T>::rotate_main(d, kp, a, st);
-    CK(cudaStreamSynchronize(st));
     return check_device_status();
-  }
-
-  std::vector<int32_t> counts_snapshot;
-  void snapshot_counts() {
-    counts_snapshot.assign((size_t)kp.ncell_shift, 0);
-    if (sizeof(T) == 4) {
-      std::vector<float> a((size_t)kp.ncell_shift * 4);
-      cudaMemcpyAsync(a.data(), d.acc, a.size() * 4, cudaMemcpyDeviceToHost, st);
-      cudaStreamSynchronize(st);
-      for (int64_t c = 0; c < kp.ncell_shift; ++c) counts_snapshot[(size_t)c] = (int32_t)a[(size_t)(4 * c)];
-    } else {
-      std::vector<double> a((size_t)kp.ncell_shift * 4);
-      cudaMemcpyAsync(a.data(), d.acc, a.size() * 8, cudaMemcpyDeviceToHost, st);
-      cudaStreamSynchronize(st);
-      for (int64_t c = 0; c < kp.ncell_shift; ++c) counts_snapshot[(size_t)c] = (int32_t)a[(size_t)(4 * c)];
-    }
   }
 
   int reaction_stage() override {
@@ -1009,7 +1002,6 @@ struct Engine : EngineBase {
     flush_shell();
     StepArgs a = args(cstep);
     Launch<T>::cells(d, kp, a, 2, st);
-    CK(cudaStreamSynchronize(st));
     return check_device_status();
   }
 
@@ -1335,9 +1327,7 @@ struct Engine : EngineBase {
         if (cm) cm[3 * c + q] = (double)r[(size_t)(6 * c + q)];
         if (axis) axis[3 * c + q] = (double)r[(size_t)(6 * c + 3 + q)];
       }
-    if (count)
-      for (int64_t c = 0; c < kp.ncell_shift; ++c)
-        count[c] = (size_t)c < counts_snapshot.size() ? counts_snapshot[(size_t)c] : 0;
+    if (count) CK(cudaMemcpy(count, cnt_snap, 4 * (size_t)kp.ncell_shift, cudaMemcpyDeviceToHost));
     return MPCMD_OK;
   }
 

@@ -205,6 +205,8 @@ struct Launch {
   static void affected(const Dev<T>& d, const KParams<T>& kp, const StepArgs& a, cudaStream_t st);
   static void accumulate_main(const Dev<T>& d, const KParams<T>& kp, const StepArgs& a, int what, cudaStream_t st);
   static void cells(const Dev<T>& d, const KParams<T>& kp, const StepArgs& a, int what, cudaStream_t st);
+  // particles per shifted cell from the collision sums (before cells clears them)
+  static void cell_counts(const Dev<T>& d, const KParams<T>& kp, uint32_t* out, cudaStream_t st);
   static void rotate_main(const Dev<T>& d, const KParams<T>& kp, const StepArgs& a, cudaStream_t st);
   // lower bounds of the distance of each bin to the spheres' list radius (for the watch list)
   static void gap_field(const Dev<T>& d, const KParams<T>& kp, int horizon, cudaStream_t st);

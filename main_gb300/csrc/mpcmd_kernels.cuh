@@ -2564,6 +2564,19 @@ void Launch<T>::cells(const Dev<T>& d, const KParams<T>& kp, const StepArgs& a, 
   LAUNCH_COUNT();
 }
 
+template <typename T>
+__global__ void k_cell_counts(Dev<T> d, KParams<T> kp, uint32_t* out) {
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < kp.ncell_shift; c += stride)
+    out[c] = (uint32_t)reinterpret_cast<const T*>(d.acc)[4 * c];   // (float4 or four doubles per cell)
+}
+
+template <typename T>
+void Launch<T>::cell_counts(const Dev<T>& d, const KParams<T>& kp, uint32_t* out, cudaStream_t st) {
+  k_cell_counts<T><<<1024, TPB, 0, st>>>(d, kp, out);
+  LAUNCH_COUNT();
+}
+
 // Watch list support: for every coarse bin, a lower bound on the distance
 // from any point of the bin to the list radius (r_c 2^(1/6) + skin) of any
 // sphere, clamped at 0 (float bits, so atomicMin orders them).  Bins farther
