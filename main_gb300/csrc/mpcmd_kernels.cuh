@@ -1647,338 +1647,12 @@ __device__ __forceinline__ double dmin_image(double d, double L) {
   return d;
 }
 
-// One thread per dimer (evolve_mod.f95:605-636 totals, :679-724 RATTLE
-// velocities, :320-417 RATTLE positions of the next step), on register copies
-// of the dimer state.  mode bit 0: finish the force step (totals +
-// RATTLE-v); bit 1: RATTLE-x.  The FP64 parity build performs the reference's
-// operation sequence; the FP32 production build multiplies by precomputed
-// reciprocals and wraps the positions once after the RATTLE-x iterations (the
-// constraint uses minimum-image separations, so the in-loop wraps of the
-// reference only change the stored result, which the final wrap reproduces).
-template <typename T>
-__global__ void k_dimer(Dev<T> d, KParams<T> kp, StepArgs a, int mode, double w3, int rattle_max) {
-  if (d.ctr->abort_step) return;
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= kp.nd) return;
-  constexpr bool fast = sizeof(T) == 4;
-  const double dt = kp.dtd, Mc = kp.mc, Mn = kp.mn, Dcn = kp.dcn;
-  const double hIMc = kp.hIMc, hIMn = kp.hIMn, IIM = kp.IIM;
-  const double iMc = kp.iMc, iMn = kp.iMn, iD2 = kp.iD2, iMcdt = kp.iMcdt, iMndt = kp.iMndt;
-  const bool per = kp.geometry == 1;
-  const int nwrap = per ? 3 : 2;
-  const int s1 = 2 * k, s2 = 2 * k + 1;
-  double X1[3], X2[3], V1[3], V2[3], F1[3], F2[3], Q1[3], Q2[3];
-  for (int c = 0; c < 3; ++c) {
-    X1[c] = d.dpos[3 * s1 + c]; X2[c] = d.dpos[3 * s2 + c];
-    V1[c] = d.dvel[3 * s1 + c]; V2[c] = d.dvel[3 * s2 + c];
-    F1[c] = d.dfrc[3 * s1 + c]; F2[c] = d.dfrc[3 * s2 + c];
-    Q1[c] = d.dq[3 * s1 + c]; Q2[c] = d.dq[3 * s2 + c];
-  }
-  unsigned long long iters = 0;
-  if (mode & 1) {
-    double pot = 0.;
-    for (int i = 0; i < 2; ++i) {
-      const int s = 2 * k + i;
-      double* F = i == 0 ? F1 : F2;
-      double fw = 0., pw = 0.;
-      if (!per) lj_wall(kp, (i == 0 ? X1 : X2)[2], i == 0 ? kp.rwc : kp.rwn, w3, fw, pw);
-      F[0] = d.facc[4 * s + 0] + d.fmot[4 * s + 0];
-      F[1] = d.facc[4 * s + 1] + d.fmot[4 * s + 1];
-      F[2] = d.facc[4 * s + 2] + d.fmot[4 * s + 2] + fw;
-      pot += d.facc[4 * s + 3] + d.fmot[4 * s + 3] + pw;
-      d.facc[4 * s + 0] = 0.; d.facc[4 * s + 1] = 0.; d.facc[4 * s + 2] = 0.; d.facc[4 * s + 3] = 0.;
-    }
-    d.dpot[k] = pot;
-    for (int c = 0; c < 3; ++c) { V1[c] = Q1[c] + hIMc * F1[c]; V2[c] = Q2[c] + hIMn * F2[c]; }
-    int acc = 0;
-    for (;;) {
-      double dV[3], dd[3];
-      for (int c = 0; c < 3; ++c) { dV[c] = V1[c] - V2[c]; dd[c] = X1[c] - X2[c]; }
-      dd[0] = dmin_image(dd[0], kp.Ld[0]);
-      dd[1] = dmin_image(dd[1], kp.Ld[1]);
-      if (per) dd[2] = dmin_image(dd[2], kp.Ld[2]);
-      double Con2diff = 2.0 * (dV[0] * dd[0] + dV[1] * dd[1] + dV[2] * dd[2]);
-      if (fabs(Con2diff) < 1.e-8) break;
-      if (acc == rattle_max) { atomicOr(&d.ctr->status, DEV_ERR_RATTLE); break; }
-      if (fast) {
-        const double O2 = -(0.5 * (IIM * Con2diff) * iD2);
-        for (int c = 0; c < 3; ++c) {
-          V1[c] = V1[c] + O2 * dd[c] * iMc;
-          V2[c] = V2[c] - O2 * dd[c] * iMn;
-        }
-      } else {
-        double O = -(0.25 * (IIM * Con2diff) / (Dcn * Dcn));
-        for (int c = 0; c < 3; ++c) {
-          V1[c] = V1[c] + 2.0 * O * dd[c] / Mc;
-          V2[c] = V2[c] - 2.0 * O * dd[c] / Mn;
-        }
-      }
-      acc++;
-    }
-    iters += acc;
-    for (int c = 0; c < 3; ++c) {
-      d.dvel[3 * s1 + c] = V1[c]; d.dvel[3 * s2 + c] = V2[c];
-      d.dfrc[3 * s1 + c] = F1[c]; d.dfrc[3 * s2 + c] = F2[c];
-    }
-  }
-  if (mode & 2) {
-    double pr1[3], pr2[3], dP[3];
-    for (int c = 0; c < 3; ++c) { pr1[c] = X1[c]; pr2[c] = X2[c]; dP[c] = X1[c] - X2[c]; }
-    dP[0] = dmin_image(dP[0], kp.Ld[0]);
-    dP[1] = dmin_image(dP[1], kp.Ld[1]);
-    if (per) dP[2] = dmin_image(dP[2], kp.Ld[2]);
-    for (int c = 0; c < 3; ++c) { Q1[c] = V1[c] + hIMc * F1[c]; Q2[c] = V2[c] + hIMn * F2[c]; }
-    for (int c = 0; c < 3; ++c) { X1[c] = X1[c] + dt * Q1[c]; X2[c] = X2[c] + dt * Q2[c]; }
-    if (!fast) {
-      for (int c = 0; c < nwrap; ++c) {
-        X1[c] = X1[c] - kp.Ld[c] * floor(X1[c] / kp.Ld[c]);
-        X2[c] = X2[c] - kp.Ld[c] * floor(X2[c] / kp.Ld[c]);
-      }
-    }
-    int acc = 0;
-    for (;;) {
-      double dd[3];
-      for (int c = 0; c < 3; ++c) dd[c] = X1[c] - X2[c];
-      dd[0] = dmin_image(dd[0], kp.Ld[0]);
-      dd[1] = dmin_image(dd[1], kp.Ld[1]);
-      if (per) dd[2] = dmin_image(dd[2], kp.Ld[2]);
-      double Con1diff = (dd[0] * dd[0] + dd[1] * dd[1] + dd[2] * dd[2]) - Dcn * Dcn;
-      if (fabs(Con1diff) < 1.e-6) break;
-      if (acc == rattle_max) { atomicOr(&d.ctr->status, DEV_ERR_RATTLE); break; }
-      const double den = dd[0] * dP[0] + dd[1] * dP[1] + dd[2] * dP[2];
-      double G;
-      if (fast) {
-        // the iteration converges to the tolerance whatever the last bits of
-        // G are: a float reciprocal refined twice replaces the division
-        double r = (double)__frcp_rn((float)den);
-        r = r * (2.0 - den * r);
-        r = r * (2.0 - den * r);
-        G = -(0.25 * Con1diff * IIM) * r;
-      } else {
-        G = -(0.25 * Con1diff * IIM / den);
-      }
-      if (fast) {
-        const double G2 = 2.0 * G;
-        for (int c = 0; c < 3; ++c) {
-          X1[c] = pr1[c] + Q1[c] * dt + G2 * dP[c] * iMc;
-          X2[c] = pr2[c] + Q2[c] * dt - G2 * dP[c] * iMn;
-          Q1[c] = Q1[c] + G2 * dP[c] * iMcdt;
-          Q2[c] = Q2[c] - G2 * dP[c] * iMndt;
-        }
-      } else {
-        for (int c = 0; c < 3; ++c) {
-          X1[c] = pr1[c] + Q1[c] * dt + 2.0 * G * dP[c] / Mc;
-          X2[c] = pr2[c] + Q2[c] * dt - 2.0 * G * dP[c] / Mn;
-        }
-        for (int c = 0; c < nwrap; ++c) {
-          X1[c] = X1[c] - kp.Ld[c] * floor(X1[c] / kp.Ld[c]);
-          X2[c] = X2[c] - kp.Ld[c] * floor(X2[c] / kp.Ld[c]);
-        }
-        for (int c = 0; c < 3; ++c) {
-          Q1[c] = Q1[c] + 2.0 * G * dP[c] / (Mc * dt);
-          Q2[c] = Q2[c] - 2.0 * G * dP[c] / (Mn * dt);
-        }
-      }
-      acc++;
-    }
-    if (fast) {
-      // one step moves a sphere far less than a box edge: a single shift
-      for (int c = 0; c < nwrap; ++c) {
-        const double L = kp.Ld[c];
-        if (X1[c] >= L) X1[c] -= L; else if (X1[c] < 0.0) X1[c] += L;
-        if (X2[c] >= L) X2[c] -= L; else if (X2[c] < 0.0) X2[c] += L;
-        if (!(X1[c] >= 0.0 && X1[c] < L)) X1[c] = X1[c] - L * floor(X1[c] / L);
-        if (!(X2[c] >= 0.0 && X2[c] < L)) X2[c] = X2[c] - L * floor(X2[c] / L);
-      }
-    }
-    iters += acc;
-    for (int c = 0; c < 3; ++c) {
-      d.dpos[3 * s1 + c] = X1[c]; d.dpos[3 * s2 + c] = X2[c];
-      d.dq[3 * s1 + c] = Q1[c]; d.dq[3 * s2 + c] = Q2[c];
-    }
-    for (int i = 0; i < 2; ++i) {
-      const double* X = i == 0 ? X1 : X2;
-      const double fx = floor(X[0]), fy = floor(X[1]), fz = floor(X[2]);
-      SphereRel<T> r;
-      r.cx = (int)fx; r.cy = (int)fy; r.cz = (int)fz;
-      r.ox = (T)(X[0] - fx); r.oy = (T)(X[1] - fy); r.oz = (T)(X[2] - fz);
-      d.srel[2 * k + i] = r;
-    }
-  }
-  if (iters) atomicAdd(&d.ctr->rattle_iters, iters);
-}
-
 // rotational_code/2d_array/forces_mod.f95:177-201: harmonic z tether.
 __device__ __forceinline__ void harmonic_tether(const double zdim, const double zdimeq, const double k_harm,
                                                 double& f, double& pot) {
   const double zdiff = zdim - zdimeq;
   f = -1. * k_harm * zdiff;
   pot = 0.5 * k_harm * (zdiff * zdiff);
-}
-
-// One thread per anchored rotor (rotational_code/2d_array/evolve_mod.f95:
-// 533-557 totals with the tether, :596-650 RATTLE velocities, :283-391
-// RATTLE positions), in the reference's FP64 operation sequence in both
-// builds (a handful of rotors per run).  Besides the bond, the positions hold
-// the midpoint 0.5 (X1 + X2) (wrapped into the box in x and y) at the anchor,
-// with the correction H = -4 IIM (midpoint - anchor) applied as H / (2 M) to
-// each sphere, and the velocities hold the midpoint velocity at zero.
-template <typename T>
-__global__ void k_rotor(Dev<T> d, KParams<T> kp, StepArgs a, int mode, int rattle_max) {
-  if (d.ctr->abort_step) return;
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= kp.nd) return;
-  const double dt = kp.dtd, Mc = kp.mc, Mn = kp.mn, Dcn = kp.dcn;
-  const double hIMc = kp.hIMc, hIMn = kp.hIMn, IIM = kp.IIM;
-  // the FP32 build multiplies by precomputed reciprocals where the reference
-  // divides (FP64 divisions dominate the iteration chain on this part); the
-  // FP64 parity build keeps the reference's operation sequence
-  constexpr bool fast = sizeof(T) == 4;
-  const double iMc = kp.iMc, iMn = kp.iMn, iD2 = kp.iD2, iMcdt = kp.iMcdt, iMndt = kp.iMndt;
-  const bool per = kp.geometry == 1;
-  const int nwrap = per ? 3 : 2;
-  const int s1 = 2 * k, s2 = 2 * k + 1;
-  double X1[3], X2[3], V1[3], V2[3], F1[3], F2[3], Q1[3], Q2[3], A[3];
-  for (int c = 0; c < 3; ++c) {
-    X1[c] = d.dpos[3 * s1 + c]; X2[c] = d.dpos[3 * s2 + c];
-    V1[c] = d.dvel[3 * s1 + c]; V2[c] = d.dvel[3 * s2 + c];
-    F1[c] = d.dfrc[3 * s1 + c]; F2[c] = d.dfrc[3 * s2 + c];
-    Q1[c] = d.dq[3 * s1 + c]; Q2[c] = d.dq[3 * s2 + c];
-    A[c] = d.anchor[3 * k + c];
-  }
-  unsigned long long iters = 0;
-  if (mode & 1) {
-    double pot = 0.;
-    for (int i = 0; i < 2; ++i) {
-      const int s = 2 * k + i;
-      double* F = i == 0 ? F1 : F2;
-      double fw = 0., pw = 0.;
-      harmonic_tether((i == 0 ? X1 : X2)[2], kp.tether_z, kp.tether_k, fw, pw);
-      F[0] = d.facc[4 * s + 0];
-      F[1] = d.facc[4 * s + 1];
-      F[2] = d.facc[4 * s + 2] + fw;
-      pot += d.facc[4 * s + 3] + pw;
-      d.facc[4 * s + 0] = 0.; d.facc[4 * s + 1] = 0.; d.facc[4 * s + 2] = 0.; d.facc[4 * s + 3] = 0.;
-    }
-    d.dpot[k] = pot;
-    for (int c = 0; c < 3; ++c) { V1[c] = Q1[c] + hIMc * F1[c]; V2[c] = Q2[c] + hIMn * F2[c]; }
-    int acc = 0;
-    for (;;) {
-      double dV[3], dd[3], Vm[3];
-      for (int c = 0; c < 3; ++c) { dV[c] = V1[c] - V2[c]; dd[c] = X1[c] - X2[c]; }
-      dd[0] = dmin_image(dd[0], kp.Ld[0]);
-      dd[1] = dmin_image(dd[1], kp.Ld[1]);
-      if (per) dd[2] = dmin_image(dd[2], kp.Ld[2]);
-      const double Con2diff = dV[0] * dd[0] + dV[1] * dd[1] + dV[2] * dd[2];
-      for (int c = 0; c < 3; ++c) Vm[c] = 0.5 * (V1[c] + V2[c]);
-      if (fabs(Con2diff) < 1.e-8 && fabs(Vm[0]) < 1.e-8 && fabs(Vm[1]) < 1.e-8 && fabs(Vm[2]) < 1.e-8) break;
-      if (acc == rattle_max) { atomicOr(&d.ctr->status, DEV_ERR_RATTLE); break; }
-      if (fast) {
-        const double O = -(0.25 * (IIM * Con2diff) * iD2);
-        for (int c = 0; c < 3; ++c) {
-          const double hP = -(2.0 * Vm[c] * IIM);
-          V1[c] = V1[c] + (O * dd[c] + hP) * iMc;
-          V2[c] = V2[c] + (hP - O * dd[c]) * iMn;
-        }
-      } else {
-        const double O = -(0.25 * (IIM * Con2diff) / (Dcn * Dcn));
-        for (int c = 0; c < 3; ++c) {
-          const double P = -(4.0 * Vm[c] * IIM);
-          V1[c] = V1[c] + O * dd[c] / Mc + 0.5 * P / Mc;
-          V2[c] = V2[c] - O * dd[c] / Mn + 0.5 * P / Mn;
-        }
-      }
-      acc++;
-    }
-    iters += acc;
-    for (int c = 0; c < 3; ++c) {
-      d.dvel[3 * s1 + c] = V1[c]; d.dvel[3 * s2 + c] = V2[c];
-      d.dfrc[3 * s1 + c] = F1[c]; d.dfrc[3 * s2 + c] = F2[c];
-    }
-  }
-  if (mode & 2) {
-    double pr1[3], pr2[3], dP[3];
-    for (int c = 0; c < 3; ++c) { pr1[c] = X1[c]; pr2[c] = X2[c]; dP[c] = X1[c] - X2[c]; }
-    dP[0] = dmin_image(dP[0], kp.Ld[0]);
-    dP[1] = dmin_image(dP[1], kp.Ld[1]);
-    if (per) dP[2] = dmin_image(dP[2], kp.Ld[2]);
-    for (int c = 0; c < 3; ++c) { Q1[c] = V1[c] + hIMc * F1[c]; Q2[c] = V2[c] + hIMn * F2[c]; }
-    for (int c = 0; c < 3; ++c) { X1[c] = X1[c] + dt * Q1[c]; X2[c] = X2[c] + dt * Q2[c]; }
-    for (int c = 0; c < nwrap; ++c) {
-      X1[c] = X1[c] - kp.Ld[c] * floor(X1[c] / kp.Ld[c]);
-      X2[c] = X2[c] - kp.Ld[c] * floor(X2[c] / kp.Ld[c]);
-    }
-    int acc = 0;
-    for (;;) {
-      double dd[3], D[3];
-      for (int c = 0; c < 3; ++c) dd[c] = X1[c] - X2[c];
-      dd[0] = dmin_image(dd[0], kp.Ld[0]);
-      dd[1] = dmin_image(dd[1], kp.Ld[1]);
-      if (per) dd[2] = dmin_image(dd[2], kp.Ld[2]);
-      for (int c = 0; c < 3; ++c) {
-        double m = 0.5 * (X1[c] + X2[c]);
-        if (c < 2) {
-          if (m >= kp.Ld[c]) m = m - kp.Ld[c];
-          else if (m < 0.) m = m + kp.Ld[c];
-        }
-        D[c] = m - A[c];
-      }
-      const double Con1diff = (dd[0] * dd[0] + dd[1] * dd[1] + dd[2] * dd[2]) - Dcn * Dcn;
-      if (fabs(Con1diff) < 1.e-6 && fabs(D[0]) < 1.e-6 && fabs(D[1]) < 1.e-6 && fabs(D[2]) < 1.e-6) break;
-      if (acc == rattle_max) { atomicOr(&d.ctr->status, DEV_ERR_RATTLE); break; }
-      const double den = dd[0] * dP[0] + dd[1] * dP[1] + dd[2] * dP[2];
-      if (fast) {
-        // a float reciprocal refined twice replaces the division (the
-        // iteration converges to the tolerance whatever G's last bits are)
-        double r = (double)__frcp_rn((float)den);
-        r = r * (2.0 - den * r);
-        r = r * (2.0 - den * r);
-        const double G = -(0.25 * Con1diff * IIM) * r;
-        for (int c = 0; c < 3; ++c) {
-          const double hH = -(2.0 * IIM * D[c]);
-          const double u1 = G * dP[c] + hH, u2 = hH - G * dP[c];
-          X1[c] = pr1[c] + Q1[c] * dt + u1 * iMc;
-          X2[c] = pr2[c] + Q2[c] * dt + u2 * iMn;
-          const double L = kp.Ld[c];
-          if (X1[c] >= L) X1[c] -= L; else if (X1[c] < 0.0) X1[c] += L;
-          if (X2[c] >= L) X2[c] -= L; else if (X2[c] < 0.0) X2[c] += L;
-          Q1[c] = Q1[c] + u1 * iMcdt;
-          Q2[c] = Q2[c] + u2 * iMndt;
-        }
-      } else {
-        const double G = -(0.25 * Con1diff * IIM / den);
-        double H[3];
-        for (int c = 0; c < 3; ++c) H[c] = -(4.0 * IIM * D[c]);
-        for (int c = 0; c < 3; ++c) {
-          X1[c] = pr1[c] + Q1[c] * dt + G * dP[c] / Mc + 0.5 * H[c] / Mc;
-          X2[c] = pr2[c] + Q2[c] * dt - G * dP[c] / Mn + 0.5 * H[c] / Mn;
-        }
-        for (int c = 0; c < 3; ++c) {
-          X1[c] = X1[c] - kp.Ld[c] * floor(X1[c] / kp.Ld[c]);
-          X2[c] = X2[c] - kp.Ld[c] * floor(X2[c] / kp.Ld[c]);
-        }
-        for (int c = 0; c < 3; ++c) {
-          Q1[c] = Q1[c] + G * dP[c] / (Mc * dt) + 0.5 * H[c] / (Mc * dt);
-          Q2[c] = Q2[c] - G * dP[c] / (Mn * dt) + 0.5 * H[c] / (Mn * dt);
-        }
-      }
-      acc++;
-    }
-    iters += acc;
-    for (int c = 0; c < 3; ++c) {
-      d.dpos[3 * s1 + c] = X1[c]; d.dpos[3 * s2 + c] = X2[c];
-      d.dq[3 * s1 + c] = Q1[c]; d.dq[3 * s2 + c] = Q2[c];
-    }
-    for (int i = 0; i < 2; ++i) {
-      const double* X = i == 0 ? X1 : X2;
-      const double fx = floor(X[0]), fy = floor(X[1]), fz = floor(X[2]);
-      SphereRel<T> r;
-      r.cx = (int)fx; r.cy = (int)fy; r.cz = (int)fz;
-      r.ox = (T)(X[0] - fx); r.oy = (T)(X[1] - fy); r.oz = (T)(X[2] - fz);
-      d.srel[2 * k + i] = r;
-    }
-  }
-  if (iters) atomicAdd(&d.ctr->rattle_iters, iters);
 }
 
 // Sum over the four lanes of a dimer's group (mask: those lanes, which
@@ -1990,14 +1664,37 @@ __device__ __forceinline__ double group4_sum(unsigned mask, double v) {
   return v;
 }
 
-// The FP32 build's dimer step with the three Cartesian components of a dimer
-// on three lanes of a 4-lane group (the fourth holds zeros and the energy):
-// the same update as k_dimer's fast path (totals, RATTLE velocities, RATTLE
-// positions, single-shift wrap), with the constraint dot products summed
-// across the group.  On this part FP64 instructions are issued at a few lanes
-// per SM cycle, so the per-dimer chain of FP64 instructions, not the lane
-// count, sets the time; splitting the components shortens that chain about
-// threefold.  The FP64 parity build keeps k_dimer and the oracle's order.
+// a / b for a loop-invariant b with rb = 1 / b rounded to nearest: one
+// correction step of the quotient a * rb, which rounds as the division does
+// (Markstein, IBM J. Res. Dev. 34, 1990, theorem 2; b's mantissa not all ones).
+// Three FP64 instructions instead of the dozen of a division.
+__device__ __forceinline__ double div_const(double a, double b, double rb) {
+  const double q = a * rb;
+  return fma(fma(-q, b, a), rb, q);
+}
+
+// X - L floor(X / L); inside the box, where the floor is 0, without the division.
+__device__ __forceinline__ double wrap_box(double X, double L) {
+  return X >= 0.0 && X < L ? X : X - L * floor(X / L);
+}
+
+// The dimer step (evolve_mod.f95:605-636 totals, :679-724 RATTLE velocities,
+// :320-417 RATTLE positions of the next step) with the three Cartesian
+// components of a dimer on three lanes of a 4-lane group (the fourth holds
+// zeros and the energy), the constraint dot products summed across the group.
+// mode bit 0: finish the force step (totals + RATTLE-v); bit 1: RATTLE-x.
+// Bound by latency: FP64 instructions are issued at two lanes per SM cycle, so
+// the per-dimer chain of FP64 instructions, not the lane count, sets the time;
+// splitting the components shortens that chain about threefold.
+//
+// The FP64 parity build performs the reference's operation sequence on every
+// component (group4_sum adds the components in its order), divisions and
+// in-loop wraps included.  The FP32 build multiplies by precomputed
+// reciprocals and wraps the positions once after the RATTLE-x iterations (the
+// constraint uses minimum-image separations, so the in-loop wraps only change
+// the stored result, which the final wrap reproduces).  One thread per dimer
+// took 19.3 us in the FP64 build (one dimer, 30^3 box), four lanes 13.4 us, and
+// 7.2 us with the divisions by constants through div_const and wrap_box.
 template <typename T>
 __global__ void k_dimer_split(Dev<T> d, KParams<T> kp, StepArgs a, int mode, double w3, int rattle_max) {
   if (d.ctr->abort_step) return;
@@ -2007,7 +1704,8 @@ __global__ void k_dimer_split(Dev<T> d, KParams<T> kp, StepArgs a, int mode, dou
   const bool live = k < kp.nd;        // the whole 4-lane group agrees
   const int kk = live ? k : 0;
   const bool comp = c < 3;
-  const double dt = kp.dtd, Dcn = kp.dcn;
+  constexpr bool fast = sizeof(T) == 4;
+  const double dt = kp.dtd, Dcn = kp.dcn, Mc = kp.mc, Mn = kp.mn;
   const double hIMc = kp.hIMc, hIMn = kp.hIMn, IIM = kp.IIM;
   const double iMc = kp.iMc, iMn = kp.iMn, iD2 = kp.iD2, iMcdt = kp.iMcdt, iMndt = kp.iMndt;
   const bool per = kp.geometry == 1;
@@ -2052,9 +1750,15 @@ __global__ void k_dimer_split(Dev<T> d, KParams<T> kp, StepArgs a, int mode, dou
       const double Con2diff = 2.0 * group4_sum(gmask, (V1 - V2) * dd);
       if (!live || fabs(Con2diff) < 1.e-8) break;
       if (acc == rattle_max) { if (c == 0) atomicOr(&d.ctr->status, DEV_ERR_RATTLE); break; }
-      const double O2 = -(0.5 * (IIM * Con2diff) * iD2);
-      V1 = V1 + O2 * dd * iMc;
-      V2 = V2 - O2 * dd * iMn;
+      if constexpr (fast) {
+        const double O2 = -(0.5 * (IIM * Con2diff) * iD2);
+        V1 = V1 + O2 * dd * iMc;
+        V2 = V2 - O2 * dd * iMn;
+      } else {
+        const double O = -div_const(0.25 * (IIM * Con2diff), Dcn * Dcn, iD2);
+        V1 = V1 + div_const(2.0 * O * dd, Mc, iMc);
+        V2 = V2 - div_const(2.0 * O * dd, Mn, iMn);
+      }
       acc++;
     }
     iters += acc;
@@ -2070,6 +1774,7 @@ __global__ void k_dimer_split(Dev<T> d, KParams<T> kp, StepArgs a, int mode, dou
     if (!comp) dP = 0.;
     Q1 = V1 + hIMc * F1; Q2 = V2 + hIMn * F2;
     X1 = X1 + dt * Q1; X2 = X2 + dt * Q2;
+    if (!fast && wrapc) { X1 = wrap_box(X1, L); X2 = wrap_box(X2, L); }
     int acc = 0;
     for (;;) {
       double dd = X1 - X2;
@@ -2079,17 +1784,29 @@ __global__ void k_dimer_split(Dev<T> d, KParams<T> kp, StepArgs a, int mode, dou
       if (!live || fabs(Con1diff) < 1.e-6) break;
       if (acc == rattle_max) { if (c == 0) atomicOr(&d.ctr->status, DEV_ERR_RATTLE); break; }
       const double den = group4_sum(gmask, dd * dP);
-      double r = (double)__frcp_rn((float)den);
-      r = r * (2.0 - den * r);
-      r = r * (2.0 - den * r);
-      const double G2 = 2.0 * (-(0.25 * Con1diff * IIM) * r);
-      X1 = pr1 + Q1 * dt + G2 * dP * iMc;
-      X2 = pr2 + Q2 * dt - G2 * dP * iMn;
-      Q1 = Q1 + G2 * dP * iMcdt;
-      Q2 = Q2 - G2 * dP * iMndt;
+      if constexpr (fast) {
+        // the iteration converges to the tolerance whatever the last bits of
+        // G are: a float reciprocal refined twice replaces the division
+        double r = (double)__frcp_rn((float)den);
+        r = r * (2.0 - den * r);
+        r = r * (2.0 - den * r);
+        const double G2 = 2.0 * (-(0.25 * Con1diff * IIM) * r);
+        X1 = pr1 + Q1 * dt + G2 * dP * iMc;
+        X2 = pr2 + Q2 * dt - G2 * dP * iMn;
+        Q1 = Q1 + G2 * dP * iMcdt;
+        Q2 = Q2 - G2 * dP * iMndt;
+      } else {
+        const double G = -(0.25 * Con1diff * IIM / den);
+        X1 = pr1 + Q1 * dt + div_const(2.0 * G * dP, Mc, iMc);
+        X2 = pr2 + Q2 * dt - div_const(2.0 * G * dP, Mn, iMn);
+        if (wrapc) { X1 = wrap_box(X1, L); X2 = wrap_box(X2, L); }
+        Q1 = Q1 + div_const(2.0 * G * dP, Mc * dt, iMcdt);
+        Q2 = Q2 - div_const(2.0 * G * dP, Mn * dt, iMndt);
+      }
       acc++;
     }
-    if (wrapc && (c < 2 || per)) {
+    if (fast && wrapc) {
+      // one step moves a sphere far less than a box edge: a single shift
       if (X1 >= L) X1 -= L; else if (X1 < 0.0) X1 += L;
       if (X2 >= L) X2 -= L; else if (X2 < 0.0) X2 += L;
       if (!(X1 >= 0.0 && X1 < L)) X1 = X1 - L * floor(X1 / L);
@@ -2112,7 +1829,7 @@ __global__ void k_dimer_split(Dev<T> d, KParams<T> kp, StepArgs a, int mode, dou
 
 // Sphere force totals and dimer potentials of a restart (restart_mod.f95:
 // 505-528), one thread per dimer: the same sums as the first stage of
-// k_dimer / k_dimer_split / k_rotor (pair sums, motor-motor forces, the wall
+// k_dimer_split / k_rotor_split (pair sums, motor-motor forces, the wall
 // or the rotor tether), with no RATTLE.
 template <typename T>
 __global__ void k_sphere_totals(Dev<T> d, KParams<T> kp, double w3) {
@@ -2141,12 +1858,15 @@ void Launch<T>::sphere_totals(const Dev<T>& d, const KParams<T>& kp, double w3, 
   LAUNCH_COUNT();
 }
 
-// The FP32 build's rotor step (k_rotor's fast path) with the three Cartesian
-// components of a rotor on three lanes of a 4-lane group, the constraint dot
-// products summed across the group and the convergence tests taken over it;
-// the fourth lane holds zeros and the energy.  As for k_dimer_split, the
-// per-rotor chain of FP64 instructions sets the time, and the split shortens
-// it about threefold.
+// The step of an anchored rotor (rotational_code/2d_array/evolve_mod.f95:
+// 533-557 totals with the tether, :596-650 RATTLE velocities, :283-391 RATTLE
+// positions) on four lanes as k_dimer_split.  Besides the bond, the positions
+// hold the midpoint 0.5 (X1 + X2) (wrapped into the box in x and y) at the
+// anchor, with the correction H = -4 IIM (midpoint - anchor) applied as
+// H / (2 M) to each sphere, and the velocities hold the midpoint velocity at
+// zero; the convergence tests are taken over the group.  The FP64 build keeps
+// the reference's operation sequence per component, the FP32 build multiplies
+// by reciprocals.
 template <typename T>
 __global__ void k_rotor_split(Dev<T> d, KParams<T> kp, StepArgs a, int mode, int rattle_max) {
   if (d.ctr->abort_step) return;
@@ -2156,7 +1876,8 @@ __global__ void k_rotor_split(Dev<T> d, KParams<T> kp, StepArgs a, int mode, int
   const bool live = k < kp.nd;        // the whole 4-lane group agrees
   const int kk = live ? k : 0;
   const bool comp = c < 3;
-  const double dt = kp.dtd, Dcn = kp.dcn;
+  constexpr bool fast = sizeof(T) == 4;
+  const double dt = kp.dtd, Dcn = kp.dcn, Mc = kp.mc, Mn = kp.mn;
   const double hIMc = kp.hIMc, hIMn = kp.hIMn, IIM = kp.IIM;
   const double iMc = kp.iMc, iMn = kp.iMn, iD2 = kp.iD2, iMcdt = kp.iMcdt, iMndt = kp.iMndt;
   const bool per = kp.geometry == 1;
@@ -2204,10 +1925,17 @@ __global__ void k_rotor_split(Dev<T> d, KParams<T> kp, StepArgs a, int mode, int
       const bool vm_ok = __all_sync(gmask, !comp || fabs(Vm) < 1.e-8);
       if (!live || (fabs(Con2diff) < 1.e-8 && vm_ok)) break;
       if (acc == rattle_max) { if (c == 0) atomicOr(&d.ctr->status, DEV_ERR_RATTLE); break; }
-      const double O = -(0.25 * (IIM * Con2diff) * iD2);
-      const double hP = -(2.0 * Vm * IIM);
-      V1 = V1 + (O * dd + hP) * iMc;
-      V2 = V2 + (hP - O * dd) * iMn;
+      if constexpr (fast) {
+        const double O = -(0.25 * (IIM * Con2diff) * iD2);
+        const double hP = -(2.0 * Vm * IIM);
+        V1 = V1 + (O * dd + hP) * iMc;
+        V2 = V2 + (hP - O * dd) * iMn;
+      } else {
+        const double O = -div_const(0.25 * (IIM * Con2diff), Dcn * Dcn, iD2);
+        const double P = -(4.0 * Vm * IIM);
+        V1 = V1 + div_const(O * dd, Mc, iMc) + div_const(0.5 * P, Mc, iMc);
+        V2 = V2 - div_const(O * dd, Mn, iMn) + div_const(0.5 * P, Mn, iMn);
+      }
       acc++;
     }
     iters += acc;
@@ -2223,9 +1951,14 @@ __global__ void k_rotor_split(Dev<T> d, KParams<T> kp, StepArgs a, int mode, int
     if (!comp) dP = 0.;
     Q1 = V1 + hIMc * F1; Q2 = V2 + hIMn * F2;
     X1 = X1 + dt * Q1; X2 = X2 + dt * Q2;
-    if (comp && (c < 2 || per)) {
-      if (X1 >= L) X1 -= L; else if (X1 < 0.0) X1 += L;
-      if (X2 >= L) X2 -= L; else if (X2 < 0.0) X2 += L;
+    if (mi) {
+      if constexpr (fast) {
+        if (X1 >= L) X1 -= L; else if (X1 < 0.0) X1 += L;
+        if (X2 >= L) X2 -= L; else if (X2 < 0.0) X2 += L;
+      } else {
+        X1 = wrap_box(X1, L);
+        X2 = wrap_box(X2, L);
+      }
     }
     int acc = 0;
     for (;;) {
@@ -2243,20 +1976,30 @@ __global__ void k_rotor_split(Dev<T> d, KParams<T> kp, StepArgs a, int mode, int
       if (!live || (fabs(Con1diff) < 1.e-6 && d_ok)) break;
       if (acc == rattle_max) { if (c == 0) atomicOr(&d.ctr->status, DEV_ERR_RATTLE); break; }
       const double den = group4_sum(gmask, dd * dP);
-      double r = (double)__frcp_rn((float)den);
-      r = r * (2.0 - den * r);
-      r = r * (2.0 - den * r);
-      const double G = -(0.25 * Con1diff * IIM) * r;
-      const double hH = -(2.0 * IIM * D);
-      const double u1 = G * dP + hH, u2 = hH - G * dP;
-      X1 = pr1 + Q1 * dt + u1 * iMc;
-      X2 = pr2 + Q2 * dt + u2 * iMn;
-      if (comp) {   // every axis wraps inside the iteration (2d_array/evolve_mod.f95:365-369)
-        if (X1 >= L) X1 -= L; else if (X1 < 0.0) X1 += L;
-        if (X2 >= L) X2 -= L; else if (X2 < 0.0) X2 += L;
+      if constexpr (fast) {
+        double r = (double)__frcp_rn((float)den);
+        r = r * (2.0 - den * r);
+        r = r * (2.0 - den * r);
+        const double G = -(0.25 * Con1diff * IIM) * r;
+        const double hH = -(2.0 * IIM * D);
+        const double u1 = G * dP + hH, u2 = hH - G * dP;
+        X1 = pr1 + Q1 * dt + u1 * iMc;
+        X2 = pr2 + Q2 * dt + u2 * iMn;
+        if (comp) {   // every axis wraps inside the iteration (2d_array/evolve_mod.f95:365-369)
+          if (X1 >= L) X1 -= L; else if (X1 < 0.0) X1 += L;
+          if (X2 >= L) X2 -= L; else if (X2 < 0.0) X2 += L;
+        }
+        Q1 = Q1 + u1 * iMcdt;
+        Q2 = Q2 + u2 * iMndt;
+      } else {
+        const double G = -(0.25 * Con1diff * IIM / den);
+        const double H = -(4.0 * IIM * D);
+        X1 = pr1 + Q1 * dt + div_const(G * dP, Mc, iMc) + div_const(0.5 * H, Mc, iMc);
+        X2 = pr2 + Q2 * dt - div_const(G * dP, Mn, iMn) + div_const(0.5 * H, Mn, iMn);
+        if (comp) { X1 = wrap_box(X1, L); X2 = wrap_box(X2, L); }
+        Q1 = Q1 + div_const(G * dP, Mc * dt, iMcdt) + div_const(0.5 * H, Mc * dt, iMcdt);
+        Q2 = Q2 - div_const(G * dP, Mn * dt, iMndt) + div_const(0.5 * H, Mn * dt, iMndt);
       }
-      Q1 = Q1 + u1 * iMcdt;
-      Q2 = Q2 + u2 * iMndt;
       acc++;
     }
     iters += acc;
@@ -2278,18 +2021,10 @@ template <typename T>
 void Launch<T>::dimer(const Dev<T>& d, const KParams<T>& kp, const StepArgs& a, int mode, double w3,
                       int rattle_max, cudaStream_t st) {
   if (kp.nd == 0) return;
-  if (kp.rotor && sizeof(T) == 4) {
-    const int threads = 4 * kp.nd;
-    k_rotor_split<T><<<(threads + 31) / 32, 32, 0, st>>>(d, kp, a, mode, rattle_max);
-  } else if (kp.rotor) {
-    k_rotor<T><<<(kp.nd + 63) / 64, 64, 0, st>>>(d, kp, a, mode, rattle_max);
-  } else if (sizeof(T) == 4) {
-    // four lanes per dimer, one 32-lane block per eight dimers (spread over the SMs)
-    const int threads = 4 * kp.nd;
-    k_dimer_split<T><<<(threads + 31) / 32, 32, 0, st>>>(d, kp, a, mode, w3, rattle_max);
-  } else {
-    k_dimer<T><<<(kp.nd + 63) / 64, 64, 0, st>>>(d, kp, a, mode, w3, rattle_max);
-  }
+  // four lanes per dimer, one 32-lane block per eight dimers (spread over the SMs)
+  const int blocks = (4 * kp.nd + 31) / 32;
+  if (kp.rotor) k_rotor_split<T><<<blocks, 32, 0, st>>>(d, kp, a, mode, rattle_max);
+  else k_dimer_split<T><<<blocks, 32, 0, st>>>(d, kp, a, mode, w3, rattle_max);
   LAUNCH_COUNT();
 }
 
