@@ -163,6 +163,8 @@ struct StepArgs {
   int g_force;
   int g_rotate;
   int g_far;           // SMs x resident blocks of k_rebuild_far
+  int far_steps;       // steps of TPB particles in a tile of k_rebuild_far
+  int rot_steps;       // steps of TPB particles in a tile of k_rotate_main (even)
   int g_cells;         // SMs x resident blocks of k_cells (one wave)
   int g_shell;         // SMs x resident blocks of k_shell_advance (one wave)
   int watch_build;     // > 0 (the period in steps): rotate_main / rotate_shell build the watch list

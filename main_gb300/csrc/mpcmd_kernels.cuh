@@ -50,6 +50,21 @@ __device__ __forceinline__ void accum_dist(const Dev<T>& d, const KParams<T>& kp
   atomicMin(&d.dfirst[4 * (size_t)cid + sp], key);
 }
 
+// First item of this thread in a grid-stride loop over n items by `blocks`
+// blocks (stride blocks * TPB), 32 consecutive items per warp.  A list of at
+// most two warps per block is dealt warp by warp over the blocks instead of
+// block by block: the few warps of a small shell then run on as many SMs (a
+// warp's FP64 instruction takes its SM's FP64 pipe for 16 cycles, so eight warps
+// of one block take eight times as long as on eight SMs).  One dimer in 30^3
+// cells, FP64: 13.4 -> 10.2 us per MD step of k_force.  Longer lists keep
+// neighbours in a block: dealt out as well, those of 64 dimers cost a 128 x 128
+// x 16 box 3 % of its period.
+__device__ __forceinline__ int64_t wave_first(int64_t n, int blocks) {
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (n <= (int64_t)blocks * 64) return ((int64_t)w * blocks + blockIdx.x) * 32 + lane;
+  return (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+}
+
 // Main index of the particle in slot i (slot = index until an order-only
 // re-sort moves particles).
 template <typename T>
@@ -708,7 +723,7 @@ __global__ void __launch_bounds__(TPB, 4) k_rebuild(Dev<T> d, KParams<T> kp, Ste
   const T vs_bound = (a.horizon > 0 && !a.mpc) ? sphere_speed_bound<T>(d.ctr) : (T)0;
   if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&d.ctr->acc_rebuild, (unsigned long long)nloop);
   auto pidx = [&](int64_t k) -> int64_t { return listed ? (int64_t)d.watch[k] : k; };
-  const int64_t first = (int64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31) + lane;
+  const int64_t first = wave_first(nloop, (int)gridDim.x);
   uint8_t pf_f = 0;
   uint32_t pf_cell = 0, pf_lid = 0;   // (the main index only after a re-sort)
   T pf_ox = 0, pf_oy = 0, pf_oz = 0, pf_vx = 0, pf_vy = 0, pf_vz = 0;
@@ -722,7 +737,7 @@ __global__ void __launch_bounds__(TPB, 4) k_rebuild(Dev<T> d, KParams<T> kp, Ste
     pf_vx = d.p.vx[q]; pf_vy = d.p.vy[q]; pf_vz = d.p.vz[q];
     if (want_lid) pf_lid = d.lid[q];
   }
-  for (int64_t base = (int64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31); base < nloop; base += stride) {
+  for (int64_t base = first - lane; base < nloop; base += stride) {
     const int64_t k = base + lane;
     const int64_t i = k < nloop ? pidx(k) : kp.n;
     bool dist = false;
@@ -954,21 +969,21 @@ __global__ void __launch_bounds__(TPB, 4) k_rebuild_far(Dev<T> d, KParams<T> kp,
   __shared__ uint32_t wl_buf[(TPB / 32) * WL_CAP];
   uint32_t* wbuf = wl_buf + (threadIdx.x >> 5) * WL_CAP;
   unsigned wn = 0;
-  // Blocks take tiles of FAR_TILE consecutive particles in a grid stride,
+  // Blocks take tiles of consecutive particles (a.far_steps times TPB) in a grid stride,
   // the warps of a block interleaved in 32-particle steps inside a tile: the
   // GPU still sweeps the arrays front to back, and the near list a warp
   // stages holds particles of one tile at a time, so the shell built from it
   // keeps their spatial (cell) order.
   // (32-bit indices: particle counts are below 2^31, and an index plus one
   // tile stride stays below 2^32)
-  constexpr int FAR_STEPS = 8;    // 2048-particle tiles (4096 and 1024 measured slower at 256^3)
-  constexpr uint32_t FAR_TILE = (uint32_t)FAR_STEPS * TPB;
+  const int steps = a.far_steps;
+  const uint32_t far_tile = (uint32_t)steps * TPB;
   const uint32_t n32 = (uint32_t)kp.n;
-  const uint32_t tile_stride = gridDim.x * FAR_TILE;
-  uint32_t i = blockIdx.x * FAR_TILE + threadIdx.x;
+  const uint32_t tile_stride = gridDim.x * far_tile;
+  uint32_t i = blockIdx.x * far_tile + threadIdx.x;
   int step = 0;
   auto advance = [&](uint32_t j, int st) -> uint32_t {   // the index after j (at step st of its tile)
-    return st + 1 < FAR_STEPS ? j + TPB : j - (uint32_t)(FAR_STEPS - 1) * TPB + tile_stride;
+    return st + 1 < steps ? j + TPB : j - (uint32_t)(steps - 1) * TPB + tile_stride;
   };
   uint8_t pf_f = FLAG_HOME_SHELL;
   uint32_t pf_cell = 0, pf_lid = 0;   // (the main index only after a re-sort)
@@ -980,7 +995,7 @@ __global__ void __launch_bounds__(TPB, 4) k_rebuild_far(Dev<T> d, KParams<T> kp,
     if (distrib && d.lid) pf_lid = d.lid[i];
   }
   // the loop runs while the warp's step base is inside the array (warp-uniform)
-  for (; i - lane < n32; i = advance(i, step), step = step + 1 < FAR_STEPS ? step + 1 : 0) {
+  for (; i - lane < n32; i = advance(i, step), step = step + 1 < steps ? step + 1 : 0) {
     const bool in = i < n32;
     const uint8_t f = pf_f;
     uint32_t cell = pf_cell;
@@ -1073,11 +1088,25 @@ __global__ void __launch_bounds__(TPB, 4) k_rebuild_far(Dev<T> d, KParams<T> kp,
   block_max_to<T>(&d.ctr->maxv2, vmax2);
 }
 
+// Steps of TPB particles per tile: as many as give every block of the grid a
+// tile, at most `most` (a power of two; longer tiles keep the lists' order and
+// the arrays' sweep, but 270,000 particles in tiles of 4,096 leave nine blocks
+// of ten idle: k_rotate_main took 15.6 us there and takes 6.3, in FP64 108 and
+// 52, k_rebuild_far 17.3 and 8.5, in FP64 71 and 41).
+constexpr int FAR_STEPS_MAX = 8;    // 2048-particle tiles (4096 and 1024 measured slower at 256^3)
+constexpr int ROT_STEPS_MAX = 16;
+inline int tile_steps(int64_t n, int grid, int most) {
+  int s = most;
+  while (s > 1 && n < (int64_t)s * TPB * grid) s >>= 1;
+  return s;
+}
+
 template <typename T>
 void Launch<T>::rebuild_split(const Dev<T>& d, const KParams<T>& kp, const StepArgs& a, cudaStream_t st) {
   cudaMemsetAsync(&d.ctr->n_near, 0, sizeof(unsigned int), st);
-  k_rebuild_far<T><<<a.g_far, TPB, 0, st>>>(d, kp, a);
   StepArgs b = a;
+  b.far_steps = tile_steps(kp.n, a.g_far, FAR_STEPS_MAX);
+  k_rebuild_far<T><<<a.g_far, TPB, 0, st>>>(d, kp, b);
   b.near = 1;
   b.use_watch = 0;
   k_rebuild<T><<<a.g_rebuild, TPB, 0, st>>>(d, kp, b);
@@ -1214,7 +1243,7 @@ __global__ void __launch_bounds__(TPB, sizeof(T) == 4 ? 5 : 1) k_force(Dev<T> d,
   T msdmax = (T)0;
   // warp-aligned grid-stride loop: a warp stays converged for the per-sphere
   // warp reductions below
-  for (int64_t base = (int64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31); base < (int64_t)nin; base += stride) {
+  for (int64_t base = wave_first(nin, a.g_force) - lane; base < (int64_t)nin; base += stride) {
     const int64_t j = base + lane;
     const bool act = j < (int64_t)nin;
     uint32_t cell = 0, idx = 0;
@@ -1391,7 +1420,7 @@ __global__ void __launch_bounds__(TPB) k_shell_advance(Dev<T> d, KParams<T> kp, 
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   const T vs = sphere_speed_bound<T>(d.ctr);
   T msdmax = (T)0;
-  for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < (int64_t)nin; j += stride) {
+  for (int64_t j = wave_first(nin, (int)gridDim.x); j < (int64_t)nin; j += stride) {
     T vx = d.sh.vx[j], vy = d.sh.vy[j], vz = d.sh.vz[j];
     if (rotate) {
       T r[6];
@@ -2405,18 +2434,18 @@ __global__ void __launch_bounds__(TPB) k_rotate_main(Dev<T> d, KParams<T> kp, St
   uint32_t* wbuf = wl_buf + (threadIdx.x >> 5) * WL_CAP;
   unsigned wn = 0;
   const int lane = threadIdx.x & 31;
-  // blocks take tiles of ROT_TILE consecutive particles in a grid stride (two
+  // blocks take tiles of consecutive particles (a.rot_steps times TPB) in a grid stride (two
   // 256-particle steps per iteration), so that the watch list a warp stages
   // keeps the particles' cell order
   // (32-bit indices: particle counts are below 2^31)
-  constexpr int ROT_STEPS = 16;
-  constexpr uint32_t ROT_TILE = (uint32_t)ROT_STEPS * TPB;
+  const int steps = a.rot_steps;   // even
+  const uint32_t rot_tile = (uint32_t)steps * TPB;
   const uint32_t n32 = (uint32_t)kp.n;
-  const uint32_t tile_stride = gridDim.x * ROT_TILE;
+  const uint32_t tile_stride = gridDim.x * rot_tile;
   int step = 0;
-  for (uint32_t i0 = blockIdx.x * ROT_TILE + threadIdx.x; i0 - lane < n32;
-       i0 = step + 2 < ROT_STEPS ? i0 + 2 * TPB : i0 - (uint32_t)(ROT_STEPS - 2) * TPB + tile_stride,
-       step = step + 2 < ROT_STEPS ? step + 2 : 0) {
+  for (uint32_t i0 = blockIdx.x * rot_tile + threadIdx.x; i0 - lane < n32;
+       i0 = step + 2 < steps ? i0 + 2 * TPB : i0 - (uint32_t)(steps - 2) * TPB + tile_stride,
+       step = step + 2 < steps ? step + 2 : 0) {
     const uint32_t i1 = i0 + TPB;
     const bool h0 = i0 < n32;
     const bool h1 = i1 < n32;
@@ -2479,7 +2508,9 @@ __global__ void __launch_bounds__(TPB) k_rotate_main(Dev<T> d, KParams<T> kp, St
 
 template <typename T>
 void Launch<T>::rotate_main(const Dev<T>& d, const KParams<T>& kp, const StepArgs& a, cudaStream_t st) {
-  k_rotate_main<T><<<a.g_rotate, TPB, 0, st>>>(d, kp, a);
+  StepArgs b = a;
+  b.rot_steps = std::max(2, tile_steps(kp.n, a.g_rotate, ROT_STEPS_MAX));
+  k_rotate_main<T><<<a.g_rotate, TPB, 0, st>>>(d, kp, b);
   LAUNCH_COUNT();
 }
 
