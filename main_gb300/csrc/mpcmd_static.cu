@@ -53,6 +53,10 @@ namespace {
 constexpr int64_t kMaxCells = MPCMD_STATIC_MAX_CELLS;
 constexpr int kMaxDevices = 64;
 constexpr int kThreads = 256;
+// Largest set whose particles each form their cell's map: a map takes some 200
+// FP64 instructions, 2 us for 8,192 particles on 152 SMs, about what the cells
+// kernel's launch costs.
+constexpr int64_t kOwnMap = 8192;
 
 // per shifted cell, 12 doubles (three whole sectors): first the count (an
 // unsigned int) and the sums of vx, vy, vz, then the map v -> M v + b as rows
@@ -148,43 +152,58 @@ __global__ void __launch_bounds__(kThreads) k_static_accumulate(KParams<double> 
   }
 }
 
-// The collision of every cell as an affine map, one thread per cell: centre of
-// mass and random axis (k_cells), M the rotation by the angle about the axis
-// (both forms of rotate_v; the projection form turns the other way),
-// b = v_cm - M v_cm.
-__global__ void __launch_bounds__(kThreads) k_static_cells(KParams<double> kp, uint32_t step, double* acc) {
+// The collision of a cell as an affine map v -> M v + b: centre of mass and
+// random axis (k_cells), M the rotation by the angle about the axis (both forms
+// of rotate_v; the projection form turns the other way), b = v_cm - M v_cm.
+// a0, a1: the cell's count and velocity sums.  False for an empty cell (no
+// particle reads it).
+struct Map {
+  double M[3][3], b[3];
+};
+__device__ __forceinline__ bool cell_map(const KParams<double>& kp, uint32_t cell, uint32_t step, double2 a0, double2 a1,
+                                         Map& w) {
   const double pi = 3.141592653589793;
   const double c = kp.cosrot, c1 = 1.0 - c, sn = kp.rotation_sense > 0 ? kp.sinrot : -kp.sinrot;
+  const unsigned int cnt = (unsigned int)__double2loint(a0.x);
+  if (cnt == 0u) return false;
+  const double n = (double)cnt;
+  const double m[3] = {a0.y / n, a1.x / n, a1.y / n};
+  double u1, u2, sp, cp;
+  contract_pair(kp.seed, TAG_AXIS, cell, 0, step, u1, u2);
+  sincos(2.0 * pi * u1, &sp, &cp);
+  const double theta = 2.0 * u2 - 1.0, r = sqrt(1.0 - theta * theta);
+  const double u[3] = {r * cp, r * sp, theta};
+  const double su[3] = {sn * u[0], sn * u[1], sn * u[2]};
+  const double xy = c1 * u[0] * u[1], xz = c1 * u[0] * u[2], yz = c1 * u[1] * u[2];
+  w.M[0][0] = fma(c1 * u[0], u[0], c); w.M[0][1] = xy - su[2]; w.M[0][2] = xz + su[1];
+  w.M[1][0] = xy + su[2]; w.M[1][1] = fma(c1 * u[1], u[1], c); w.M[1][2] = yz - su[0];
+  w.M[2][0] = xz - su[1]; w.M[2][1] = yz + su[0]; w.M[2][2] = fma(c1 * u[2], u[2], c);
+#pragma unroll
+  for (int q = 0; q < 3; ++q)
+    w.b[q] = m[q] - fma(w.M[q][2], m[2], fma(w.M[q][1], m[1], w.M[q][0] * m[0]));
+  return true;
+}
+
+__global__ void __launch_bounds__(kThreads) k_static_cells(KParams<double> kp, uint32_t step, double* acc) {
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < kp.ncell_shift; i += stride) {
     double2* a = reinterpret_cast<double2*>(acc + kRec * (size_t)i);
-    const double2 a0 = a[0], a1 = a[1];
-    const unsigned int cnt = (unsigned int)__double2loint(a0.x);
-    if (cnt == 0u) continue;   // no particle reads an empty cell
-    const double n = (double)cnt;
-    const double m[3] = {a0.y / n, a1.x / n, a1.y / n};
-    double u1, u2, sp, cp;
-    contract_pair(kp.seed, TAG_AXIS, (uint32_t)i, 0, step, u1, u2);
-    sincos(2.0 * pi * u1, &sp, &cp);
-    const double theta = 2.0 * u2 - 1.0, r = sqrt(1.0 - theta * theta);
-    const double u[3] = {r * cp, r * sp, theta};
-    const double su[3] = {sn * u[0], sn * u[1], sn * u[2]};
-    const double xy = c1 * u[0] * u[1], xz = c1 * u[0] * u[2], yz = c1 * u[1] * u[2];
-    const double M[3][3] = {{fma(c1 * u[0], u[0], c), xy - su[2], xz + su[1]},
-                            {xy + su[2], fma(c1 * u[1], u[1], c), yz - su[0]},
-                            {xz - su[1], yz + su[0], fma(c1 * u[2], u[2], c)}};
+    Map w;
+    if (!cell_map(kp, (uint32_t)i, step, a[0], a[1], w)) continue;
 #pragma unroll
     for (int q = 0; q < 3; ++q) {
-      const double b = m[q] - fma(M[q][2], m[2], fma(M[q][1], m[1], M[q][0] * m[0]));
-      a[2 * q] = make_double2(M[q][0], M[q][1]);
-      a[2 * q + 1] = make_double2(M[q][2], b);
+      a[2 * q] = make_double2(w.M[q][0], w.M[q][1]);
+      a[2 * q + 1] = make_double2(w.M[q][2], w.b[q]);
     }
   }
 }
 
+// OWN_MAP: every particle forms its cell's map from the sums itself (the sets
+// of at most kOwnMap particles, which no cells kernel precedes).
+template <bool OWN_MAP>
 __global__ void __launch_bounds__(kThreads) k_static_rotate(KParams<double> kp, const double* x, const double* y,
                                                             const double* z, double* vx, double* vy, double* vz,
-                                                            int64_t n, Shift s, const double* acc) {
+                                                            int64_t n, Shift s, uint32_t step, const double* acc) {
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += stride) {
     uint32_t key = fast_key(kp, x[i], y[i], z[i], s);
@@ -192,10 +211,17 @@ __global__ void __launch_bounds__(kThreads) k_static_rotate(KParams<double> kp, 
     const double2* a = reinterpret_cast<const double2*>(acc + kRec * (size_t)key);
     const double v0 = vx[i], v1 = vy[i], v2 = vz[i];
     double w[3];
+    if constexpr (OWN_MAP) {
+      Map c;
+      if (!cell_map(kp, key, step, a[0], a[1], c)) continue;
 #pragma unroll
-    for (int q = 0; q < 3; ++q) {
-      const double2 h = a[2 * q], l = a[2 * q + 1];
-      w[q] = fma(h.x, v0, fma(h.y, v1, fma(l.x, v2, l.y)));
+      for (int q = 0; q < 3; ++q) w[q] = fma(c.M[q][0], v0, fma(c.M[q][1], v1, fma(c.M[q][2], v2, c.b[q])));
+    } else {
+#pragma unroll
+      for (int q = 0; q < 3; ++q) {
+        const double2 h = a[2 * q], l = a[2 * q + 1];
+        w[q] = fma(h.x, v0, fma(h.y, v1, fma(l.x, v2, l.y)));
+      }
     }
     vx[i] = w[0]; vy[i] = w[1]; vz[i] = w[2];
   }
@@ -258,8 +284,12 @@ extern "C" int mpcmd_collide_static(const double* x, const double* y, const doub
   const int tgrid = (int)std::min<int64_t>((ncs + kThreads - 1) / kThreads, (int64_t)nsm * 8);
   k_static_clear<<<tgrid, kThreads, 0, st>>>(acc, ncs);
   k_static_accumulate<<<grid, kThreads, 0, st>>>(kp, x, y, z, vx, vy, vz, n, s, acc);
-  k_static_cells<<<tgrid, kThreads, 0, st>>>(kp, (uint32_t)step, acc);
-  k_static_rotate<<<grid, kThreads, 0, st>>>(kp, x, y, z, vx, vy, vz, n, s, acc);
+  if (n <= kOwnMap) {
+    k_static_rotate<true><<<grid, kThreads, 0, st>>>(kp, x, y, z, vx, vy, vz, n, s, (uint32_t)step, acc);
+  } else {
+    k_static_cells<<<tgrid, kThreads, 0, st>>>(kp, (uint32_t)step, acc);
+    k_static_rotate<false><<<grid, kThreads, 0, st>>>(kp, x, y, z, vx, vy, vz, n, s, (uint32_t)step, acc);
+  }
   if (cudaPeekAtLastError() != cudaSuccess) return MPCMD_ERR_CUDA;
   return MPCMD_OK;
 }
