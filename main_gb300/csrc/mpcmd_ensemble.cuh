@@ -91,6 +91,12 @@ struct Glob {
   int pad;
 };
 
+// One shell work tile: entries [e0, e0 + cnt) of replica rep.
+struct STile {
+  uint32_t rep, cnt;
+  int64_t e0;
+};
+
 template <typename T>
 struct EDev {
   const Rep<T>* rep;
@@ -129,7 +135,7 @@ struct EDev {
   const int64_t* ct_lo;    // local cell range of the tile
   const int64_t* ct_hi;
   int n_ctiles;
-  uint32_t* st_prefix;     // [R + 1] first shell tile of each replica
+  STile* stile;            // shell tiles of every replica
   uint32_t* rt_prefix;     // [R + 1] first rebuild tile of each replica (0 tiles when it does not rebuild)
   int tile;                // particles per tile
   // samples
@@ -459,7 +465,9 @@ __global__ void __launch_bounds__(MAX_BLOCK) k_ens_rebuild(EDev<T> d, int mode) 
             const int64_t e = R.soff + slot;
             d.sh_idx[e] = (uint32_t)i;
             d.sh_mask[e] = (uint8_t)mask;
-            for (int q = 0; q < 6; ++q) d.sh_fp[6 * e + q] = (T)0;
+            // (the run's first half kick, of a prepared state, uses zero pair forces)
+            if (!(mode & M_LAZY))
+              for (int q = 0; q < 6; ++q) d.sh_fp[6 * e + q] = (T)0;
             d.sh_msd[e] = (T)0;
           } else {
             atomicOr(&y.status, E_ERR_SHELL);
@@ -474,30 +482,14 @@ __global__ void __launch_bounds__(MAX_BLOCK) k_ens_rebuild(EDev<T> d, int mode) 
   }
 }
 
-// After the rebuild: time_penetrate of the rebuilt replicas
-// (main_pattern.f95:187, evolve_mod.f95:555-563), the shell work tiles of
-// every replica, and the step counter.  One block.
+// The shell tiles of every replica, from the shell sizes.  One block.
 template <typename T>
-__global__ void k_ens_finalize(EDev<T> d, int shell_block, int advance_step) {
-  __shared__ unsigned part[1024];
+__device__ __forceinline__ void write_shell_tiles(const EDev<T>& d, int shell_block, unsigned* part /* [blockDim] */) {
   const int nt = blockDim.x;
   const int chunk = (d.R + nt - 1) / nt;
   const int lo = min(d.R, (int)threadIdx.x * chunk), hi = min(d.R, lo + chunk);
   unsigned local = 0;
-  for (int r = lo; r < hi; ++r) {
-    Dyn<T>& y = d.dyn[r];
-    const Rep<T>& R = d.rep[r];
-    if (y.rebuild) {
-      const double maxt = __longlong_as_double((long long)y.maxv2);
-      y.time_penetrate = (int)floor((0.5 * R.skin / sqrt(maxt)) / R.kp.dtd);
-      y.time_count = 0;
-      y.rebuild = 0;
-      y.maxv2 = 0ull;
-      y.rebuilds += 1;
-      if (y.n_shell > (unsigned)R.scap) y.n_shell = (unsigned)R.scap;
-    }
-    local += (y.n_shell + shell_block - 1) / shell_block;
-  }
+  for (int r = lo; r < hi; ++r) local += (d.dyn[r].n_shell + shell_block - 1) / shell_block;
   part[threadIdx.x] = local;
   __syncthreads();
   // inclusive scan of the per-thread tile counts (Hillis-Steele)
@@ -509,14 +501,43 @@ __global__ void k_ens_finalize(EDev<T> d, int shell_block, int advance_step) {
   }
   unsigned run = threadIdx.x ? part[threadIdx.x - 1] : 0u;
   for (int r = lo; r < hi; ++r) {
-    d.st_prefix[r] = run;
-    run += (d.dyn[r].n_shell + shell_block - 1) / shell_block;
+    const unsigned n = d.dyn[r].n_shell;
+    const int64_t e0 = d.rep[r].soff;
+    for (unsigned k = 0; k < n; k += shell_block)
+      d.stile[run++] = STile{(uint32_t)r, min((unsigned)shell_block, n - k), e0 + k};
   }
-  if (threadIdx.x == nt - 1) {
-    d.st_prefix[d.R] = part[nt - 1];
-    d.g->ntiles_s = part[nt - 1];
-    if (advance_step) d.g->cstep += 1;
+  if (threadIdx.x == nt - 1) d.g->ntiles_s = part[nt - 1];
+}
+
+template <typename T>
+__global__ void k_ens_tiles(EDev<T> d, int shell_block) {
+  __shared__ unsigned part[1024];
+  write_shell_tiles(d, shell_block, part);
+}
+
+// After the rebuild: time_penetrate of the rebuilt replicas
+// (main_pattern.f95:187, evolve_mod.f95:555-563), the shell work tiles (when a
+// replica rebuilt) and the step counter.  One block.
+template <typename T>
+__global__ void k_ens_finalize(EDev<T> d, int shell_block, int advance_step) {
+  __shared__ unsigned part[1024];
+  int any = 0;
+  for (int r = threadIdx.x; r < d.R; r += blockDim.x) {
+    Dyn<T>& y = d.dyn[r];
+    const Rep<T>& R = d.rep[r];
+    if (y.rebuild) {
+      any = 1;
+      const double maxt = __longlong_as_double((long long)y.maxv2);
+      y.time_penetrate = (int)floor((0.5 * R.skin / sqrt(maxt)) / R.kp.dtd);
+      y.time_count = 0;
+      y.rebuild = 0;
+      y.maxv2 = 0ull;
+      y.rebuilds += 1;
+      if (y.n_shell > (unsigned)R.scap) y.n_shell = (unsigned)R.scap;
+    }
   }
+  if (threadIdx.x == 0 && advance_step) d.g->cstep += 1;
+  if (__syncthreads_or(any)) write_shell_tiles(d, shell_block, part);
 }
 
 // --------------------------------------------------------------- forces ----
@@ -527,34 +548,44 @@ __global__ void k_ens_finalize(EDev<T> d, int shell_block, int advance_step) {
 // free flight of the next step with max_solvent_dist (:225-316, :457-463)
 // [M_ADVANCE].  The kicks add the C pair force, then the N pair force
 // (kick_lists order); the FP32 build adds their sum.
-template <typename T>
-__global__ void __launch_bounds__(MAX_BLOCK) k_ens_force(EDev<T> d, int mode) {
+//
+// Bound by the entries' gathered states (67 bytes an entry read and written)
+// and, for few replicas, by the chain of dependent loads in front of them: a
+// tile's descriptor gives its replica and entries in one load (a binary search
+// over the tile prefix was four to eight).  The pair forces pass through
+// memory only from a step that ends a call or a period (M_FORCE alone) to the
+// M_ADVANCE that opens the next; a fused step neither reads nor keeps them,
+// which was 48 bytes an entry: 54 us per MD step for 256 replicas against 83,
+// 5.5 us against 7.7 for 16.
+template <typename T, int MODE>
+__global__ void __launch_bounds__(MAX_BLOCK) k_ens_force(EDev<T> d) {
+  constexpr bool FORCE = (MODE & M_FORCE) != 0, ADVANCE = (MODE & M_ADVANCE) != 0;
   __shared__ double red[8 * 32];
   __shared__ float redf[8 * 32];
   __shared__ T redm[32];
   const unsigned ntiles = d.g->ntiles_s;
   for (unsigned t = blockIdx.x; t < ntiles; t += gridDim.x) {
-    const int r = tile_rep(d.st_prefix, d.R, t);
-    Dyn<T>& y = d.dyn[r];
-    const Rep<T>& R = d.rep[r];
-    const KParams<T>& kp = R.kp;
-    const int64_t j = (int64_t)(t - d.st_prefix[r]) * blockDim.x + threadIdx.x;
-    const bool valid = j < (int64_t)y.n_shell;
+    const STile tile = d.stile[t];
+    Dyn<T>& y = d.dyn[tile.rep];
+    const KParams<T>& kp = d.rep[tile.rep].kp;
     T sums[8] = {(T)0, (T)0, (T)0, (T)0, (T)0, (T)0, (T)0, (T)0};
     T msd = (T)0;
-    if (valid) {
-      const int64_t e = R.soff + j;
+    if (threadIdx.x < tile.cnt) {
+      const int64_t e = tile.e0 + threadIdx.x;
       const uint32_t i = d.sh_idx[e];
-      const int mask = d.sh_mask[e];
+      const int mask = FORCE ? d.sh_mask[e] : 0;
+      T msd0 = (T)0;   // loaded with the rest: its use at the end would wait on it
+      if (ADVANCE) msd0 = d.sh_msd[e];
       uint32_t cell = d.cell[i];
       T ox = d.ox[i], oy = d.oy[i], oz = d.oz[i];
       T vx = d.vx[i], vy = d.vy[i], vz = d.vz[i];
       uint8_t f = d.flag[i];
       T fp[6];
-      for (int q = 0; q < 6; ++q) fp[q] = d.sh_fp[6 * e + q];
-      if (mode & M_FORCE) {
+#pragma unroll
+      for (int q = 0; q < 6; ++q) fp[q] = FORCE ? (T)0 : d.sh_fp[6 * e + q];
+      if (FORCE) {
+#pragma unroll
         for (int s = 0; s < 2; ++s) {
-          fp[3 * s] = fp[3 * s + 1] = fp[3 * s + 2] = (T)0;
           if (!(mask & (1 << s))) continue;
           T dx, dy, dz;
           const T dR2 = sep2(kp, cell, ox, oy, oz, y.srel[s], dx, dy, dz);
@@ -571,8 +602,8 @@ __global__ void __launch_bounds__(MAX_BLOCK) k_ens_force(EDev<T> d, int mode) {
         }
       }
       const T h = kp.hIM[f & FLAG_SPECIES];
-      const int nk = ((mode & M_FORCE) ? 1 : 0) + ((mode & M_ADVANCE) ? 1 : 0);
-      for (int k = 0; k < nk; ++k) {
+#pragma unroll
+      for (int k = 0; k < (FORCE ? 1 : 0) + (ADVANCE ? 1 : 0); ++k) {
         if (sizeof(T) == 8) {
           vx = vx + h * fp[0]; vy = vy + h * fp[1]; vz = vz + h * fp[2];
           vx = vx + h * fp[3]; vy = vy + h * fp[4]; vz = vz + h * fp[5];
@@ -580,19 +611,21 @@ __global__ void __launch_bounds__(MAX_BLOCK) k_ens_force(EDev<T> d, int mode) {
           vx += h * (fp[0] + fp[3]); vy += h * (fp[1] + fp[4]); vz += h * (fp[2] + fp[5]);
         }
       }
-      if (mode & M_ADVANCE) {
+      if (ADVANCE) {
         stream_one(kp, (const uint8_t*)nullptr, cell, ox, oy, oz, vx, vy, vz, f, false, 0);
-        msd = d.sh_msd[e] + (vx * vx + vy * vy + vz * vz) * (kp.dt * kp.dt);
+        msd = msd0 + (vx * vx + vy * vy + vz * vz) * (kp.dt * kp.dt);
         d.sh_msd[e] = msd;
         d.cell[i] = cell;
         d.ox[i] = ox; d.oy[i] = oy; d.oz[i] = oz;
       }
       d.vx[i] = vx; d.vy[i] = vy; d.vz[i] = vz;
-      d.flag[i] = f;
-      if (mode & M_FORCE)
+      if (FORCE) d.flag[i] = f;
+      if (FORCE && !ADVANCE) {
+#pragma unroll
         for (int q = 0; q < 6; ++q) d.sh_fp[6 * e + q] = fp[q];
+      }
     }
-    if (mode & M_FORCE) {
+    if (FORCE) {
       if (sizeof(T) == 4) {
         float sf[8];
         for (int q = 0; q < 8; ++q) sf[q] = (float)sums[q];
@@ -607,7 +640,7 @@ __global__ void __launch_bounds__(MAX_BLOCK) k_ens_force(EDev<T> d, int mode) {
             if (sd[q] != 0.) atomicAdd(&y.facc[q], sd[q]);
       }
     }
-    if (mode & M_ADVANCE) {
+    if (ADVANCE) {
       const T m = block_max(msd, redm);
       if (threadIdx.x == 0 && m > (T)0) atomicMax(&y.maxmsd, ord_bits(to_f64(m)));
     }

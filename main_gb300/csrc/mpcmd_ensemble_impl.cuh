@@ -188,7 +188,7 @@ struct Ensemble : EnsembleBase {
     s |= alloc(scan_tmp, scan_tmp_words(ctot));
     Rep<T>* drep = nullptr; Dyn<T>* ddyn = nullptr; Glob* dg = nullptr;
     s |= alloc(drep, R); s |= alloc(ddyn, R); s |= alloc(dg, 1);
-    s |= alloc(d.st_prefix, R + 1);
+    s |= alloc(d.stile, stot / 32 + R);   // (at least 32 entries in every tile but a replica's last)
     s |= alloc(d.rt_prefix, R + 1);
     s |= alloc(d_mass, 4 * (int64_t)R); s |= alloc(d_obs, 8 * (int64_t)R);
     if (s) return MPCMD_ERR_ALLOC;
@@ -196,7 +196,6 @@ struct Ensemble : EnsembleBase {
     ECK(cudaMemcpyAsync(drep, hrep.data(), sizeof(Rep<T>) * R, cudaMemcpyHostToDevice, st));
     ECK(cudaMemsetAsync(ddyn, 0, sizeof(Dyn<T>) * R, st));
     ECK(cudaMemsetAsync(dg, 0, sizeof(Glob), st));
-    ECK(cudaMemsetAsync(d.st_prefix, 0, sizeof(uint32_t) * (R + 1), st));
     ECK(cudaMemsetAsync(d.rt_prefix, 0, sizeof(uint32_t) * (R + 1), st));
     ECK(cudaMemsetAsync(d.acc, 0, (sizeof(T) == 4 ? 16 : 32) * (size_t)ctot, st));
     ECK(cudaMemsetAsync(d.dcnt, 0, 4 * (size_t)ctot, st));
@@ -254,10 +253,11 @@ struct Ensemble : EnsembleBase {
     d.n_ptiles = (int)np; d.n_ctiles = (int)nc;
     int occ_p = 0, occ_s = 0;
     ECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_p, k_ens_rebuild<T>, b, 0));
-    ECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_s, k_ens_force<T>, sb, 0));
+    ECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_s, k_ens_force<T, M_FORCE | M_ADVANCE>, sb, 0));
     g_part = nsm * std::max(occ_p, 1);
     g_shell = nsm * std::max(occ_s, 1);
     invalidate_graph();
+    if (prepared) L_tiles();   // the lists' tiles follow the shell tile size
     return MPCMD_OK;
   }
 
@@ -268,7 +268,13 @@ struct Ensemble : EnsembleBase {
   }
 
   // ---------------------------------------------------------- launches --
-  void L_force(int mode) { k_ens_force<T><<<g_shell, sblock, 0, st>>>(d, mode); ++launches; }
+  void L_force(int mode) {
+    if (mode == M_FORCE) k_ens_force<T, M_FORCE><<<g_shell, sblock, 0, st>>>(d);
+    else if (mode == M_ADVANCE) k_ens_force<T, M_ADVANCE><<<g_shell, sblock, 0, st>>>(d);
+    else k_ens_force<T, M_FORCE | M_ADVANCE><<<g_shell, sblock, 0, st>>>(d);
+    ++launches;
+  }
+  void L_tiles() { k_ens_tiles<T><<<1, 1024, 0, st>>>(d, sblock); ++launches; }
   void L_dimer(int mode) {
     if (sizeof(T) == 4) {
       // four lanes per replica, one 32-lane block per eight replicas (spread over the SMs)
@@ -645,7 +651,7 @@ struct Ensemble : EnsembleBase {
                       {d.vy, sizeof(T) * (size_t)ntot}, {d.vz, sizeof(T) * (size_t)ntot}, {d.flag, (size_t)ntot},
                       {d.sh_idx, 4 * (size_t)stot}, {d.sh_mask, (size_t)stot}, {d.sh_fp, 6 * sizeof(T) * (size_t)stot},
                       {d.sh_msd, sizeof(T) * (size_t)stot}, {d.dyn, sizeof(Dyn<T>) * (size_t)R},
-                      {d.g, sizeof(Glob)}, {d.st_prefix, 4 * (size_t)(R + 1)},
+                      {d.g, sizeof(Glob)},
                       {d.rt_prefix, 4 * (size_t)(R + 1)}};
       for (auto& rg : snap_regions) {
         void* p = nullptr;
@@ -659,6 +665,7 @@ struct Ensemble : EnsembleBase {
       for (size_t k = 0; k < snap_regions.size(); ++k)
         ECK(cudaMemcpyAsync(snap_regions[k].first, snap_copies[k], snap_regions[k].second, cudaMemcpyDeviceToDevice, st));
       cstep = snap_cstep; prepared = snap_prepared; need_advance = snap_need_advance; vel_pending = snap_vel_pending;
+      if (prepared) L_tiles();
     }
     ECK(cudaStreamSynchronize(st));
     return MPCMD_OK;
