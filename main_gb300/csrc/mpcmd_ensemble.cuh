@@ -13,7 +13,7 @@
 // one replica) at a time, so a block-level reduction is always a reduction
 // within one replica.  The particle and cell tiles are fixed at creation; the
 // shell tiles follow the shell sizes, which each replica's rebuilds change on
-// the device (k_ens_finalize rescans them).  Nothing in a collision period
+// the device (k_ens_rebuild rewrites them).  Nothing in a collision period
 // needs the host: the rebuild decision of each replica (displacement
 // criterion, time_penetrate, collision step: evolve_mod.f95:457-465) is taken
 // by k_ens_dimer and read by the rebuild kernel, which skips the tiles of the
@@ -22,10 +22,11 @@
 // Step sequence (main_pattern.f95:203-225 for every replica), kernels in
 // launch order:
 //   k_ens_dimer  (VEL)   totals and RATTLE velocities of the previous step
-//   k_ens_dimer  (POS)   time_count + 1, RATTLE positions, rebuild decision
+//   k_ens_dimer  (POS)   time_count + 1, RATTLE positions, rebuild decision;
+//                        the rebuild's tiles (its last block)
 //   k_ens_rebuild        lazy streaming of the outside particles and the new
-//                        lists of the rebuilding replicas
-//   k_ens_finalize       time_penetrate, shell tiles, step counter
+//                        lists of the rebuilding replicas; step counter,
+//                        time_penetrate and shell tiles (its last block)
 //   k_ens_force          forces, catalysis, sphere sums, second half kick; fused
 //                        with the next step's first half kick and free flight
 //   collision steps:     k_ens_collide (shifted keys, collision sums,
@@ -85,10 +86,9 @@ struct Dyn {
 };
 
 struct Glob {
-  unsigned cstep;          // step being executed (advanced by k_ens_finalize)
+  unsigned cstep;          // step being executed (advanced at the end of k_ens_rebuild)
   unsigned ntiles_s;       // shell tiles
-  int status;
-  int pad;
+  unsigned arrived[2];     // blocks that have finished: dimer step, rebuild
 };
 
 // One shell work tile: entries [e0, e0 + cnt) of replica rep.
@@ -136,6 +136,8 @@ struct EDev {
   const int64_t* ct_hi;
   int n_ctiles;
   STile* stile;            // shell tiles of every replica
+  uint32_t* st_prefix;     // [R] first shell tile of each replica
+  uint32_t* rt_need;       // [R] rebuild tiles of each replica (0 when it does not rebuild)
   uint32_t* rt_prefix;     // [R + 1] first rebuild tile of each replica (0 tiles when it does not rebuild)
   int tile;                // particles per tile
   // samples
@@ -396,37 +398,140 @@ __device__ __forceinline__ int tile_rep(const uint32_t* prefix, int R, unsigned 
   return lo;
 }
 
-// Plan of a rebuild: the particle tiles of the replicas whose rebuild flag
-// k_ens_dimer set, as a prefix over replicas.  One block.
+// Inclusive scan of one value per thread over the block into part[].
+__device__ __forceinline__ void block_scan(unsigned* part, unsigned v) {
+  part[threadIdx.x] = v;
+  __syncthreads();
+  for (unsigned o = 1; o < blockDim.x; o <<= 1) {
+    const unsigned w = threadIdx.x >= o ? part[threadIdx.x - o] : 0u;
+    __syncthreads();
+    part[threadIdx.x] += w;
+    __syncthreads();
+  }
+}
+
+// Rebuild tiles of a replica of n particles.
+template <typename T>
+__device__ __forceinline__ uint32_t rebuild_tiles(const EDev<T>& d, const Rep<T>& R) {
+  return ((uint32_t)R.n + (uint32_t)d.tile - 1u) / (uint32_t)d.tile;
+}
+
+// Plan of a rebuild: the tiles of the rebuilding replicas (rt_need) as a
+// prefix over replicas (one block, at most 256 threads).  rt_need may have been
+// written by other blocks of this launch.
+template <typename T>
+__device__ __forceinline__ void write_plan(const EDev<T>& d, unsigned* part) {
+  constexpr int KEEP = 8;   // values kept in registers between the two passes
+  const int nt = blockDim.x;
+  const int chunk = (d.R + nt - 1) / nt;
+  const int lo = min(d.R, (int)threadIdx.x * chunk), hi = min(d.R, lo + chunk);
+  unsigned v[KEEP], local = 0;
+#pragma unroll
+  for (int k = 0; k < KEEP; ++k) v[k] = lo + k < hi ? __ldcg(&d.rt_need[lo + k]) : 0u;
+#pragma unroll
+  for (int k = 0; k < KEEP; ++k) local += v[k];
+  for (int r = lo + KEEP; r < hi; ++r) local += __ldcg(&d.rt_need[r]);
+  block_scan(part, local);
+  unsigned run = threadIdx.x ? part[threadIdx.x - 1] : 0u;
+#pragma unroll
+  for (int k = 0; k < KEEP; ++k) {
+    if (lo + k < hi) d.rt_prefix[lo + k] = run;
+    run += v[k];
+  }
+  for (int r = lo + KEEP; r < hi; ++r) { d.rt_prefix[r] = run; run += __ldcg(&d.rt_need[r]); }
+  if (threadIdx.x == nt - 1) d.rt_prefix[d.R] = part[nt - 1];
+}
+
+// The plan of a prepared state, whose rebuild flags the host has set.
 template <typename T>
 __global__ void k_ens_plan(EDev<T> d) {
-  __shared__ unsigned part[1024];
+  __shared__ unsigned part[256];
+  for (int r = threadIdx.x; r < d.R; r += blockDim.x)
+    d.rt_need[r] = d.dyn[r].rebuild ? rebuild_tiles(d, d.rep[r]) : 0u;
+  __threadfence();
+  __syncthreads();
+  write_plan(d, part);
+}
+
+// Whether this block is the last of `blocks` to arrive (every thread of the
+// block gets the answer): what the others wrote before arriving is visible to
+// it.  The counter returns to zero for the next launch.
+__device__ __forceinline__ bool last_block(unsigned* counter, unsigned blocks) {
+  __shared__ bool last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    last = atomicAdd(counter, 1u) == blocks - 1u;
+    if (last) *counter = 0u;
+  }
+  __syncthreads();
+  if (last) __threadfence();
+  return last;
+}
+
+// The shell tiles of every replica, from the shell sizes.  One block.
+template <typename T>
+__device__ __forceinline__ void write_shell_tiles(const EDev<T>& d, int shell_block, unsigned* part) {
   const int nt = blockDim.x;
   const int chunk = (d.R + nt - 1) / nt;
   const int lo = min(d.R, (int)threadIdx.x * chunk), hi = min(d.R, lo + chunk);
   unsigned local = 0;
-  for (int r = lo; r < hi; ++r)
-    if (d.dyn[r].rebuild) local += (unsigned)((d.rep[r].n + d.tile - 1) / d.tile);
-  part[threadIdx.x] = local;
-  __syncthreads();
-  for (int o = 1; o < nt; o <<= 1) {
-    unsigned v = threadIdx.x >= (unsigned)o ? part[threadIdx.x - o] : 0u;
-    __syncthreads();
-    part[threadIdx.x] += v;
-    __syncthreads();
-  }
+  for (int r = lo; r < hi; ++r) local += (__ldcg(&d.dyn[r].n_shell) + shell_block - 1) / shell_block;
+  block_scan(part, local);
   unsigned run = threadIdx.x ? part[threadIdx.x - 1] : 0u;
   for (int r = lo; r < hi; ++r) {
-    d.rt_prefix[r] = run;
-    if (d.dyn[r].rebuild) run += (unsigned)((d.rep[r].n + d.tile - 1) / d.tile);
+    d.st_prefix[r] = run;
+    run += (__ldcg(&d.dyn[r].n_shell) + shell_block - 1) / shell_block;
   }
-  if (threadIdx.x == nt - 1) d.rt_prefix[d.R] = part[nt - 1];
+  if (threadIdx.x == nt - 1) d.g->ntiles_s = part[nt - 1];
+  __threadfence();   // (the prefixes are read back from L2)
+  __syncthreads();
+  // a warp per replica writes its tiles
+  const int lane = threadIdx.x & 31;
+  for (int r = threadIdx.x >> 5; r < d.R; r += nt >> 5) {
+    const unsigned n = __ldcg(&d.dyn[r].n_shell), first = __ldcg(&d.st_prefix[r]);
+    const int64_t e0 = d.rep[r].soff;
+    for (unsigned k = lane; k * shell_block < n; k += 32)
+      d.stile[first + k] =
+          STile{(uint32_t)r, min((unsigned)shell_block, n - k * shell_block), e0 + (int64_t)k * shell_block};
+  }
 }
 
 template <typename T>
-__global__ void __launch_bounds__(MAX_BLOCK) k_ens_rebuild(EDev<T> d, int mode) {
+__global__ void k_ens_tiles(EDev<T> d, int shell_block) {
+  __shared__ unsigned part[256];
+  write_shell_tiles(d, shell_block, part);
+}
+
+// After the lists of the rebuilding replicas are complete (the last block of
+// the rebuild): their time_penetrate (main_pattern.f95:187,
+// evolve_mod.f95:555-563) and the shell work tiles.
+template <typename T>
+__device__ __forceinline__ void finish_rebuild(const EDev<T>& d, int shell_block, unsigned* part) {
+  for (int r = threadIdx.x; r < d.R; r += blockDim.x) {
+    Dyn<T>& y = d.dyn[r];
+    const Rep<T>& R = d.rep[r];
+    if (y.rebuild) {
+      const double maxt = __longlong_as_double((long long)__ldcg(&y.maxv2));
+      y.time_penetrate = (int)floor((0.5 * R.skin / sqrt(maxt)) / R.kp.dtd);
+      y.time_count = 0;
+      y.rebuild = 0;
+      y.maxv2 = 0ull;
+      y.rebuilds += 1;
+      if (__ldcg(&y.n_shell) > (unsigned)R.scap) y.n_shell = (unsigned)R.scap;
+    }
+  }
+  __threadfence();   // (the clamped sizes are read back from L2)
+  __syncthreads();
+  write_shell_tiles(d, shell_block, part);
+}
+
+template <typename T>
+__global__ void __launch_bounds__(MAX_BLOCK) k_ens_rebuild(EDev<T> d, int mode, int shell_block, int advance_step) {
   __shared__ T red[32];
+  __shared__ unsigned part[MAX_BLOCK];
   const unsigned ntiles = d.rt_prefix[d.R];
+  if (advance_step && blockIdx.x == 0 && threadIdx.x == 0) d.g->cstep += 1;   // (nothing in this launch reads it)
   for (unsigned t = blockIdx.x; t < ntiles; t += gridDim.x) {
     const int r = tile_rep(d.rt_prefix, d.R, t);
     Dyn<T>& y = d.dyn[r];
@@ -480,64 +585,10 @@ __global__ void __launch_bounds__(MAX_BLOCK) k_ens_rebuild(EDev<T> d, int mode) 
       if (threadIdx.x == 0 && m > (T)0) atomicMax(&y.maxv2, ord_bits(to_f64(m)));
     }
   }
-}
-
-// The shell tiles of every replica, from the shell sizes.  One block.
-template <typename T>
-__device__ __forceinline__ void write_shell_tiles(const EDev<T>& d, int shell_block, unsigned* part /* [blockDim] */) {
-  const int nt = blockDim.x;
-  const int chunk = (d.R + nt - 1) / nt;
-  const int lo = min(d.R, (int)threadIdx.x * chunk), hi = min(d.R, lo + chunk);
-  unsigned local = 0;
-  for (int r = lo; r < hi; ++r) local += (d.dyn[r].n_shell + shell_block - 1) / shell_block;
-  part[threadIdx.x] = local;
-  __syncthreads();
-  // inclusive scan of the per-thread tile counts (Hillis-Steele)
-  for (int o = 1; o < nt; o <<= 1) {
-    unsigned v = threadIdx.x >= (unsigned)o ? part[threadIdx.x - o] : 0u;
-    __syncthreads();
-    part[threadIdx.x] += v;
-    __syncthreads();
-  }
-  unsigned run = threadIdx.x ? part[threadIdx.x - 1] : 0u;
-  for (int r = lo; r < hi; ++r) {
-    const unsigned n = d.dyn[r].n_shell;
-    const int64_t e0 = d.rep[r].soff;
-    for (unsigned k = 0; k < n; k += shell_block)
-      d.stile[run++] = STile{(uint32_t)r, min((unsigned)shell_block, n - k), e0 + k};
-  }
-  if (threadIdx.x == nt - 1) d.g->ntiles_s = part[nt - 1];
-}
-
-template <typename T>
-__global__ void k_ens_tiles(EDev<T> d, int shell_block) {
-  __shared__ unsigned part[1024];
-  write_shell_tiles(d, shell_block, part);
-}
-
-// After the rebuild: time_penetrate of the rebuilt replicas
-// (main_pattern.f95:187, evolve_mod.f95:555-563), the shell work tiles (when a
-// replica rebuilt) and the step counter.  One block.
-template <typename T>
-__global__ void k_ens_finalize(EDev<T> d, int shell_block, int advance_step) {
-  __shared__ unsigned part[1024];
-  int any = 0;
-  for (int r = threadIdx.x; r < d.R; r += blockDim.x) {
-    Dyn<T>& y = d.dyn[r];
-    const Rep<T>& R = d.rep[r];
-    if (y.rebuild) {
-      any = 1;
-      const double maxt = __longlong_as_double((long long)y.maxv2);
-      y.time_penetrate = (int)floor((0.5 * R.skin / sqrt(maxt)) / R.kp.dtd);
-      y.time_count = 0;
-      y.rebuild = 0;
-      y.maxv2 = 0ull;
-      y.rebuilds += 1;
-      if (y.n_shell > (unsigned)R.scap) y.n_shell = (unsigned)R.scap;
-    }
-  }
-  if (threadIdx.x == 0 && advance_step) d.g->cstep += 1;
-  if (__syncthreads_or(any)) write_shell_tiles(d, shell_block, part);
+  // the last of the blocks that had work finishes the rebuild (most MD steps
+  // rebuild no replica and end here)
+  if ((mode & M_LISTS) && blockIdx.x < ntiles && last_block(&d.g->arrived[1], min(ntiles, gridDim.x)))
+    finish_rebuild(d, shell_block, part);
 }
 
 // --------------------------------------------------------------- forces ----
@@ -648,174 +699,25 @@ __global__ void __launch_bounds__(MAX_BLOCK) k_ens_force(EDev<T> d) {
 }
 
 // ---------------------------------------------------------------- dimer ----
-// One thread per replica, the FP64 operation sequence of the reference:
 // M_VEL  sphere totals (evolve_mod.f95:605-636) and RATTLE velocities
 //        (:679-724); on a collision step also the propulsion-speed sample
 //        (Output_SelkovDimer.f90:168-172) and the grid shift of the collision
 //        (mpc_rotation_mod.f95:102-107);
 // M_POS  time_count + 1, RATTLE positions of the next step (:320-417) and the
-//        rebuild decision (:457-465).
+//        rebuild decision (:457-465); the last block then plans the rebuild.
+// With the rebuild's end in its own last block, an MD step is three launches
+// instead of five: 16 replicas 2.05 -> 1.92 ms per logged period.
+// The three Cartesian components of a replica's dimer run on three lanes of a
+// 4-lane group (the fourth lane holds zeros and the replica's scalar work),
+// every dot product summed over the group: at GB300's FP64 rate the per-replica
+// chain of FP64 instructions sets the kernel's time, and the split shortens it
+// about threefold.  The group sums add the same terms in the same order as a
+// single thread would ((x + y) + (z + 0)), so the FP64 build keeps the
+// reference's operation sequence (divisions by constants through div_const,
+// wraps through wrap_box, as k_dimer_split); the FP32 build multiplies by
+// precomputed reciprocals and wraps the positions once after the iterations.
 template <typename T>
 __global__ void k_ens_dimer(EDev<T> d, int mode, int rattle_max) {
-  const int r = blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= d.R) return;
-  Dyn<T>& y = d.dyn[r];
-  const Rep<T>& R = d.rep[r];
-  const KParams<T>& kp = R.kp;
-  const double dt = kp.dtd, Mc = kp.mc, Mn = kp.mn, Dcn = kp.dcn;
-  const double hIMc = kp.hIMc, hIMn = kp.hIMn, IIM = kp.IIM;
-  // the FP32 build multiplies by precomputed reciprocals and wraps the
-  // positions once after the iterations (the constraint uses minimum-image
-  // separations); the FP64 build keeps the reference's operation sequence
-  constexpr bool fast = sizeof(T) == 4;
-  double X1[3], X2[3], V1[3], V2[3], F1[3], F2[3], Q1[3], Q2[3];
-  for (int c = 0; c < 3; ++c) {
-    X1[c] = y.dpos[c]; X2[c] = y.dpos[3 + c];
-    V1[c] = y.dvel[c]; V2[c] = y.dvel[3 + c];
-    F1[c] = y.dfrc[c]; F2[c] = y.dfrc[3 + c];
-    Q1[c] = y.dq[c]; Q2[c] = y.dq[3 + c];
-  }
-  unsigned long long iters = 0;
-  if (mode & M_VEL) {
-    for (int c = 0; c < 3; ++c) { F1[c] = y.facc[c]; F2[c] = y.facc[4 + c]; }
-    y.pot = y.facc[3] + y.facc[7];
-    for (int q = 0; q < 8; ++q) y.facc[q] = 0.;
-    for (int c = 0; c < 3; ++c) { V1[c] = Q1[c] + hIMc * F1[c]; V2[c] = Q2[c] + hIMn * F2[c]; }
-    int acc = 0;
-    for (;;) {
-      double dV[3], dd[3];
-      for (int c = 0; c < 3; ++c) { dV[c] = V1[c] - V2[c]; dd[c] = dmi(X1[c] - X2[c], kp.Ld[c]); }
-      const double Con2diff = 2.0 * (dV[0] * dd[0] + dV[1] * dd[1] + dV[2] * dd[2]);
-      if (fabs(Con2diff) < 1.e-8) break;
-      if (acc == rattle_max) { atomicOr(&y.status, E_ERR_RATTLE); break; }
-      if (fast) {
-        const double O2 = -(0.5 * (IIM * Con2diff) * kp.iD2);
-        for (int c = 0; c < 3; ++c) {
-          V1[c] = V1[c] + O2 * dd[c] * kp.iMc;
-          V2[c] = V2[c] - O2 * dd[c] * kp.iMn;
-        }
-      } else {
-        const double O = -(0.25 * (IIM * Con2diff) / (Dcn * Dcn));
-        for (int c = 0; c < 3; ++c) {
-          V1[c] = V1[c] + 2.0 * O * dd[c] / Mc;
-          V2[c] = V2[c] - 2.0 * O * dd[c] / Mn;
-        }
-      }
-      acc++;
-    }
-    iters += acc;
-    for (int c = 0; c < 3; ++c) {
-      y.dvel[c] = V1[c]; y.dvel[3 + c] = V2[c];
-      y.dfrc[c] = F1[c]; y.dfrc[3 + c] = F2[c];
-    }
-    const unsigned step = d.g->cstep;
-    if (step % (unsigned)d.mpc_every == 0u) {
-      double dd[3], len2 = 0.;
-      for (int c = 0; c < 3; ++c) { dd[c] = dmi(X1[c] - X2[c], kp.Ld[c]); len2 += dd[c] * dd[c]; }
-      const double len = sqrt(len2);
-      double s = 0.;
-      for (int c = 0; c < 3; ++c) s += ((Mc * V1[c] + Mn * V2[c]) / (Mn + Mc)) * (dd[c] / len);
-      if (d.hist > 0) {
-        const long long k = y.vdot_n;
-        if (k < d.hist)
-          for (int c = 0; c < 3; ++c) d.axes[((size_t)r * d.hist + k) * 3 + c] = (float)(dd[c] / len);
-      }
-      y.vdot_sum += s;
-      y.vdot_n += 1;
-      double u0, u1, u2, u3;
-      contract_pair(kp.seed, TAG_SHIFT, 0, 0, step, u0, u1);
-      contract_pair(kp.seed, TAG_SHIFT, 0, 1, step, u2, u3);
-      y.shift[0] = u0 - 0.5; y.shift[1] = u1 - 0.5; y.shift[2] = u2 - 0.5;
-      for (int c = 0; c < 3; ++c) y.shf[c] = (float)y.shift[c];
-    }
-  }
-  if (mode & M_POS) {
-    const unsigned step = d.g->cstep + 1u;
-    y.time_count += 1;
-    double pr1[3], pr2[3], dP[3];
-    for (int c = 0; c < 3; ++c) { pr1[c] = X1[c]; pr2[c] = X2[c]; dP[c] = dmi(X1[c] - X2[c], kp.Ld[c]); }
-    for (int c = 0; c < 3; ++c) { Q1[c] = V1[c] + hIMc * F1[c]; Q2[c] = V2[c] + hIMn * F2[c]; }
-    for (int c = 0; c < 3; ++c) { X1[c] = X1[c] + dt * Q1[c]; X2[c] = X2[c] + dt * Q2[c]; }
-    if (!fast)
-      for (int c = 0; c < 3; ++c) {
-        X1[c] = X1[c] - kp.Ld[c] * floor(X1[c] / kp.Ld[c]);
-        X2[c] = X2[c] - kp.Ld[c] * floor(X2[c] / kp.Ld[c]);
-      }
-    int acc = 0;
-    for (;;) {
-      double dd[3];
-      for (int c = 0; c < 3; ++c) dd[c] = dmi(X1[c] - X2[c], kp.Ld[c]);
-      const double Con1diff = (dd[0] * dd[0] + dd[1] * dd[1] + dd[2] * dd[2]) - Dcn * Dcn;
-      if (fabs(Con1diff) < 1.e-6) break;
-      if (acc == rattle_max) { atomicOr(&y.status, E_ERR_RATTLE); break; }
-      const double den = dd[0] * dP[0] + dd[1] * dP[1] + dd[2] * dP[2];
-      if (fast) {
-        // the iteration converges to the tolerance whatever the last bits of
-        // G are: a float reciprocal refined twice replaces the division
-        double rr = (double)__frcp_rn((float)den);
-        rr = rr * (2.0 - den * rr);
-        rr = rr * (2.0 - den * rr);
-        const double G2 = 2.0 * (-(0.25 * Con1diff * IIM) * rr);
-        for (int c = 0; c < 3; ++c) {
-          X1[c] = pr1[c] + Q1[c] * dt + G2 * dP[c] * kp.iMc;
-          X2[c] = pr2[c] + Q2[c] * dt - G2 * dP[c] * kp.iMn;
-          Q1[c] = Q1[c] + G2 * dP[c] * kp.iMcdt;
-          Q2[c] = Q2[c] - G2 * dP[c] * kp.iMndt;
-        }
-      } else {
-        const double G = -(0.25 * Con1diff * IIM / den);
-        for (int c = 0; c < 3; ++c) {
-          X1[c] = pr1[c] + Q1[c] * dt + 2.0 * G * dP[c] / Mc;
-          X2[c] = pr2[c] + Q2[c] * dt - 2.0 * G * dP[c] / Mn;
-        }
-        for (int c = 0; c < 3; ++c) {
-          X1[c] = X1[c] - kp.Ld[c] * floor(X1[c] / kp.Ld[c]);
-          X2[c] = X2[c] - kp.Ld[c] * floor(X2[c] / kp.Ld[c]);
-        }
-        for (int c = 0; c < 3; ++c) {
-          Q1[c] = Q1[c] + 2.0 * G * dP[c] / (Mc * dt);
-          Q2[c] = Q2[c] - 2.0 * G * dP[c] / (Mn * dt);
-        }
-      }
-      acc++;
-    }
-    if (fast)
-      for (int c = 0; c < 3; ++c) {
-        const double L = kp.Ld[c];
-        if (X1[c] >= L) X1[c] -= L; else if (X1[c] < 0.0) X1[c] += L;
-        if (X2[c] >= L) X2[c] -= L; else if (X2[c] < 0.0) X2[c] += L;
-        if (!(X1[c] >= 0.0 && X1[c] < L)) X1[c] = X1[c] - L * floor(X1[c] / L);
-        if (!(X2[c] >= 0.0 && X2[c] < L)) X2[c] = X2[c] - L * floor(X2[c] / L);
-      }
-    iters += acc;
-    for (int c = 0; c < 3; ++c) {
-      y.dpos[c] = X1[c]; y.dpos[3 + c] = X2[c];
-      y.dq[c] = Q1[c]; y.dq[3 + c] = Q2[c];
-    }
-    set_srel(y, 0, X1);
-    set_srel(y, 1, X2);
-    const double maxv = __longlong_as_double((long long)y.maxmsd);
-    const double thr = (double)kp.msd_thr;
-    const bool rb = maxv > thr || y.time_count == y.time_penetrate || step % (unsigned)d.mpc_every == 0u;
-    y.maxmsd = 0ull;
-    if (rb) {
-      y.rebuild = 1;
-      y.n_shell = 0;
-      y.maxv2 = 0ull;
-    }
-  }
-  if (iters) y.rattle_iters += iters;
-}
-
-// The FP32 build's dimer step with the three Cartesian components of a
-// replica's dimer on three lanes of a 4-lane group (the fourth lane holds
-// zeros and the replica's scalar work): the update of k_ens_dimer's fast
-// path, with every dot product summed over the group.  At GB300's FP64 rate
-// the per-replica chain of FP64 instructions sets the kernel's time, and the
-// split shortens it about threefold.  The group sums add the same terms in
-// the same order as the one-thread form ((x + y) + (z + 0)).
-template <typename T>
-__global__ void k_ens_dimer_split(EDev<T> d, int mode, int rattle_max) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   const int r = t >> 2, c = t & 3;
   const unsigned gmask = 0xFu << (threadIdx.x & 28);   // this group's four lanes
@@ -827,6 +729,7 @@ __global__ void k_ens_dimer_split(EDev<T> d, int mode, int rattle_max) {
   const double L = kp.Ld[comp ? c : 0];
   const double dt = kp.dtd, Mc = kp.mc, Mn = kp.mn, Dcn = kp.dcn;
   const double hIMc = kp.hIMc, hIMn = kp.hIMn, IIM = kp.IIM;
+  constexpr bool fast = sizeof(T) == 4;
   double X1 = 0., X2 = 0., V1 = 0., V2 = 0., F1 = 0., F2 = 0., Q1 = 0., Q2 = 0.;
   if (live && comp) {
     X1 = y.dpos[c]; X2 = y.dpos[3 + c];
@@ -850,9 +753,15 @@ __global__ void k_ens_dimer_split(EDev<T> d, int mode, int rattle_max) {
       const double Con2diff = 2.0 * group4_sum(gmask, (V1 - V2) * dd);
       if (!live || fabs(Con2diff) < 1.e-8) break;
       if (acc == rattle_max) { if (c == 0) atomicOr(&y.status, E_ERR_RATTLE); break; }
-      const double O2 = -(0.5 * (IIM * Con2diff) * kp.iD2);
-      V1 = V1 + O2 * dd * kp.iMc;
-      V2 = V2 - O2 * dd * kp.iMn;
+      if constexpr (fast) {
+        const double O2 = -(0.5 * (IIM * Con2diff) * kp.iD2);
+        V1 = V1 + O2 * dd * kp.iMc;
+        V2 = V2 - O2 * dd * kp.iMn;
+      } else {
+        const double O = -div_const(0.25 * (IIM * Con2diff), Dcn * Dcn, kp.iD2);
+        V1 = V1 + div_const(2.0 * O * dd, Mc, kp.iMc);
+        V2 = V2 - div_const(2.0 * O * dd, Mn, kp.iMn);
+      }
       acc++;
     }
     iters += acc;
@@ -888,6 +797,7 @@ __global__ void k_ens_dimer_split(EDev<T> d, int mode, int rattle_max) {
     if (comp) {
       Q1 = V1 + hIMc * F1; Q2 = V2 + hIMn * F2;
       X1 = X1 + dt * Q1; X2 = X2 + dt * Q2;
+      if constexpr (!fast) { X1 = wrap_box(X1, L); X2 = wrap_box(X2, L); }
     }
     int acc = 0;
     for (;;) {
@@ -896,24 +806,35 @@ __global__ void k_ens_dimer_split(EDev<T> d, int mode, int rattle_max) {
       if (!live || fabs(Con1diff) < 1.e-6) break;
       if (acc == rattle_max) { if (c == 0) atomicOr(&y.status, E_ERR_RATTLE); break; }
       const double den = group4_sum(gmask, dd * dP);
-      // a float reciprocal refined twice replaces the division (the
-      // iteration converges to the tolerance whatever G's last bits are)
-      double rr = (double)__frcp_rn((float)den);
-      rr = rr * (2.0 - den * rr);
-      rr = rr * (2.0 - den * rr);
-      const double G2 = 2.0 * (-(0.25 * Con1diff * IIM) * rr);
-      X1 = pr1 + Q1 * dt + G2 * dP * kp.iMc;
-      X2 = pr2 + Q2 * dt - G2 * dP * kp.iMn;
-      Q1 = Q1 + G2 * dP * kp.iMcdt;
-      Q2 = Q2 - G2 * dP * kp.iMndt;
+      if constexpr (fast) {
+        // a float reciprocal refined twice replaces the division (the
+        // iteration converges to the tolerance whatever G's last bits are)
+        double rr = (double)__frcp_rn((float)den);
+        rr = rr * (2.0 - den * rr);
+        rr = rr * (2.0 - den * rr);
+        const double G2 = 2.0 * (-(0.25 * Con1diff * IIM) * rr);
+        X1 = pr1 + Q1 * dt + G2 * dP * kp.iMc;
+        X2 = pr2 + Q2 * dt - G2 * dP * kp.iMn;
+        Q1 = Q1 + G2 * dP * kp.iMcdt;
+        Q2 = Q2 - G2 * dP * kp.iMndt;
+      } else {
+        const double G = -(0.25 * Con1diff * IIM / den);
+        X1 = pr1 + Q1 * dt + div_const(2.0 * G * dP, Mc, kp.iMc);
+        X2 = pr2 + Q2 * dt - div_const(2.0 * G * dP, Mn, kp.iMn);
+        if (comp) { X1 = wrap_box(X1, L); X2 = wrap_box(X2, L); }
+        Q1 = Q1 + div_const(2.0 * G * dP, Mc * dt, kp.iMcdt);
+        Q2 = Q2 - div_const(2.0 * G * dP, Mn * dt, kp.iMndt);
+      }
       acc++;
     }
     iters += acc;
     if (live && comp) {
-      if (X1 >= L) X1 -= L; else if (X1 < 0.0) X1 += L;
-      if (X2 >= L) X2 -= L; else if (X2 < 0.0) X2 += L;
-      if (!(X1 >= 0.0 && X1 < L)) X1 = X1 - L * floor(X1 / L);
-      if (!(X2 >= 0.0 && X2 < L)) X2 = X2 - L * floor(X2 / L);
+      if constexpr (fast) {
+        if (X1 >= L) X1 -= L; else if (X1 < 0.0) X1 += L;
+        if (X2 >= L) X2 -= L; else if (X2 < 0.0) X2 += L;
+        X1 = wrap_box(X1, L);
+        X2 = wrap_box(X2, L);
+      }
       y.dpos[c] = X1; y.dpos[3 + c] = X2;
       y.dq[c] = Q1; y.dq[3 + c] = Q2;
       // the sphere positions as cell + offset (set_srel), one axis per lane
@@ -932,6 +853,7 @@ __global__ void k_ens_dimer_split(EDev<T> d, int mode, int rattle_max) {
       const double thr = (double)kp.msd_thr;
       const bool rb = maxv > thr || tc == y.time_penetrate || step % (unsigned)d.mpc_every == 0u;
       y.maxmsd = 0ull;
+      d.rt_need[r] = rb ? rebuild_tiles(d, R) : 0u;
       if (rb) {
         y.rebuild = 1;
         y.n_shell = 0;
@@ -940,6 +862,10 @@ __global__ void k_ens_dimer_split(EDev<T> d, int mode, int rattle_max) {
     }
   }
   if (live && c == 0 && iters) y.rattle_iters += iters;
+  if (mode & M_POS) {
+    __shared__ unsigned part[256];
+    if (last_block(&d.g->arrived[0], gridDim.x)) write_plan(d, part);
+  }
 }
 
 // ------------------------------------------------------------ collision ----

@@ -188,6 +188,7 @@ struct Ensemble : EnsembleBase {
     s |= alloc(scan_tmp, scan_tmp_words(ctot));
     Rep<T>* drep = nullptr; Dyn<T>* ddyn = nullptr; Glob* dg = nullptr;
     s |= alloc(drep, R); s |= alloc(ddyn, R); s |= alloc(dg, 1);
+    s |= alloc(d.st_prefix, R); s |= alloc(d.rt_need, R);
     s |= alloc(d.stile, stot / 32 + R);   // (at least 32 entries in every tile but a replica's last)
     s |= alloc(d.rt_prefix, R + 1);
     s |= alloc(d_mass, 4 * (int64_t)R); s |= alloc(d_obs, 8 * (int64_t)R);
@@ -274,19 +275,16 @@ struct Ensemble : EnsembleBase {
     else k_ens_force<T, M_FORCE | M_ADVANCE><<<g_shell, sblock, 0, st>>>(d);
     ++launches;
   }
-  void L_tiles() { k_ens_tiles<T><<<1, 1024, 0, st>>>(d, sblock); ++launches; }
+  void L_tiles() { k_ens_tiles<T><<<1, 256, 0, st>>>(d, sblock); ++launches; }
   void L_dimer(int mode) {
-    if (sizeof(T) == 4) {
-      // four lanes per replica, one 32-lane block per eight replicas (spread over the SMs)
-      k_ens_dimer_split<T><<<(4 * R + 31) / 32, 32, 0, st>>>(d, mode, rattle_max);
-    } else {
-      k_ens_dimer<T><<<(R + 127) / 128, 128, 0, st>>>(d, mode, rattle_max);
-    }
+    // four lanes per replica; blocks of eight replicas spread over the SMs (of
+    // 64 for thousands of replicas, whose plan one block writes)
+    const int tpb = R <= 2048 ? 32 : 256;
+    k_ens_dimer<T><<<(4 * R + tpb - 1) / tpb, tpb, 0, st>>>(d, mode, rattle_max);
     ++launches;
   }
-  void L_plan() { k_ens_plan<T><<<1, 1024, 0, st>>>(d); ++launches; }
-  void L_rebuild(int mode) { k_ens_rebuild<T><<<g_part, block, 0, st>>>(d, mode); ++launches; }
-  void L_finalize(int adv) { k_ens_finalize<T><<<1, 1024, 0, st>>>(d, sblock, adv); ++launches; }
+  void L_plan() { k_ens_plan<T><<<1, 256, 0, st>>>(d); ++launches; }
+  void L_rebuild(int mode, int adv) { k_ens_rebuild<T><<<g_part, block, 0, st>>>(d, mode, sblock, adv); ++launches; }
   void L_sort() {
     const int g = nsm * 8;
     cudaMemsetAsync(d.scnt, 0, 4 * (size_t)ctot, st);
@@ -316,15 +314,13 @@ struct Ensemble : EnsembleBase {
     if (need_advance) { L_force(M_ADVANCE); need_advance = false; }
     L_dimer((vel_pending ? M_VEL : 0) | M_POS);
     vel_pending = false;
-    L_plan();
     if (sort_step(s)) {
-      L_rebuild(M_LAZY);
+      L_rebuild(M_LAZY, 1);
       L_sort();
-      L_rebuild(M_LISTS);
+      L_rebuild(M_LISTS, 0);
     } else {
-      L_rebuild(M_LAZY | M_LISTS);
+      L_rebuild(M_LAZY | M_LISTS, 1);
     }
-    L_finalize(1);
     if (mpc) {
       L_force(M_FORCE);
       L_dimer(M_VEL);
@@ -537,8 +533,7 @@ struct Ensemble : EnsembleBase {
     ECK(cudaMemcpyAsync(d.g, &g, sizeof(g), cudaMemcpyHostToDevice, st));
     if (sort_step(cstep)) L_sort();
     L_plan();
-    L_rebuild(M_LISTS);
-    L_finalize(0);
+    L_rebuild(M_LISTS, 0);
     need_advance = true;
     vel_pending = false;
     prepared = true;
