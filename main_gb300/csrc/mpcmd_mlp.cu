@@ -3,31 +3,37 @@
 // outputs) trained and evaluated by this file's own kernels on the
 // fifth-generation tensor cores of sm_103a.
 //
-// Inference is one kernel, k_infer: a CTA takes 128 input rows through every
-// layer, the hidden activations staying in shared memory.
+// k_chain takes 128 rows of a batch through every layer in one CTA, the
+// activations staying in tensor memory.  Inference is one launch of it; a
+// training step is four launches:
+//   k_chain<FORWARD>   the same pass, which also keeps the pre-activations and
+//                      the transposed activations, and ends in the loss and the
+//                      output gradient instead of the outputs;
+//   k_dx               the gradient of the last hidden layer, the one
+//                      contraction over the wide output layer (K = n_out), its
+//                      columns spread over CTAs;
+//   k_chain<BACKWARD>  the gradients of the other hidden layers, layer after
+//                      layer on chip;
+//   k_dw               every layer's weight and bias gradients, which no longer
+//                      depend on one another, with Adam in the epilogue.
+// (A step of 256 rows through four hidden layers of 256 to 2,050 outputs: 87 us
+// a call, about 60 of them kernels, where 31 launches through memory took 305.
+// All of it is latency: a contraction's MMAs wait for one another.)
+// Every contraction is C[M, N] = A[M, K] . B[N, K]^T with both operands BF16
+// and K-major.
 //
-// Training contractions (forward, input gradient, weight gradient) are one
-// GEMM form, C[M, N] = A[M, K] . B[N, K]^T with A and B BF16 and K-major, and
-// one persistent kernel, k_gemm, with one CTA per SM walking its share of the
-// 128 x BN output tiles.
-//
-// Warp roles of both: one thread streams tiles into a ring of shared-memory
-// stages with TMA (cp.async.bulk.tensor, 128-byte swizzle, mbarriers); one
-// thread issues tcgen05.mma (kind::f16, BF16 operands, FP32 accumulator in
-// tensor memory) and releases each stage with tcgen05.commit; the epilogue
-// warps read the accumulator back with tcgen05.ld (a warp reaches the 32 TMEM
-// lanes of its quarter; the warps of a quarter take its 32-column chunks in
-// turn) and apply the fused epilogue: bias + SiLU with the pre-activation kept
-// for the backward pass (forward hidden), bias (output), SiLU' of the kept
-// pre-activation (input gradient), or the FP32 weight gradient.  Two
-// accumulators in tensor memory let the epilogue of one tile overlap the loads
-// and MMAs of the next.  Row-major outputs go through a per-warp 32-row
-// staging tile in shared memory so that every store writes whole rows; the
-// forms that the next GEMM needs transposed are written from the
-// thread-per-row layout, so that every operand stays K-major.  Every mbarrier
-// wait is bounded (two seconds of globaltimer): on expiry the kernel raises an
-// error flag, skips its remaining work, waits for its copies and MMAs in
-// flight and still frees its tensor memory.
+// Warp roles of all three: one thread streams tiles into a ring of
+// shared-memory stages with TMA (cp.async.bulk.tensor, 128-byte swizzle,
+// mbarriers); one thread issues tcgen05.mma (kind::f16, BF16 operands, FP32
+// accumulator in tensor memory) and releases each stage with tcgen05.commit;
+// the epilogue warps read the accumulator back with tcgen05.ld (a warp reaches
+// the 32 TMEM lanes of its quarter, a lane holds a row) and apply the fused
+// epilogue.  What the next GEMM needs transposed is written from that
+// thread-per-row layout, consecutive lanes to consecutive rows, so that every
+// operand stays K-major; the pre-activations are kept transposed for the same
+// reason.  Every mbarrier wait is bounded (two seconds of globaltimer): on
+// expiry the kernel raises an error flag, skips its remaining work, waits for
+// its copies and MMAs in flight and still frees its tensor memory.
 //
 // Weights are kept in FP32 (master copy for Adam) and in BF16 twice: [N, K]
 // for the forward GEMM and [K, N] for the input-gradient GEMM.
@@ -42,49 +48,14 @@
 #include <vector>
 
 #include "mpcmd.h"
+#include "mpcmd_device.cuh"   // PairSum
 
 namespace {
 
+using mpcmd::PairSum;
+
 constexpr int BM = 128;        // output rows per tile (the MMA's M)
 constexpr int BK = 64;         // K per stage: one 128-byte swizzle row of BF16
-constexpr int EPI_WARPS = 16;                 // four per TMEM lane quarter
-constexpr int THREADS = 64 + 32 * EPI_WARPS;   // producer warp, MMA warp, epilogue warps
-constexpr int A_STAGE = BM * BK * 2;   // 16 KiB
-
-enum Epilogue : int { EP_HIDDEN = 0, EP_OUT = 2, EP_DX = 3, EP_DW = 4 };
-
-// Words per row of the epilogue staging tile: 36 where a mode writes FP32
-// rows, 20 where it writes BF16 rows only (16-byte rows, conflict-free
-// quarter warps either way).
-template <int MODE>
-__host__ __device__ constexpr int stage_pitch() {
-  return MODE == EP_DX ? 20 : 36;
-}
-template <int BN>
-__host__ __device__ constexpr int ring_box() { return A_STAGE + BN * BK * 2; }
-template <int BN, int MODE>
-__host__ __device__ constexpr int stages() {
-  // as many ring stages (at most 4) as fit beside the staging tiles in 227 KB
-  return (232448 - 1024 - 512 - EPI_WARPS * 32 * stage_pitch<MODE>() * 4) / ring_box<BN>() >= 4
-             ? 4
-             : (232448 - 1024 - 512 - EPI_WARPS * 32 * stage_pitch<MODE>() * 4) / ring_box<BN>();
-}
-
-struct GemmArgs {
-  int M, N, K;              // C[M, N] = A[M, K] . B[N, K]^T, multiples of 128 / BN / 64
-  int mode;
-  int m_valid, n_valid;     // rows / columns of the output that are stored
-  float* out_f32;           // EP_OUT: y [m_valid, ldo]; EP_DW: gradient [M, ldo]
-  int ldo;
-  __nv_bfloat16* out_bf16;  // EP_HIDDEN, EP_DX: [M, ldb]
-  int ldb;
-  __nv_bfloat16* out_t;     // EP_HIDDEN, EP_DX: transposed [N, ldt]
-  int ldt;
-  const float* bias;        // EP_HIDDEN, EP_OUT: [N]
-  float* z;                 // EP_HIDDEN: pre-activation written; EP_DX: read; [M, ldz]
-  int ldz;
-  int* err;
-};
 
 // ------------------------------------------------------------ PTX ----
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
@@ -206,6 +177,17 @@ __device__ __forceinline__ void mma_commit(uint32_t bar) {
 __device__ __forceinline__ void tmem_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tmem_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 // A 32 x 32 block of the accumulator (lane = row, values = columns).
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
+  uint32_t u[16];
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n\t"
+      "tcgen05.wait::ld.sync.aligned;"
+      : "=r"(u[0]), "=r"(u[1]), "=r"(u[2]), "=r"(u[3]), "=r"(u[4]), "=r"(u[5]), "=r"(u[6]), "=r"(u[7]), "=r"(u[8]),
+        "=r"(u[9]), "=r"(u[10]), "=r"(u[11]), "=r"(u[12]), "=r"(u[13]), "=r"(u[14]), "=r"(u[15])
+      : "r"(taddr));
+#pragma unroll
+  for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(u[i]);
+}
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32]) {
   uint32_t r[32];
   asm volatile(
@@ -285,225 +267,9 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
   return *reinterpret_cast<const uint32_t*>(&p);
 }
 
-// Epilogue of a warp's 32 x 32 block: rows row0.. (this thread: row0 +
-// lane), columns n..n+31, accumulators v[] in the tcgen05.ld 32x32b layout
-// (lane = row, registers = consecutive columns).  The arithmetic runs in that
-// layout; row-major outputs leave through store_rows, the transposed copies
-// as one BF16 per lane and column (consecutive lanes = consecutive rows).
-// bias: the 32 columns' biases (16-byte aligned, read four at a time, the same
-// address in every lane).
-template <int MODE>
-__device__ __forceinline__ void epilogue_chunk(const GemmArgs& a, const float* bias, uint32_t* buf,
-                                               const float (&v)[32], int row0, int n, int rows, int lane) {
-  const int m = row0 + lane;
-  const bool row_ok = lane < rows;
-  const float4* bp = reinterpret_cast<const float4*>(bias);
-  if constexpr (MODE == EP_HIDDEN) {
-      uint32_t zw[32], hw[16];
-#pragma unroll
-      for (int q = 0; q < 32; q += 4) {
-        const float4 b4 = bp[q / 4];
-        zw[q] = __float_as_uint(v[q] + b4.x); zw[q + 1] = __float_as_uint(v[q + 1] + b4.y);
-        zw[q + 2] = __float_as_uint(v[q + 2] + b4.z); zw[q + 3] = __float_as_uint(v[q + 3] + b4.w);
-      }
-      store_rows<32, 16, stage_pitch<MODE>()>(buf, zw, lane, reinterpret_cast<char*>(a.z + n), row0,
-                                              (size_t)a.ldz * 4, rows);
-#pragma unroll
-      for (int q = 0; q < 16; ++q)
-        hw[q] = pack_bf16(silu_f(__uint_as_float(zw[2 * q])), silu_f(__uint_as_float(zw[2 * q + 1])));
-      if (row_ok) {
-        const __nv_bfloat16* h = reinterpret_cast<const __nv_bfloat16*>(hw);
-#pragma unroll
-        for (int q = 0; q < 32; ++q) a.out_t[(size_t)(n + q) * a.ldt + m] = h[q];
-      }
-      store_rows<16, 16, stage_pitch<MODE>()>(buf, hw, lane, reinterpret_cast<char*>(a.out_bf16 + n), row0,
-                                              (size_t)a.ldb * 2, rows);
-  } else if constexpr (MODE == EP_OUT) {
-      uint32_t yw[32];
-#pragma unroll
-      for (int q = 0; q < 32; q += 4) {
-        const float4 b4 = bp[q / 4];
-        yw[q] = __float_as_uint(v[q] + b4.x); yw[q + 1] = __float_as_uint(v[q + 1] + b4.y);
-        yw[q + 2] = __float_as_uint(v[q + 2] + b4.z); yw[q + 3] = __float_as_uint(v[q + 3] + b4.w);
-      }
-      // y rows have the caller's pitch: pieces as wide as its alignment allows
-      const int wlim = a.n_valid - n < 32 ? a.n_valid - n : 32;
-      char* yb = reinterpret_cast<char*>(a.out_f32 + n);
-      constexpr int P = stage_pitch<MODE>();
-      if ((a.ldo & 3) == 0) store_rows<32, 16, P>(buf, yw, lane, yb, row0, (size_t)a.ldo * 4, rows, wlim);
-      else if ((a.ldo & 1) == 0) store_rows<32, 8, P>(buf, yw, lane, yb, row0, (size_t)a.ldo * 4, rows, wlim);
-      else store_rows<32, 4, P>(buf, yw, lane, yb, row0, (size_t)a.ldo * 4, rows, wlim);
-  } else if constexpr (MODE == EP_DW) {
-      uint32_t gw[32];
-#pragma unroll
-      for (int q = 0; q < 32; ++q) gw[q] = __float_as_uint(v[q]);
-      store_rows<32, 16, stage_pitch<MODE>()>(buf, gw, lane, reinterpret_cast<char*>(a.out_f32 + n), row0,
-                                              (size_t)a.ldo * 4, rows);
-  } else if constexpr (MODE == EP_DX) {
-      uint32_t gw[16];
-      if (row_ok) {
-        const float4* zp = reinterpret_cast<const float4*>(a.z + (size_t)m * a.ldz + n);
-#pragma unroll
-        for (int q = 0; q < 8; ++q) {
-          const float4 z4 = zp[q];
-          gw[2 * q] = pack_bf16(v[4 * q] * dsilu_f(z4.x), v[4 * q + 1] * dsilu_f(z4.y));
-          gw[2 * q + 1] = pack_bf16(v[4 * q + 2] * dsilu_f(z4.z), v[4 * q + 3] * dsilu_f(z4.w));
-        }
-        const __nv_bfloat16* g = reinterpret_cast<const __nv_bfloat16*>(gw);
-#pragma unroll
-        for (int q = 0; q < 32; ++q) a.out_t[(size_t)(n + q) * a.ldt + m] = g[q];
-      } else {
-#pragma unroll
-        for (int q = 0; q < 16; ++q) gw[q] = 0u;
-      }
-      store_rows<16, 16, stage_pitch<MODE>()>(buf, gw, lane, reinterpret_cast<char*>(a.out_bf16 + n), row0,
-                                              (size_t)a.ldb * 2, rows);
-  }
-}
-
-// ------------------------------------------------------------ GEMM ----
-template <int BN, int MODE>
-__host__ __device__ constexpr size_t gemm_smem_bytes() {
-  return 1024 + (size_t)stages<BN, MODE>() * ring_box<BN>() + (size_t)EPI_WARPS * 32 * stage_pitch<MODE>() * 4 +
-         (2 * stages<BN, MODE>() + 5) * 8 + 16;
-}
-
-template <int BN, int MODE>
-__global__ void __launch_bounds__(THREADS, 1)
-    k_gemm(const __grid_constant__ CUtensorMap ta, const __grid_constant__ CUtensorMap tb, GemmArgs a) {
-  constexpr int S = stages<BN, MODE>();
-  constexpr int SBOX = ring_box<BN>();
-  constexpr int P = stage_pitch<MODE>();
-  static_assert(S >= 2 && gemm_smem_bytes<BN, MODE>() <= 232448, "shared memory of one CTA");
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-  uint8_t* sRing = smem;                                                        // stage ring
-  uint32_t* stage_all = reinterpret_cast<uint32_t*>(sRing + S * SBOX);
-  uint64_t* bars = reinterpret_cast<uint64_t*>(stage_all + EPI_WARPS * 32 * P);
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * S + 5);
-  __shared__ volatile int bail;        // a wait of this CTA expired
-  __shared__ int issued;               // stage loads the producer issued
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int tiles_n = a.N / BN, tiles_m = (a.M + BM - 1) / BM;
-  const int units = tiles_m * tiles_n;
-  const int nk = a.K / BK;
-  const int mlim = (MODE == EP_OUT || MODE == EP_DW) ? a.m_valid : a.M;
-  // barriers: full[S], empty[S] (ring), accf[2], acce[2] (accumulators), done
-  const uint32_t full0 = smem_u32(bars), empty0 = smem_u32(bars + S), accf0 = smem_u32(bars + 2 * S),
-                 acce0 = smem_u32(bars + 2 * S + 2), done = smem_u32(bars + 2 * S + 4);
-
-  if (threadIdx.x == 0) {
-    bail = 0;
-    issued = 0;
-    for (int s = 0; s < S; ++s) {
-      mbar_init(full0 + 8 * s, 1);
-      mbar_init(empty0 + 8 * s, 1);
-    }
-    for (int b = 0; b < 2; ++b) {
-      mbar_init(accf0 + 8 * b, 1);
-      mbar_init(acce0 + 8 * b, EPI_WARPS);
-    }
-    mbar_init(done, 1);
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-  }
-  if (warp == 1) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
-                 "r"(2 * BN)
-                 : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-  }
-  tmem_fence_before();
-  __syncthreads();
-  tmem_fence_after();
-  const uint32_t tmem = *tmem_slot;
-
-  if (warp == 0) {
-    if (lane == 0) {
-      // TMA producer
-      int g = 0;
-      for (int u = blockIdx.x; u < units && !bail; u += gridDim.x) {
-        const int mt = u / tiles_n, nt = u % tiles_n;
-        for (int k = 0; k < nk; ++k) {
-          const int s = g % S;
-          if (g >= S && !mbar_wait(empty0 + 8 * s, ((uint32_t)(g / S) & 1u) ^ 1u, a.err)) { bail = 1; break; }
-          mbar_expect_tx(full0 + 8 * s, SBOX);
-          uint8_t* st = sRing + s * SBOX;
-          tma_load_2d(smem_u32(st), &ta, full0 + 8 * s, k * BK, mt * BM);
-          tma_load_2d(smem_u32(st + A_STAGE), &tb, full0 + 8 * s, k * BK, nt * BN);
-          ++g;
-        }
-      }
-      issued = g;
-    }
-  } else if (warp == 1) {
-    if (lane == 0) {
-      // MMA issuer: tile j accumulates into buffer j & 1
-      constexpr uint32_t idesc = f16_idesc(BM, BN);
-      int g = 0, j = 0;
-      bool ok = true;
-      for (int u = blockIdx.x; u < units && ok && !bail; u += gridDim.x, ++j) {
-        const int b = j & 1;
-        if (j >= 2 && !mbar_wait(acce0 + 8 * b, ((uint32_t)(j >> 1) & 1u) ^ 1u, a.err)) { ok = false; bail = 1; break; }
-        tmem_fence_after();
-        const uint32_t acc = tmem + (uint32_t)(b * BN);
-        for (int k = 0; k < nk; ++k, ++g) {
-          const int s = g % S;
-          if (!mbar_wait(full0 + 8 * s, (uint32_t)(g / S) & 1u, a.err)) { ok = false; bail = 1; break; }
-          tmem_fence_after();
-          const uint32_t a0 = smem_u32(sRing + s * SBOX), b0 = a0 + A_STAGE;
-#pragma unroll
-          for (int kk = 0; kk < BK / 16; ++kk)
-            mma_bf16(acc, sw128_desc(a0 + 32 * kk), sw128_desc(b0 + 32 * kk), idesc, (k > 0 || kk > 0) ? 1u : 0u);
-          mma_commit(empty0 + 8 * s);
-        }
-        if (!ok) break;
-        mma_commit(accf0 + 8 * b);   // arrives when the tile's MMAs have completed
-      }
-      mma_commit(done);   // arrives when every MMA issued above has completed
-    }
-  } else {
-    // epilogue: warp w reaches TMEM lanes 32 (w % 4) ..; the warps of a
-    // quarter take its 32-column chunks in turn
-    const int ew = warp - 2;
-    const int quarter = warp & 3;
-    constexpr int GROUPS = EPI_WARPS / 4;
-    uint32_t* buf = stage_all + ew * 32 * P;
-    int j = 0;
-    for (int u = blockIdx.x; u < units; u += gridDim.x, ++j) {
-      const int b = j & 1;
-      if (!mbar_wait(accf0 + 8 * b, (uint32_t)(j >> 1) & 1u, a.err)) { bail = 1; break; }
-      tmem_fence_after();
-      const int row0 = (u / tiles_n) * BM + quarter * 32, n0 = (u % tiles_n) * BN;
-      const int rows = mlim - row0 < 32 ? mlim - row0 : 32;
-      for (int c0 = (ew >> 2) * 32; c0 < BN; c0 += 32 * GROUPS) {
-        float v[32];
-        tmem_ld32(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(b * BN + c0), v);
-        epilogue_chunk<MODE>(a, a.bias + n0 + c0, buf, v, row0, n0 + c0, rows, lane);
-      }
-      tmem_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(acce0 + 8 * b);
-    }
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    // every MMA has completed, and so has every load that was issued (the
-    // most recent phase of each stage; on the normal path all were consumed),
-    // before the tensor memory is freed and the CTA exits
-    mbar_wait(done, 0, a.err);
-    const int g1 = issued;
-    for (int g = g1 - S < 0 ? 0 : g1 - S; g < g1; ++g) mbar_wait(full0 + 8 * (g % S), (uint32_t)(g / S) & 1u, a.err);
-  }
-  tmem_fence_before();
-  __syncthreads();
-  tmem_fence_after();
-  if (warp == 1)
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2 * BN) : "memory");
-}
-
-// ------------------------------------------------------- inference ----
-// The whole forward pass of 128 rows in one CTA.  Bound by the FP32 output it
+// ------------------------------------------------- chain of layers ----
+// The layers of 128 rows in one CTA; the modes share everything but what enters
+// the chain, what an epilogue computes and where it goes.  Bound by the FP32 output it
 // writes (n_out values a row, 537 MB for the surrogate's 65,536 points, 81 us
 // at the measured HBM rate) and the weights it streams from L2 for large calls,
 // and by the chain of layers for small ones, so:
@@ -527,8 +293,8 @@ __global__ void __launch_bounds__(THREADS, 1)
 //     of CTAs by output columns, each repeating the (much cheaper) hidden
 //     layers: with fewer row tiles than SMs all of them, else the last partial
 //     wave.
-// One launch instead of six (one conversion and five GEMMs with the activations
-// through L2): with the call's own cost, 64 points take 43 us against 80, 65,536
+// Inference: one launch instead of six (one conversion and five GEMMs with the
+// activations through L2): with the call's own cost, 64 points take 43 us against 80, 65,536
 // points 196 against 283.  A hidden layer takes 3 us (1 us of MMAs, then its
 // epilogue, then the next: a chain), 256 output columns of 128 rows 4.4 us.
 constexpr int INF_GROUPS = 3;                      // epilogue groups of four warps
@@ -543,13 +309,15 @@ constexpr int INF_CHUNKS = 4;                      // 32-column chunks of a warp
 constexpr int MAX_HIDDEN = 16;                     // hidden layers of a configuration
 constexpr uint32_t TM_ACC = 128;                   // first accumulator column (A before it)
 
+enum ChainMode : int { INFER = 0, FORWARD = 1, BACKWARD = 2 };
+
 struct InferMaps {             // (boxes of half the rows: one CTA's share)
   CUtensorMap w[MAX_HIDDEN];   // hidden layer l: 64 x H
   CUtensorMap out, tail;       // output layer: 64 x 128 and 64 x tail_n
 };
 struct InferArgs {
-  int layers, H, n_in, rows;
-  int tiles;            // output jobs per row tile
+  int layers, H, n_in, rows;   // layers of the chain (BACKWARD: all hidden ones but the last)
+  int tiles;            // output jobs per row tile (BACKWARD: none)
   int tail_n;           // width of the last output job (a multiple of 16)
   int whole, part, split;   // rounds of whole row-tile pairs; pairs left over, each split this many ways
   int n_out;
@@ -557,6 +325,19 @@ struct InferArgs {
   const float* bias[MAX_HIDDEN];
   const float* bias_out;
   float* y;             // [rows, n_out]
+  // Training.  FORWARD keeps x^T [64, rows], the pre-activations [H, rows] and
+  // the activations [H, rows] of every layer and writes the output gradient as
+  // [rows, npad] and [npad, rows]; BACKWARD takes the last hidden layer's
+  // gradient [rows, H] and writes those of the layers below, [H, rows], last
+  // first (zt and at in the same order).
+  const float *t, *w;   // targets [rows, n_out], output weights [n_out]
+  float inv_rows;       // 1 / rows where that is exact, else 0
+  int npad;
+  float* zt[MAX_HIDDEN];
+  __nv_bfloat16* at[MAX_HIDDEN];
+  __nv_bfloat16 *xt, *dy, *dyt;
+  const __nv_bfloat16* dz;
+  double* loss;         // [CTAs * INF_EPI] partial sums of w (y - t)^2
   int* err;
 };
 
@@ -575,6 +356,39 @@ __device__ __forceinline__ bool infer_item(const InferArgs& a, int v, int& mt, i
   t0 = a.tiles * q / a.split;
   t1 = a.tiles * (q + 1) / a.split;
   return true;
+}
+
+// Whether this CTA keeps piece i of what a training pass keeps (32 columns of
+// a layer, counted through the layers): the CTAs that share a row tile all
+// compute its layers, and take turns in writing them.
+__device__ __forceinline__ bool keeps(const InferArgs& a, int v, int i) {
+  return v < a.whole || i % a.split == ((int)blockIdx.x >> 1) % a.split;
+}
+
+// 4 or 16 bytes to shared memory (this thread sees them after cp.async.wait_all).
+template <int N>
+__device__ __forceinline__ void copy_async(void* dst, const void* src) {
+  if constexpr (N == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+  else asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+
+// A training step's kernels are launched early (programmatic dependent launch):
+// a kernel lets the next one start once it holds its tensor memory, and the next
+// one sets itself up, then waits until the kernel before it has ended with its
+// results visible.
+__device__ __forceinline__ void let_next_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// Consecutive columns of a lane's row, packed in pairs, as a column each of a
+// transposed matrix (consecutive lanes: consecutive rows).
+template <int N>
+__device__ __forceinline__ void put_columns(__nv_bfloat16* dst, size_t ld, const uint32_t (&w)[N]) {
+  unsigned short* d = reinterpret_cast<unsigned short*>(dst);
+#pragma unroll
+  for (int q = 0; q < N; ++q) {
+    d[(size_t)(2 * q) * ld] = (unsigned short)(w[q] & 0xFFFFu);
+    d[(size_t)(2 * q + 1) * ld] = (unsigned short)(w[q] >> 16);
+  }
 }
 
 // A 32-row block of y of INF_WIDE columns through the warp's staging tile: the
@@ -618,10 +432,11 @@ __device__ __forceinline__ void store_block(const uint32_t* buf, int lane, char*
   }
 }
 
-// VB: the largest of 16, 8 and 4 bytes that divides the address of every row of y
-template <int VB>
+// VB (INFER): the largest of 16, 8 and 4 bytes that divides the address of
+// every row of y
+template <int MODE, int VB>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(INF_THREADS, 1)
-    k_infer(const __grid_constant__ InferMaps maps, const __grid_constant__ InferArgs a) {
+    k_chain(const __grid_constant__ InferMaps maps, const __grid_constant__ InferArgs a) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* sRing = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   uint32_t* stage_all = reinterpret_cast<uint32_t*>(sRing + INF_STAGES * INF_STAGE);
@@ -631,7 +446,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(INF_THREADS, 1)
   __shared__ volatile int bail;   // a wait of this CTA expired
   __shared__ int issued;          // stages the producer filled
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int nkh = a.H / BK;
+  const int nkh = a.H / BK, nk0 = MODE == BACKWARD ? nkh : 1;   // K boxes of a layer, of the first
   // barriers: full, empty (ring), accf, acce (output accumulators), hacc (a
   // hidden layer's MMAs have completed), hready (the A operand of the next
   // layer is written and the accumulator read), done
@@ -642,7 +457,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(INF_THREADS, 1)
     issued = 0;
     // (a stage is free when both CTAs' MMAs have read it: either may write it)
     for (int s = 0; s < INF_STAGES; ++s) { mbar_init(full0 + 8 * s, 1); mbar_init(empty0 + 8 * s, 2); }
-    for (int b = 0; b < INF_GROUPS; ++b) { mbar_init(accf0 + 8 * b, 1); mbar_init(acce0 + 8 * b, 4); }
+    for (int b = 0; b < INF_GROUPS; ++b) { mbar_init(accf0 + 8 * b, 1); mbar_init(acce0 + 8 * b, MODE == FORWARD ? INF_EPI : 4); }
     mbar_init(hacc, 1);
     mbar_init(hready, INF_EPI);
     mbar_init(done, 1);
@@ -660,6 +475,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(INF_THREADS, 1)
   cluster_sync();   // both CTAs' barriers exist before either signals them
   tmem_fence_after();
   const uint32_t tmem = *tmem_slot;
+  if constexpr (MODE != INFER) let_next_start();
+  if constexpr (MODE == BACKWARD) wait_for_previous();
 
   if (warp == 0) {
     if (lane == 0) {
@@ -684,7 +501,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(INF_THREADS, 1)
       bool ok = true;
       for (int v = 0; ok && !bail && infer_item(a, v, mt, t0, t1); ++v) {
         for (int l = 0; l < a.layers && ok; ++l)
-          for (int k = 0; k < (l == 0 ? 1 : nkh) && ok; ++k) ok = fill(&maps.w[l], k, 1, 0, a.H);
+          for (int k = 0; k < (l == 0 ? nk0 : nkh) && ok; ++k) ok = fill(&maps.w[l], k, 1, 0, a.H);
         for (int t = t0; t < t1 && ok; ++t) {
           const bool tail = t == a.tiles - 1;
           for (int k = 0; k < nkh && ok; k += 2)
@@ -729,7 +546,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(INF_THREADS, 1)
         for (int l = 0; l < a.layers && ok; ++l) {
           if (!(ok = wait(hready, (uint32_t)hp++ & 1u))) break;
           tmem_fence_after();
-          for (int k = 0; k < (l == 0 ? 1 : nkh) && ok; ++k) ok = stage(tmem + TM_ACC, hid, k, 1);
+          for (int k = 0; k < (l == 0 ? nk0 : nkh) && ok; ++k) ok = stage(tmem + TM_ACC, hid, k, 1);
           if (ok) mma_commit(hacc);
         }
         if (ok) ok = wait(hready, (uint32_t)hp++ & 1u);
@@ -752,16 +569,45 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(INF_THREADS, 1)
     uint32_t* buf = stage_all + ew * 32 * INF_PITCH;
     const uint32_t lanes = tmem + ((uint32_t)(quarter * 32) << 16);
     // A's columns and the reads of the accumulator before it are done
+    int published = 0;
     auto publish = [&]() {
       tmem_wait_st();
       tmem_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(hready);
+      ++published;
     };
-    // the input rows: 64 columns of K (zero-padded), 32 by each of two groups
-    auto load_input = [&](int mt) {
-      if (group < 2) {
-        const int64_t row = (int64_t)mt * BM + quarter * 32 + lane;
+    // what enters the chain: the input rows as 64 columns of K (zero-padded),
+    // 32 by each of two groups, or the rows of a gradient
+    auto load_input = [&](int mt, bool keep) {
+      const int64_t row = (int64_t)mt * BM + quarter * 32 + lane;
+      if constexpr (MODE == BACKWARD) {
+        // Through the staging tile, four lanes to a row's 64 bytes (a lane per row
+        // costs 32 lines an instruction: 3 us).
+        constexpr int P = 16 * (INF_CHUNKS - 1) + 4;
+        const int64_t r0 = (int64_t)mt * BM + quarter * 32 + (lane >> 2);
+#pragma unroll
+        for (int i = 0; i < INF_CHUNKS - 1; ++i) {
+          const int c0 = 32 * (group + INF_GROUPS * i) + 8 * (lane & 3);
+#pragma unroll
+          for (int q = 0; q < 32; q += 8)
+            if (c0 < a.H && r0 + q < a.rows)
+              copy_async<16>(buf + ((lane >> 2) + q) * P + 16 * i + 4 * (lane & 3), a.dz + (r0 + q) * a.H + c0);
+        }
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        __syncwarp();
+#pragma unroll
+        for (int i = 0; i < INF_CHUNKS - 1; ++i) {
+          uint32_t w[16];
+#pragma unroll
+          for (int q = 0; q < 16; q += 4) {
+            const uint4 v = *reinterpret_cast<const uint4*>(buf + lane * P + 16 * i + q);
+            w[q] = v.x; w[q + 1] = v.y; w[q + 2] = v.z; w[q + 3] = v.w;
+          }
+          if (32 * (group + INF_GROUPS * i) < a.H) tmem_st16(lanes + (uint32_t)(16 * (group + INF_GROUPS * i)), w);
+        }
+        __syncwarp();
+      } else if (group < 2) {
         const float* xr = a.x + row * a.n_in;
         const int have = row < a.rows ? a.n_in : 0;
         uint32_t w[16];
@@ -771,6 +617,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(INF_THREADS, 1)
           w[q] = pack_bf16(c < have ? xr[c] : 0.f, c + 1 < have ? xr[c + 1] : 0.f);
         }
         tmem_st16(lanes + (uint32_t)(16 * group), w);
+        if (MODE == FORWARD && keep && row < a.rows) put_columns(a.xt + (size_t)(32 * group) * a.rows + row, a.rows, w);
       }
       publish();
     };
@@ -783,7 +630,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(INF_THREADS, 1)
 #pragma unroll
       for (int i = 0; i < INF_CHUNKS; ++i) {
         const int c = 32 * (group + INF_GROUPS * i) + lane;
-        ahead[i] = c < a.H ? a.bias[l][c] : 0.f;
+        ahead[i] = MODE != BACKWARD && c < a.H ? a.bias[l][c] : 0.f;
       }
     };
     auto fetch_out = [&](int t) {
@@ -807,55 +654,155 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(INF_THREADS, 1)
     const size_t pitch = (size_t)a.n_out * 4;
     int o = 0, h = 0, mt, t0, t1;
     bool ok = infer_item(a, 0, mt, t0, t1);
-    if (ok) { load_input(mt); fetch_hidden(0); }
+    if (ok) { load_input(mt, keeps(a, 0, a.layers * a.H / 32)); fetch_hidden(0); }
+    double loss = 0.;
+    // FORWARD: this warp's 32 target rows of a job's columns into its staging
+    // tile, its chunks side by side
+    auto load_targets = [&](int row0, int rows, int t) {
+#pragma unroll 1
+      for (int r0 = 0; r0 < 32; r0 += 16) {
+        float v[32];   // 32 loads in flight
+#pragma unroll
+        for (int i = 0; i < 32; ++i) {
+          const int r = r0 + (i >> 1), c = 32 * (group + INF_GROUPS * (i & 1)) + lane, col = t * INF_BN + c;
+          v[i] = r < rows && c < INF_BN && col < a.n_out ? a.t[(int64_t)(row0 + r) * a.n_out + col] : 0.f;
+        }
+#pragma unroll
+        for (int i = 0; i < 32; ++i)
+          reinterpret_cast<float*>(buf)[(r0 + (i >> 1)) * INF_PITCH + 32 * (i & 1) + lane] = v[i];
+      }
+      __syncwarp();
+    };
     for (int v = 0; ok; ++v) {
-      // this group's first output job of the item
-      const int first = t0 + (group - o % 3 + 3) % 3;
+      const int64_t row = (int64_t)mt * BM + quarter * 32 + lane;
+      const int row0 = mt * BM + quarter * 32;
+      const int rows = a.rows - row0 < 32 ? a.rows - row0 : 32;
+      // this group's first output job of the item (FORWARD: the groups share every
+      // job, a training batch leaves a CTA one or two)
+      const int first = MODE == FORWARD ? t0 : t0 + (group - o % 3 + 3) % 3;
+      constexpr int stride = MODE == FORWARD ? 1 : 3;
+      if (MODE == FORWARD) load_targets(row0, rows, first);
       for (int l = 0; l < a.layers && ok; ++l, ++h) {
         put_bias();
         if (l + 1 < a.layers) fetch_hidden(l + 1);
         else if (first < t1) fetch_out(first);
+        // BACKWARD: this warp's pre-activations arrive while the MMAs run, the
+        // first chunk's in registers
+        float z0[MODE == BACKWARD ? 32 : 1];
+        if constexpr (MODE == BACKWARD) {
+          const bool real = row < a.rows;
+          const float* zp = a.zt[l] + (real ? row : 0);
+#pragma unroll
+          for (int i = 1; i < INF_CHUNKS - 1; ++i) {
+            const int c0 = 32 * (group + INF_GROUPS * i);
+            if (c0 < a.H)
+#pragma unroll
+              for (int q = 0; q < 32; ++q)
+                copy_async<4>(buf + (32 * (i - 1) + q) * 32 + lane, zp + (size_t)(c0 + q) * a.rows);
+          }
+          if (32 * group < a.H)
+#pragma unroll
+            for (int q = 0; q < 32; ++q) z0[q] = zp[(size_t)(32 * group + q) * a.rows];
+          asm volatile("cp.async.wait_all;" ::: "memory");
+        }
         if (!(ok = wait(hacc, (uint32_t)h & 1u))) break;
         int i = 0;
 #pragma unroll 1
         for (int c0 = 32 * group; c0 < a.H; c0 += 32 * INF_GROUPS, ++i) {
           float z[32];
+          const bool keep = MODE != INFER && row < a.rows && keeps(a, v, (l * a.H + c0) / 32);
           tmem_ld32(lanes + TM_ACC + (uint32_t)c0, z);
-          const float4* bp = reinterpret_cast<const float4*>(bias + 32 * i);
           uint32_t w[16];
+          if constexpr (MODE == BACKWARD) {
+            // through SiLU' of the pre-activations below
+            if (i > 0) {
 #pragma unroll
-          for (int q = 0; q < 32; q += 4) {
-            const float4 b4 = bp[q / 4];
-            w[q / 2] = pack_bf16(silu_f(z[q] + b4.x), silu_f(z[q + 1] + b4.y));
-            w[q / 2 + 1] = pack_bf16(silu_f(z[q + 2] + b4.z), silu_f(z[q + 3] + b4.w));
+              for (int q = 0; q < 32; ++q) z0[q] = __uint_as_float(buf[(32 * (i - 1) + q) * 32 + lane]);
+            }
+#pragma unroll
+            for (int q = 0; q < 16; ++q)
+              w[q] = pack_bf16(z[2 * q] * dsilu_f(z0[2 * q]), z[2 * q + 1] * dsilu_f(z0[2 * q + 1]));
+          } else {
+            const float4* bp = reinterpret_cast<const float4*>(bias + 32 * i);
+#pragma unroll
+            for (int q = 0; q < 32; q += 4) {
+              const float4 b4 = bp[q / 4];
+              z[q] += b4.x; z[q + 1] += b4.y; z[q + 2] += b4.z; z[q + 3] += b4.w;
+              w[q / 2] = pack_bf16(silu_f(z[q]), silu_f(z[q + 1]));
+              w[q / 2 + 1] = pack_bf16(silu_f(z[q + 2]), silu_f(z[q + 3]));
+            }
+            if (MODE == FORWARD && keep) {
+              float* zp = a.zt[l] + (size_t)c0 * a.rows + row;
+#pragma unroll
+              for (int q = 0; q < 32; ++q) zp[(size_t)q * a.rows] = z[q];
+            }
           }
+          if (MODE != INFER && keep) put_columns(a.at[l] + (size_t)c0 * a.rows + row, a.rows, w);
           tmem_st16(lanes + (uint32_t)(c0 / 2), w);
         }
         publish();
       }
       if (!ok) break;
-      const int row0 = mt * BM + quarter * 32;
-      const int rows = a.rows - row0 < 32 ? a.rows - row0 : 32;
       int nmt = 0, nt0 = 0, nt1 = 0;
       const bool more = infer_item(a, v + 1, nmt, nt0, nt1);
       const int last = o + t1 - t0 - 1;   // the item's last output job
       bool entered = false;
-      for (int t = first; t < t1; t += 3) {
-        const int jo = o + t - t0;
+      for (int t = first; t < t1; t += stride) {
+        const int jo = o + t - t0, b = MODE == FORWARD ? jo % 3 : group;
         put_bias();
-        if (t + 3 < t1) fetch_out(t + 3);
+        if (t + stride < t1) fetch_out(t + stride);
         else fetch_hidden(0);
-        if (!(ok = wait(accf0 + 8 * group, (uint32_t)(jo / 3) & 1u))) break;
+        if (MODE == FORWARD && t > first) load_targets(row0, rows, t);
+        if (!(ok = wait(accf0 + 8 * b, (uint32_t)(jo / 3) & 1u))) break;
         // the row tile's last MMAs have read A: the next row tile enters
-        if (jo == last && more) { load_input(nmt); entered = true; }
+        if (jo == last && more) { load_input(nmt, keeps(a, v + 1, a.layers * a.H / 32)); entered = true; }
         const int cols = min(a.n_out - t * INF_BN, INF_BN);
         const bool full = rows == 32 && cols == INF_BN;
         char* yb = reinterpret_cast<char*>(a.y + t * INF_BN) + (size_t)row0 * pitch;
 #pragma unroll 1
-        for (int c0 = 0; c0 < cols; c0 += 32) {
+        for (int c0 = MODE == FORWARD ? 32 * group : 0; c0 < cols; c0 += MODE == FORWARD ? 32 * INF_GROUPS : 32) {
           float y[32];
-          tmem_ld32(lanes + TM_ACC + (uint32_t)(group * INF_BN + c0), y);
-          if (full) {
+          tmem_ld32(lanes + TM_ACC + (uint32_t)(b * INF_BN + c0), y);
+          if constexpr (MODE == FORWARD) {
+            // Weighted squared error and its gradient 2 w (y - t) / rows.  The 32
+            // terms of a chunk add up as a float pair, its chunks in FP64 (an FP64
+            // add a term would take 8 us: the pipe has two lanes an SM).
+            const int col = t * INF_BN + c0;
+            const float4* tp = reinterpret_cast<const float4*>(buf + lane * INF_PITCH + (c0 < 32 * INF_GROUPS ? 0 : 32));
+            const float wl = col + lane < a.n_out ? a.w[col + lane] : 0.f;
+            PairSum part{0.f, 0.f};
+            uint32_t g[16];
+#pragma unroll
+            for (int q = 0; q < 32; q += 4) {
+              const float4 t4 = tp[q / 4];
+              const float tq[4] = {t4.x, t4.y, t4.z, t4.w};
+#pragma unroll
+              for (int e = 0; e < 4; ++e) {
+                const float wt = __shfl_sync(0xffffffffu, wl, q + e);
+                float d = (y[q + e] + bias[c0 + q + e]) - tq[e];
+                d = row < a.rows && col + q + e < a.n_out ? d : 0.f;
+                mpcmd::pair_add(part, __fmul_rn(__fmul_rn(wt, d), d));
+                y[q + e] = 2.f * wt * d;
+              }
+            }
+            // (a power of two divides exactly as its reciprocal multiplies)
+            if (a.inv_rows != 0.f) {
+#pragma unroll
+              for (int q = 0; q < 32; ++q) y[q] *= a.inv_rows;
+            } else {
+#pragma unroll
+              for (int q = 0; q < 32; ++q) y[q] /= (float)a.rows;
+            }
+#pragma unroll
+            for (int q = 0; q < 16; ++q) g[q] = pack_bf16(y[2 * q], y[2 * q + 1]);
+            loss += mpcmd::pair_value(part);
+            if (row < a.rows) {
+              uint4* dst = reinterpret_cast<uint4*>(a.dy + row * a.npad + col);
+#pragma unroll
+              for (int q = 0; q < 4; ++q) dst[q] = make_uint4(g[4 * q], g[4 * q + 1], g[4 * q + 2], g[4 * q + 3]);
+              put_columns(a.dyt + (size_t)col * a.rows + row, a.rows, g);
+            }
+          } else if (full) {
             stage_chunk(buf, lane, c0 % INF_WIDE, y, bias + c0);
             if ((c0 + 32) % INF_WIDE == 0) {
               __syncwarp();
@@ -870,17 +817,27 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(INF_THREADS, 1)
           }
         }
         tmem_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(acce0 + 8 * group);
+        __syncwarp();   // (FORWARD: the staging tile has been read, too)
+        if (lane == 0) mbar_arrive(acce0 + 8 * b);
       }
       if (ok && more && !entered) {
         // another group has the last output job
         if (first >= t1) fetch_hidden(0);
-        if ((ok = wait(accf0 + 8 * (last % 3), (uint32_t)(last / 3) & 1u))) load_input(nmt);
+        if constexpr (MODE == BACKWARD) {
+          // no output job: the next input may enter when every warp has read the
+          // last accumulator
+          if ((ok = wait(hready, (uint32_t)(published - 1) & 1u))) load_input(nmt, true);
+        } else if ((ok = wait(accf0 + 8 * (last % 3), (uint32_t)(last / 3) & 1u))) {
+          load_input(nmt, keeps(a, v + 1, a.layers * a.H / 32));
+        }
       }
       o += t1 - t0;
       mt = nmt; t0 = nt0; t1 = nt1;
       ok = ok && more;
+    }
+    if constexpr (MODE == FORWARD) {
+      for (int q = 16; q > 0; q >>= 1) loss += __shfl_xor_sync(0xffffffffu, loss, q);
+      if (lane == 0) a.loss[(size_t)blockIdx.x * INF_EPI + ew] = loss;
     }
   }
   __syncthreads();
@@ -900,70 +857,372 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(INF_THREADS, 1)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
 }
 
-// ------------------------------------------------------- small kernels ----
-// x [rows, n_in] (FP32) -> X0 [rows, kin] BF16 zero-padded, and X0^T [kin, rows].
-__global__ void k_prep_input(const float* x, int rows, int n_in, int kin, __nv_bfloat16* x0, __nv_bfloat16* x0t) {
-  const int total = rows * kin;
-  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < total; e += gridDim.x * blockDim.x) {
-    const int r = e / kin, c = e % kin;
-    const __nv_bfloat16 b = __float2bfloat16_rn(c < n_in ? x[(size_t)r * n_in + c] : 0.f);
-    x0[e] = b;
-    x0t[(size_t)c * rows + r] = b;
-  }
-}
+// ------------------------------------------------- training GEMMs ----
+// Pipeline of the two kernels below: tiles of 128 x BN, A and B boxes of a K
+// step in one stage, two accumulators.  Barriers full[S], empty[S], accf[2],
+// acce[2], done.
+template <int BN, int S, int EPI>
+struct Pipe {
+  static constexpr int A_STAGE = BM * BK * 2, BOX = A_STAGE + BN * BK * 2;
+  static constexpr int THREADS = 64 + 32 * EPI;
+  static constexpr uint32_t COLS = 2 * BN < 32 ? 32 : 2 * BN;
+  uint8_t* ring;
+  uint32_t full, empty, accf, acce, done, tmem;
+  int* err;
+  volatile int* bail;
 
-// Weighted squared error: loss += sum_j w_j (y - t)^2 / B, dY = 2 w_j (y - t) / B
-// as BF16 [B, npad] and its transpose [npad, B] (zero in the padded columns).
-__global__ void k_loss(const float* y, const float* t, const float* w, int B, int n_out, int npad,
-                       __nv_bfloat16* dy, __nv_bfloat16* dyt, double* loss) {
-  double acc = 0.0;
-  const int64_t total = (int64_t)B * npad;
-  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total; e += (int64_t)gridDim.x * blockDim.x) {
-    const int b = (int)(e / npad), j = (int)(e % npad);
-    float g = 0.f;
-    if (j < n_out) {
-      const float d = y[(size_t)b * n_out + j] - t[(size_t)b * n_out + j];
-      acc += (double)(w[j] * d * d) / B;
-      g = 2.f * w[j] * d / (float)B;
+  static constexpr size_t bytes(size_t extra) {
+    return 1024 + (size_t)S * BOX + (2 * S + 5) * 8 + 16 + (extra ? extra + 16 : 0);
+  }
+
+  // Shared memory, barriers and tensor memory; returns what follows the ring.
+  __device__ __forceinline__ uint8_t* open(uint8_t* raw, volatile int* bail_, int* issued, int* err_) {
+    ring = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(raw) + 1023) & ~(uintptr_t)1023);
+    uint64_t* bars = reinterpret_cast<uint64_t*>(ring + S * BOX);
+    uint32_t* slot = reinterpret_cast<uint32_t*>(bars + 2 * S + 5);
+    full = smem_u32(bars); empty = full + 8 * S; accf = empty + 8 * S; acce = accf + 16; done = acce + 16;
+    err = err_; bail = bail_;
+    if (threadIdx.x == 0) {
+      *bail = 0;
+      *issued = 0;
+      for (int s = 0; s < S; ++s) { mbar_init(full + 8 * s, 1); mbar_init(empty + 8 * s, 1); }
+      for (int b = 0; b < 2; ++b) { mbar_init(accf + 8 * b, 1); mbar_init(acce + 8 * b, EPI); }
+      mbar_init(done, 1);
+      asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
-    const __nv_bfloat16 gb = __float2bfloat16_rn(g);
-    dy[e] = gb;
-    dyt[(size_t)j * B + b] = gb;
+    if ((threadIdx.x >> 5) == 1) {
+      asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(slot)), "r"(COLS)
+                   : "memory");
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    tmem_fence_before();
+    __syncthreads();
+    tmem_fence_after();
+    tmem = *slot;
+    return reinterpret_cast<uint8_t*>(bars) + (2 * S + 5) * 8 + 16;
   }
-  for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-  if ((threadIdx.x & 31) == 0) atomicAdd(loss, acc);
-}
+  // one tile's loads (producer thread); g counts stages
+  __device__ __forceinline__ bool load(int& g, int nk, const CUtensorMap* ta, int row_a, const CUtensorMap* tb,
+                                       int row_b) {
+    for (int k = 0; k < nk; ++k) {
+      const int s = g % S;
+      if (g >= S && !mbar_wait(empty + 8 * s, ((uint32_t)(g / S) & 1u) ^ 1u, err)) { *bail = 1; return false; }
+      mbar_expect_tx(full + 8 * s, BOX);
+      tma_load_2d(smem_u32(ring + s * BOX), ta, full + 8 * s, k * BK, row_a);
+      tma_load_2d(smem_u32(ring + s * BOX + A_STAGE), tb, full + 8 * s, k * BK, row_b);
+      ++g;
+    }
+    return true;
+  }
+  // tile j's MMAs (issuer thread)
+  __device__ __forceinline__ bool multiply(int& g, int j, int nk) {
+    constexpr uint32_t idesc = f16_idesc(BM, BN);
+    const int b = j & 1;
+    if (j >= 2 && !mbar_wait(acce + 8 * b, ((uint32_t)(j >> 1) & 1u) ^ 1u, err)) { *bail = 1; return false; }
+    tmem_fence_after();
+    const uint32_t acc = tmem + (uint32_t)(b * BN);
+    for (int k = 0; k < nk; ++k, ++g) {
+      const int s = g % S;
+      if (!mbar_wait(full + 8 * s, (uint32_t)(g / S) & 1u, err)) { *bail = 1; return false; }
+      tmem_fence_after();
+      const uint32_t a0 = smem_u32(ring + s * BOX), b0 = a0 + A_STAGE;
+#pragma unroll
+      for (int kk = 0; kk < BK / 16; ++kk)
+        mma_bf16(acc, sw128_desc(a0 + 32 * kk), sw128_desc(b0 + 32 * kk), idesc, (k > 0 || kk > 0) ? 1u : 0u);
+      mma_commit(empty + 8 * s);
+    }
+    mma_commit(accf + 8 * b);
+    return true;
+  }
+  // columns c0.. of tile j's accumulator of this warp's quarter (epilogue warps)
+  __device__ __forceinline__ bool ready(int j) {
+    if (!mbar_wait(accf + 8 * (j & 1), (uint32_t)(j >> 1) & 1u, err)) { *bail = 1; return false; }
+    tmem_fence_after();
+    return true;
+  }
+  template <int N>
+  __device__ __forceinline__ void read(int j, int quarter, int c0, float (&v)[N]) {
+    const uint32_t at = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)((j & 1) * BN + c0);
+    if constexpr (N == 32) tmem_ld32(at, v);
+    else tmem_ld16(at, v);
+  }
+  __device__ __forceinline__ void release(int j) {
+    tmem_fence_before();
+    __syncwarp();
+    if ((threadIdx.x & 31) == 0) mbar_arrive(acce + 8 * (j & 1));
+  }
+  // every MMA and every load that was issued has completed before the tensor
+  // memory is freed and the CTA exits
+  __device__ __forceinline__ void close(const int* issued) {
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      mbar_wait(done, 0, err);
+      const int g1 = *issued;
+      for (int g = g1 - S < 0 ? 0 : g1 - S; g < g1; ++g) mbar_wait(full + 8 * (g % S), (uint32_t)(g / S) & 1u, err);
+    }
+    tmem_fence_before();
+    __syncthreads();
+    tmem_fence_after();
+    if ((threadIdx.x >> 5) == 1)
+      asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(COLS) : "memory");
+  }
+};
 
-// Row sums of a BF16 [n, ld] matrix over its first `cols` columns (the bias
-// gradient from the transposed output gradient): one warp per row.
-__global__ void k_rowsum(const __nv_bfloat16* a, int n, int ld, int cols, float* out) {
-  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-  if (warp >= n) return;
-  float s = 0.f;
-  for (int c = lane; c < cols; c += 32) s += __bfloat162float(a[(size_t)warp * ld + c]);
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  if (lane == 0) out[warp] = s;
-}
+// Gradient of the last hidden layer: dz = (dY . W_out) * SiLU'(z) as [rows, H]
+// and [H, rows].  Bound by its chain of MMAs: each adds 16 of K to the sum of
+// the one before, and takes 134 cycles whatever its width (64-row tiles, or 16
+// stages in flight: the same 540 cycles for 64 of K; 12 us for 2,050 outputs).
+// So the columns are spread over CTAs, 32 to each.  Block 0 also adds up the
+// loss.
+struct DxArgs {
+  int rows, H, nk;      // nk: K boxes that hold outputs (the padding is zero)
+  const float* zt;      // [H, rows]
+  __nv_bfloat16 *dz, *dzt;
+  const double* loss;   // partial sums
+  int n_loss;
+  double* loss_out;     // host memory: sum / rows
+  int* err;
+};
+using DxPipe = Pipe<32, 10, 4>;
 
-// Adam (Kingma & Ba, 2015) on one FP32 master tensor [n, k] with its
-// gradient, moments and the step's bias corrections; refreshes the BF16
-// copies [n, k] and [k, n] (wt may be null for a bias).
-__global__ void k_adam(float* p, const float* g, float* m1, float* m2, int64_t count, int k, float lr, float b1,
-                       float b2, float eps, float c1, float c2, __nv_bfloat16* wb, __nv_bfloat16* wt, int n) {
-  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < count; e += (int64_t)gridDim.x * blockDim.x) {
-    const float gr = g[e];
-    const float a1 = b1 * m1[e] + (1.f - b1) * gr;
-    const float a2 = b2 * m2[e] + (1.f - b2) * gr * gr;
-    m1[e] = a1;
-    m2[e] = a2;
-    const float v = p[e] - lr * (a1 / c1) / (sqrtf(a2 / c2) + eps);
-    p[e] = v;
-    if (wb) {
-      const __nv_bfloat16 b = __float2bfloat16_rn(v);
-      wb[e] = b;
-      if (wt) wt[(size_t)(e % k) * n + e / k] = b;
+__global__ void __launch_bounds__(DxPipe::THREADS, 1)
+    k_dx(const __grid_constant__ CUtensorMap ta, const __grid_constant__ CUtensorMap tb, DxArgs a) {
+  extern __shared__ uint8_t smem_raw[];
+  __shared__ volatile int bail;
+  __shared__ int issued;
+  DxPipe p;
+  p.open(smem_raw, &bail, &issued, a.err);
+  let_next_start();
+  wait_for_previous();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int tiles_n = a.H / 32, units = (a.rows / BM) * tiles_n;
+  if (warp == 0) {
+    if (lane == 0) {
+      int g = 0;
+      for (int u = blockIdx.x; u < units && !bail; u += gridDim.x)
+        if (!p.load(g, a.nk, &ta, (u / tiles_n) * BM, &tb, (u % tiles_n) * 32)) break;
+      issued = g;
+    }
+    __syncwarp();
+    if (blockIdx.x == 0) {
+      double s = 0.;
+#pragma unroll 8
+      for (int i = lane; i < a.n_loss; i += 32) s += a.loss[i];
+      for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+      if (lane == 0) *a.loss_out = s / (double)a.rows;
+    }
+  } else if (warp == 1) {
+    if (lane == 0) {
+      int g = 0, j = 0;
+      for (int u = blockIdx.x; u < units && !bail; u += gridDim.x, ++j)
+        if (!p.multiply(g, j, a.nk)) break;
+      mma_commit(p.done);
+    }
+  } else {
+    const int quarter = warp & 3;
+    int j = 0;
+    for (int u = blockIdx.x; u < units; u += gridDim.x, ++j) {
+      const int row = (u / tiles_n) * BM + quarter * 32 + lane, n = (u % tiles_n) * 32;
+      float z[32];   // fetched while the MMAs run
+#pragma unroll
+      for (int q = 0; q < 32; ++q) z[q] = a.zt[(size_t)(n + q) * a.rows + row];
+      if (!p.ready(j)) break;
+      float v[32];
+      p.read(j, quarter, 0, v);
+      uint32_t w[16];
+#pragma unroll
+      for (int q = 0; q < 16; ++q) w[q] = pack_bf16(v[2 * q] * dsilu_f(z[2 * q]), v[2 * q + 1] * dsilu_f(z[2 * q + 1]));
+      uint4* dst = reinterpret_cast<uint4*>(a.dz + (size_t)row * a.H + n);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) dst[q] = make_uint4(w[4 * q], w[4 * q + 1], w[4 * q + 2], w[4 * q + 3]);
+      put_columns(a.dzt + (size_t)n * a.rows + row, a.rows, w);
+      p.release(j);
     }
   }
+  p.close(&issued);
+}
+
+// Weight and bias gradients of every layer, dW = dZ^T . X^T^T over the batch and
+// db = row sums of dZ^T, and either written out or applied: Adam (Kingma & Ba,
+// 2015) on the FP32 master tensors with the step's bias corrections, which
+// refreshes the BF16 copies [n, k] and [k, n].  Work units: the 128 x 64 tiles of
+// every layer, then blocks of 64 biases; 5 of its 8 us are Adam's divisions and
+// root, so 16 warps share a tile (8: 7 us); the parameters and moments (24 bytes a
+// weight, in L2) are fetched before the previous kernel has ended.
+struct AdamArgs {
+  float lr, b1, b2, eps, c1, c2;
+};
+struct DwLayer {
+  int n, k;             // padded widths of W [n, k]
+  int first, first_bias;   // first work unit of its tiles and of its biases
+  float *w, *m, *v, *g;
+  float *bw, *bm, *bv, *bg;
+  __nv_bfloat16 *wb, *wt;
+  const __nv_bfloat16* dzt;   // [n, rows]
+};
+struct DwMaps {
+  CUtensorMap a[MAX_HIDDEN + 1], b[MAX_HIDDEN + 1];   // dZ^T [n, rows], X^T [k, rows]
+};
+struct DwArgs {
+  int layers, rows, tiles, units;   // tiles: units with MMAs
+  DwLayer l[MAX_HIDDEN + 1];
+  AdamArgs adam;
+  int* err;
+};
+constexpr int DW_EPI = 16;
+using DwPipe = Pipe<64, 4, DW_EPI>;
+constexpr int DW_PITCH = 20;   // words of a staged row
+constexpr size_t DW_SMEM = DwPipe::bytes((size_t)DW_EPI * 32 * DW_PITCH * 4);
+
+// (Zero moments, those of all padding and of inputs that are always zero, leave
+// the parameter alone; their divisions and root would take the slow path of
+// special operands: 22 us for a tile of them instead of 6.)
+__device__ __forceinline__ float adam_step(float p, float gr, float& m1, float& m2, const AdamArgs& a) {
+  const float a1 = __fmaf_rn(1.f - a.b1, gr, __fmul_rn(a.b1, m1));
+  const float a2 = __fmaf_rn(__fmul_rn(1.f - a.b2, gr), gr, __fmul_rn(a.b2, m2));
+  m1 = a1;
+  m2 = a2;
+  const bool still = a1 == 0.f && a2 == 0.f;
+  const float q = a.lr * ((still ? 1.f : a1) / a.c1) / (sqrtf((still ? 1.f : a2) / a.c2) + a.eps);
+  return still ? p : p - q;
+}
+
+template <bool UPDATE>
+__global__ void __launch_bounds__(DwPipe::THREADS, 1)
+    k_dw(const __grid_constant__ DwMaps maps, const __grid_constant__ DwArgs a) {
+  extern __shared__ uint8_t smem_raw[];
+  __shared__ volatile int bail;
+  __shared__ int issued;
+  DwPipe p;
+  uint8_t* rest = p.open(smem_raw, &bail, &issued, a.err);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int nk = a.rows / BK;
+  // layer and tile of unit u
+  auto tile_of = [&](int u, int& l, int& mt, int& nt) {
+    l = 0;
+    while (l + 1 < a.layers && u >= a.l[l + 1].first) ++l;
+    const int q = u - a.l[l].first, tn = a.l[l].k / 64;
+    mt = q / tn;
+    nt = q % tn;
+  };
+  if (warp == 0) {
+    if (lane == 0) {
+      wait_for_previous();
+      int g = 0, l, mt, nt;
+      for (int u = blockIdx.x; u < a.tiles && !bail; u += gridDim.x) {
+        tile_of(u, l, mt, nt);
+        if (!p.load(g, nk, &maps.a[l], mt * BM, &maps.b[l], nt * 64)) break;
+      }
+      issued = g;
+    }
+  } else if (warp == 1) {
+    if (lane == 0) {
+      int g = 0, j = 0;
+      for (int u = blockIdx.x; u < a.tiles && !bail; u += gridDim.x, ++j)
+        if (!p.multiply(g, j, nk)) break;
+      mma_commit(p.done);
+    }
+  } else {
+    const int ew = warp - 2, quarter = warp & 3, c0 = (ew >> 2) * 16;
+    float* buf = reinterpret_cast<float*>((reinterpret_cast<uintptr_t>(rest) + 15) & ~(uintptr_t)15) + ew * 32 * DW_PITCH;
+    int j = 0, l, mt, nt;
+    for (int u = blockIdx.x; u < a.units; u += gridDim.x) {
+      if (u < a.tiles) {
+        tile_of(u, l, mt, nt);
+        const DwLayer& ly = a.l[l];
+        // this lane's part of the 32 x 16 block: 4 columns of every eighth row
+        const int row0 = mt * BM + quarter * 32, col = nt * 64 + c0, sub = lane >> 2, q0 = 4 * (lane & 3);
+        const bool real = row0 < ly.n;   // (widths are multiples of 64)
+        const size_t at = (size_t)(row0 + sub) * ly.k + col + q0, step = 8 * (size_t)ly.k;
+        float4 x[4], m1[4], m2[4];       // fetched while the MMAs run
+        if (UPDATE && real) {
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            x[i] = *reinterpret_cast<const float4*>(ly.w + at + i * step);
+            m1[i] = *reinterpret_cast<const float4*>(ly.m + at + i * step);
+            m2[i] = *reinterpret_cast<const float4*>(ly.v + at + i * step);
+          }
+        }
+        if (!p.ready(j)) break;
+        {
+          float v[16];
+          p.read(j, quarter, c0, v);
+          p.release(j);
+#pragma unroll
+          for (int q = 0; q < 16; q += 4)
+            *reinterpret_cast<float4*>(buf + lane * DW_PITCH + q) = make_float4(v[q], v[q + 1], v[q + 2], v[q + 3]);
+        }
+        __syncwarp();
+        ++j;
+        if (real) {
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            float4* cell = reinterpret_cast<float4*>(buf + (8 * i + sub) * DW_PITCH + q0);
+            const float4 gr = *cell;
+            if constexpr (UPDATE) {
+              x[i].x = adam_step(x[i].x, gr.x, m1[i].x, m2[i].x, a.adam);
+              x[i].y = adam_step(x[i].y, gr.y, m1[i].y, m2[i].y, a.adam);
+              x[i].z = adam_step(x[i].z, gr.z, m1[i].z, m2[i].z, a.adam);
+              x[i].w = adam_step(x[i].w, gr.w, m1[i].w, m2[i].w, a.adam);
+              *reinterpret_cast<float4*>(ly.w + at + i * step) = x[i];
+              *reinterpret_cast<float4*>(ly.m + at + i * step) = m1[i];
+              *reinterpret_cast<float4*>(ly.v + at + i * step) = m2[i];
+              *reinterpret_cast<uint2*>(ly.wb + at + i * step) =
+                  make_uint2(pack_bf16(x[i].x, x[i].y), pack_bf16(x[i].z, x[i].w));
+              *cell = x[i];
+            } else {
+              *reinterpret_cast<float4*>(ly.g + at + i * step) = gr;
+            }
+          }
+          if constexpr (UPDATE) {
+            // the transposed copy from the thread-per-row layout
+            __syncwarp();
+            uint32_t w[8];
+#pragma unroll
+            for (int q = 0; q < 16; q += 4) {
+              const float4 p4 = *reinterpret_cast<const float4*>(buf + lane * DW_PITCH + q);
+              w[q / 2] = pack_bf16(p4.x, p4.y);
+              w[q / 2 + 1] = pack_bf16(p4.z, p4.w);
+            }
+            put_columns(ly.wt + (size_t)col * ly.n + row0 + lane, ly.n, w);
+          }
+        }
+        __syncwarp();
+      } else {
+        l = 0;
+        while (l + 1 < a.layers && u >= a.l[l + 1].first_bias) ++l;
+        const DwLayer& ly = a.l[l];
+        // four rows a warp, their loads in flight together; lane r finishes row r
+        const int n0 = (u - ly.first_bias) * 64 + 4 * ew, n = n0 + (lane & 3);
+        float b = 0.f, m1 = 0.f, m2 = 0.f;
+        if constexpr (UPDATE) { b = ly.bw[n]; m1 = ly.bm[n]; m2 = ly.bv[n]; }
+        wait_for_previous();
+        float s[4] = {};
+        const __nv_bfloat16* zp = ly.dzt + (size_t)n0 * a.rows + lane;
+#pragma unroll 4
+        for (int c = 0; c < a.rows; c += 32)
+#pragma unroll
+          for (int r = 0; r < 4; ++r) s[r] += __bfloat162float(zp[(size_t)r * a.rows + c]);
+        float sum = 0.f;
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+          for (int o = 16; o > 0; o >>= 1) s[r] += __shfl_xor_sync(0xffffffffu, s[r], o);
+          if (lane == r) sum = s[r];
+        }
+        if (lane < 4) {
+          if constexpr (UPDATE) {
+            ly.bw[n] = adam_step(b, sum, m1, m2, a.adam);
+            ly.bm[n] = m1;
+            ly.bv[n] = m2;
+          } else {
+            ly.bg[n] = sum;
+          }
+        }
+      }
+    }
+  }
+  p.close(&issued);
 }
 
 __global__ void k_to_bf16(const float* p, int64_t count, int k, int n, __nv_bfloat16* wb, __nv_bfloat16* wt) {
@@ -1019,14 +1278,19 @@ struct mpcmd_mlp {
   int64_t R = 0;           // largest inference call (>= batch, >= max_rows, multiple of 128)
   std::vector<Layer> layers;
   std::vector<void*> allocs;
-  __nv_bfloat16 *x0 = nullptr, *x0t = nullptr;
-  std::vector<__nv_bfloat16*> h, ht, dz, dzt;   // [L] activations, transposed, gradients, transposed
-  std::vector<float*> z;                        // [L] pre-activations
-  __nv_bfloat16 *dy = nullptr, *dyt = nullptr;
-  float* yb = nullptr;                          // [B, nout] training output
-  double* dloss = nullptr;
+  // one training batch: x^T [64, B]; per hidden layer activations and gradients
+  // [H, B], pre-activations [H, B]; the last hidden layer's gradient [B, H];
+  // the output gradient [B, npad] and [npad, B]
+  __nv_bfloat16 *x0t = nullptr, *dz = nullptr, *dy = nullptr, *dyt = nullptr;
+  std::vector<__nv_bfloat16*> ht, dzt;
+  std::vector<float*> zt;
+  double* loss_part = nullptr;
+  double* loss = nullptr;  // the last batch's loss (page-locked host memory)
   int* err = nullptr;      // raised by a kernel whose wait expired (page-locked host memory)
-  InferMaps maps{};        // weight boxes of inference (the weights stay where they are)
+  InferMaps maps{}, back{};   // weight boxes of the forward and backward chains (the weights stay where they are)
+  CUtensorMap dx_a{}, dx_b{};
+  DwMaps dw_maps{};
+  DwArgs dw{};
   int64_t step = 0;
   int sms = 1;             // SMs of the device (one persistent GEMM CTA each)
   cudaStream_t st = nullptr;
@@ -1035,6 +1299,7 @@ struct mpcmd_mlp {
     if (st) cudaStreamDestroy(st);
     for (void* p : allocs) cudaFree(p);
     if (err) cudaFreeHost(err);
+    if (loss) cudaFreeHost(loss);
   }
   template <class U>
   int alloc(U*& p, int64_t n) {
@@ -1055,58 +1320,32 @@ int status_of(mpcmd_mlp* m) {
   return *reinterpret_cast<volatile int*>(m->err) ? MPCMD_ERR_CUDA : MPCMD_OK;
 }
 
-// One persistent CTA per SM (at most one per tile).
-template <int BN, int MODE>
-void launch_one(mpcmd_mlp* m, int grid, const CUtensorMap& ta, const CUtensorMap& tb, const GemmArgs& g) {
-  k_gemm<BN, MODE><<<grid, THREADS, gemm_smem_bytes<BN, MODE>(), m->st>>>(ta, tb, g);
+// A kernel that sets itself up while the one before it in the stream still runs
+// (it calls wait_for_previous; a step of 256 rows takes 87 us instead of 97).
+template <typename... P, typename... A>
+void launch_early(void (*kernel)(P...), int grid, int threads, size_t smem, cudaStream_t st, const A&... args) {
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t c{};
+  c.gridDim = dim3((unsigned)grid);
+  c.blockDim = dim3((unsigned)threads);
+  c.dynamicSmemBytes = smem;
+  c.stream = st;
+  c.attrs = &at;
+  c.numAttrs = 1;
+  cudaLaunchKernelEx(&c, kernel, args...);
 }
 
-template <int BN>
-void launch_bn(mpcmd_mlp* m, int grid, const CUtensorMap& ta, const CUtensorMap& tb, const GemmArgs& g) {
-  switch (g.mode) {
-    case EP_HIDDEN: launch_one<BN, EP_HIDDEN>(m, grid, ta, tb, g); break;
-    case EP_OUT: launch_one<BN, EP_OUT>(m, grid, ta, tb, g); break;
-    case EP_DX: launch_one<BN, EP_DX>(m, grid, ta, tb, g); break;
-    default: launch_one<BN, EP_DW>(m, grid, ta, tb, g); break;
-  }
+template <int MODE, int VB>
+bool allow_chain() {
+  return cudaFuncSetAttribute(k_chain<MODE, VB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)INF_SMEM) ==
+         cudaSuccess;
 }
-
-template <int BN, int MODE>
-bool allow_one() {
-  return cudaFuncSetAttribute(k_gemm<BN, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (int)gemm_smem_bytes<BN, MODE>()) == cudaSuccess;
+template <bool UPDATE>
+bool allow_dw() {
+  return cudaFuncSetAttribute(k_dw<UPDATE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DW_SMEM) == cudaSuccess;
 }
-
-template <int BN>
-bool allow_smem() {
-  return allow_one<BN, EP_HIDDEN>() && allow_one<BN, EP_OUT>() && allow_one<BN, EP_DX>() && allow_one<BN, EP_DW>();
-}
-
-template <int VB>
-bool allow_infer() {
-  return cudaFuncSetAttribute(k_infer<VB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)INF_SMEM) == cudaSuccess;
-}
-
-int launch_gemm(mpcmd_mlp* m, const CUtensorMap& ta, const CUtensorMap& tb, const GemmArgs& g, int BN) {
-  const int units = ((g.M + BM - 1) / BM) * (g.N / BN);
-  const int grid = units < m->sms ? units : m->sms;
-  if (BN == 256) launch_bn<256>(m, grid, ta, tb, g);
-  else if (BN == 128) launch_bn<128>(m, grid, ta, tb, g);
-  else launch_bn<64>(m, grid, ta, tb, g);
-  return cudaPeekAtLastError() == cudaSuccess ? MPCMD_OK : MPCMD_ERR_CUDA;
-}
-
-// C[M, N] = A[M, K] . B[N, K]^T on tcgen05; A and B row-major BF16 with
-// A_rows x K and B_rows x K allocated (K-major), M, N tile multiples.
-int gemm(mpcmd_mlp* m, const void* A, int64_t a_rows, const void* Bm, int64_t b_rows, int M, int N, int K, GemmArgs g,
-         int BN) {
-  CUtensorMap ta, tb;
-  if (!make_map(&ta, A, a_rows, K, BM) || !make_map(&tb, Bm, b_rows, K, BN)) return MPCMD_ERR_CUDA;
-  g.M = M; g.N = N; g.K = K; g.err = m->err;
-  return launch_gemm(m, ta, tb, g, BN);
-}
-
-int pick_bn(int N) { return N % 256 == 0 ? 256 : (N % 128 == 0 ? 128 : 64); }
 
 // Output jobs of a row tile and the width of the last one's MMA (a multiple
 // of 16, as the instruction takes it).
@@ -1121,6 +1360,48 @@ bool make_infer_maps(mpcmd_mlp* m) {
          make_map(&m->maps.tail, lo.wb, lo.n, lo.k, infer_tail(m) / 2);
 }
 
+// Operands and work units of the training step's other launches.
+bool make_train_maps(mpcmd_mlp* m) {
+  for (int j = 0; j + 1 < m->L; ++j) {
+    const Layer& ly = m->layers[m->L - 1 - j];
+    if (!make_map(&m->back.w[j], ly.wt, ly.k, ly.n, m->H / 2)) return false;
+  }
+  const Layer& lo = m->layers[m->L];
+  if (!make_map(&m->dx_a, m->dy, m->B, m->npad, BM) || !make_map(&m->dx_b, lo.wt, lo.k, lo.n, 32)) return false;
+  DwArgs& d = m->dw;
+  d.layers = m->L + 1; d.rows = m->B; d.err = m->err;
+  int u = 0;
+  for (int l = 0; l <= m->L; ++l) {
+    const Layer& ly = m->layers[l];
+    DwLayer& q = d.l[l];
+    q.n = ly.n; q.k = ly.k;
+    q.w = ly.w; q.m = ly.mw; q.v = ly.vw; q.g = ly.gw;
+    q.bw = ly.b; q.bm = ly.mb; q.bv = ly.vb; q.bg = ly.gb;
+    q.wb = ly.wb; q.wt = ly.wt;
+    q.dzt = l == m->L ? m->dyt : m->dzt[l];
+    q.first = u;
+    u += (ly.n + BM - 1) / BM * (ly.k / 64);
+    const __nv_bfloat16* xt = l == 0 ? m->x0t : m->ht[l - 1];
+    if (!make_map(&m->dw_maps.a[l], q.dzt, ly.n, m->B, BM) || !make_map(&m->dw_maps.b[l], xt, ly.k, m->B, 64))
+      return false;
+  }
+  d.tiles = u;
+  for (int l = 0; l <= m->L; ++l) { d.l[l].first_bias = u; u += m->layers[l].n / 64; }
+  d.units = u;
+  return true;
+}
+
+// Row tiles of a chain over the CTAs: whole rounds of one row tile per SM, then
+// the left-over row-tile pairs shared as far as the SMs go.
+int chain_grid(const mpcmd_mlp* m, int64_t rows, InferArgs& a) {
+  const int pairs = (int)((rows + 2 * BM - 1) / (2 * BM)), cap = std::max(m->sms / 2, 1);
+  a.whole = pairs / cap;
+  a.part = pairs % cap;
+  const int shares = a.tiles ? a.tiles : a.layers * a.H / 32;   // (BACKWARD: the pieces kept)
+  a.split = a.part ? std::min(shares, cap / a.part) : 1;
+  return 2 * (a.whole ? cap : a.part * a.split);
+}
+
 // y [rows, nout] = network(x [rows, n_in]) (device, FP32).
 int infer(mpcmd_mlp* m, const float* x, int64_t rows, float* y) {
   InferArgs a{};
@@ -1130,83 +1411,49 @@ int infer(mpcmd_mlp* m, const float* x, int64_t rows, float* y) {
   for (int l = 0; l < m->L; ++l) a.bias[l] = m->layers[l].b;
   a.n_out = m->nout; a.y = y; a.bias_out = m->layers[m->L].b;
   a.err = m->err;
-  // whole rounds of one row tile per SM, then the left-over row-tile pairs
-  // split by output jobs as far as the SMs go
-  const int pairs = (int)((rows + 2 * BM - 1) / (2 * BM)), cap = std::max(m->sms / 2, 1);
-  a.whole = pairs / cap;
-  a.part = pairs % cap;
-  a.split = a.part ? std::min(a.tiles, cap / a.part) : 1;
-  const int grid = 2 * (a.whole ? cap : a.part * a.split);
+  const int grid = chain_grid(m, rows, a);
   const uintptr_t align = reinterpret_cast<uintptr_t>(y) | ((uintptr_t)m->nout * 4);
-  if (align % 16 == 0) k_infer<16><<<grid, INF_THREADS, INF_SMEM, m->st>>>(m->maps, a);
-  else if (align % 8 == 0) k_infer<8><<<grid, INF_THREADS, INF_SMEM, m->st>>>(m->maps, a);
-  else k_infer<4><<<grid, INF_THREADS, INF_SMEM, m->st>>>(m->maps, a);
+  if (align % 16 == 0) k_chain<INFER, 16><<<grid, INF_THREADS, INF_SMEM, m->st>>>(m->maps, a);
+  else if (align % 8 == 0) k_chain<INFER, 8><<<grid, INF_THREADS, INF_SMEM, m->st>>>(m->maps, a);
+  else k_chain<INFER, 4><<<grid, INF_THREADS, INF_SMEM, m->st>>>(m->maps, a);
   return cudaPeekAtLastError() == cudaSuccess ? MPCMD_OK : MPCMD_ERR_CUDA;
 }
 
-// Forward pass of a training batch already in x0; output y [B, nout] FP32,
-// pre-activations and transposed activations kept for the backward pass.
-int forward(mpcmd_mlp* m, float* y) {
-  const int B = m->B;
-  const void* in = m->x0;
-  int kin = m->kin;
-  for (int l = 0; l < m->L; ++l) {
-    Layer& ly = m->layers[l];
-    GemmArgs g{};
-    g.mode = EP_HIDDEN;
-    g.out_bf16 = m->h[l]; g.ldb = m->H;
-    g.out_t = m->ht[l]; g.ldt = B;
-    g.bias = ly.b;
-    g.z = m->z[l]; g.ldz = m->H;
-    int r = gemm(m, in, B, ly.wb, ly.n, B, ly.n, kin, g, pick_bn(ly.n));
-    if (r) return r;
-    in = m->h[l];
-    kin = m->H;
-  }
-  Layer& lo = m->layers[m->L];
-  GemmArgs g{};
-  g.mode = EP_OUT;
-  g.m_valid = B; g.n_valid = m->nout;
-  g.out_f32 = y; g.ldo = m->nout;
-  g.bias = lo.b;
-  return gemm(m, in, B, lo.wb, lo.n, B, lo.n, m->H, g, pick_bn(lo.n));
-}
-
 // Loss and gradients of one batch (inputs x, targets t [B, nout], output
-// weights w [nout], device); the gradients land in the layers' gw / gb.
-int backward(mpcmd_mlp* m, const float* x, const float* t, const float* w) {
-  const int B = m->B;
-  k_prep_input<<<256, 256, 0, m->st>>>(x, B, m->cfg.n_in, m->kin, m->x0, m->x0t);
-  int r = forward(m, m->yb);
-  if (r) return r;
-  cudaMemsetAsync(m->dloss, 0, sizeof(double), m->st);
-  k_loss<<<256, 256, 0, m->st>>>(m->yb, t, w, B, m->nout, m->npad, m->dy, m->dyt, m->dloss);
-  // output layer: dW = dY^T . H_L, db = column sums of dY, dH_L = dY . W
-  const __nv_bfloat16* gt = m->dyt;   // [n_l, B] gradient of the current layer's output, transposed
-  const __nv_bfloat16* gr = m->dy;    // [B, n_l]
-  for (int l = m->L; l >= 0; --l) {
-    Layer& ly = m->layers[l];
-    const __nv_bfloat16* xin_t = l > 0 ? m->ht[l - 1] : m->x0t;   // layer input, transposed [k, B]
-    GemmArgs g{};
-    g.mode = EP_DW;
-    g.m_valid = ly.n;
-    g.out_f32 = ly.gw; g.ldo = ly.k;
-    // A = gradient^T [n, B], B operand = input^T [k, B]
-    r = gemm(m, gt, ly.n, xin_t, ly.k, ly.n, ly.k, B, g, pick_bn(ly.k));
-    if (r) return r;
-    k_rowsum<<<(ly.n * 32 + 255) / 256, 256, 0, m->st>>>(gt, ly.n, B, B, ly.gb);
-    if (l == 0) break;
-    // input gradient through W and SiLU' of the previous layer's pre-activation
-    GemmArgs d{};
-    d.mode = EP_DX;
-    d.out_bf16 = m->dz[l - 1]; d.ldb = m->H;
-    d.out_t = m->dzt[l - 1]; d.ldt = B;
-    d.z = m->z[l - 1]; d.ldz = m->H;
-    r = gemm(m, gr, B, ly.wt, ly.k, B, ly.k, ly.n, d, pick_bn(ly.k));
-    if (r) return r;
-    gt = m->dzt[l - 1];
-    gr = m->dz[l - 1];
+// weights w [nout], device): written out (gw, gb), or applied when `adam` is given.
+int train_batch(mpcmd_mlp* m, const float* x, const float* t, const float* w, const AdamArgs* adam) {
+  const int B = m->B, L = m->L;
+  InferArgs a{};
+  a.layers = L; a.H = m->H; a.n_in = m->cfg.n_in; a.rows = B;
+  a.tiles = infer_tiles(m); a.tail_n = infer_tail(m);
+  a.n_out = m->nout; a.npad = m->npad;
+  a.x = x; a.t = t; a.w = w;
+  a.inv_rows = (B & (B - 1)) == 0 ? 1.f / (float)B : 0.f;
+  a.bias_out = m->layers[L].b;
+  for (int l = 0; l < L; ++l) { a.bias[l] = m->layers[l].b; a.zt[l] = m->zt[l]; a.at[l] = m->ht[l]; }
+  a.xt = m->x0t; a.dy = m->dy; a.dyt = m->dyt;
+  a.loss = m->loss_part; a.err = m->err;
+  const int grid = chain_grid(m, B, a);
+  k_chain<FORWARD, 4><<<grid, INF_THREADS, INF_SMEM, m->st>>>(m->maps, a);
+  DxArgs d{};
+  d.rows = B; d.H = m->H; d.nk = (m->nout + BK - 1) / BK;
+  d.zt = m->zt[L - 1]; d.dz = m->dz; d.dzt = m->dzt[L - 1];
+  d.loss = m->loss_part; d.n_loss = grid * INF_EPI; d.loss_out = m->loss;
+  d.err = m->err;
+  launch_early(k_dx, std::min((B / BM) * (m->H / 32), m->sms), DxPipe::THREADS, DxPipe::bytes(0), m->st, m->dx_a, m->dx_b,
+               d);
+  if (L > 1) {
+    InferArgs r{};
+    r.layers = L - 1; r.H = m->H; r.rows = B;
+    r.dz = m->dz; r.err = m->err;
+    for (int j = 0; j + 1 < L; ++j) { r.zt[j] = m->zt[L - 2 - j]; r.at[j] = m->dzt[L - 2 - j]; }
+    const int rg = chain_grid(m, B, r);
+    launch_early(k_chain<BACKWARD, 4>, rg, INF_THREADS, INF_SMEM, m->st, m->back, r);
   }
+  DwArgs g = m->dw;
+  if (adam) g.adam = *adam;
+  const int dg = std::min(g.units, m->sms);
+  launch_early(adam ? k_dw<true> : k_dw<false>, dg, DwPipe::THREADS, DW_SMEM, m->st, m->dw_maps, g);
   return cudaPeekAtLastError() == cudaSuccess ? MPCMD_OK : MPCMD_ERR_CUDA;
 }
 
@@ -1236,29 +1483,21 @@ int64_t logical_count(const mpcmd_mlp* m) {
   return c;
 }
 
+// Tensors to the logical layout or from it: the padding stays on the device.
 int copy_params(mpcmd_mlp* m, float* host, bool to_host, bool grads) {
   int64_t off = 0;
   for (Layer& ly : m->layers) {
-    std::vector<float> w((size_t)ly.n * ly.k, 0.f), b((size_t)ly.n, 0.f);
     float* dw = grads ? ly.gw : ly.w;
     float* db = grads ? ly.gb : ly.b;
-    if (to_host) {
-      if (cudaMemcpy(w.data(), dw, 4 * w.size(), cudaMemcpyDeviceToHost) != cudaSuccess) return MPCMD_ERR_CUDA;
-      if (cudaMemcpy(b.data(), db, 4 * b.size(), cudaMemcpyDeviceToHost) != cudaSuccess) return MPCMD_ERR_CUDA;
-      for (int i = 0; i < ly.n_real; ++i)
-        for (int j = 0; j < ly.k_real; ++j) host[off + (int64_t)i * ly.k_real + j] = w[(size_t)i * ly.k + j];
-      off += (int64_t)ly.n_real * ly.k_real;
-      for (int i = 0; i < ly.n_real; ++i) host[off + i] = b[i];
-      off += ly.n_real;
-    } else {
-      for (int i = 0; i < ly.n_real; ++i)
-        for (int j = 0; j < ly.k_real; ++j) w[(size_t)i * ly.k + j] = host[off + (int64_t)i * ly.k_real + j];
-      off += (int64_t)ly.n_real * ly.k_real;
-      for (int i = 0; i < ly.n_real; ++i) b[i] = host[off + i];
-      off += ly.n_real;
-      if (cudaMemcpy(dw, w.data(), 4 * w.size(), cudaMemcpyHostToDevice) != cudaSuccess) return MPCMD_ERR_CUDA;
-      if (cudaMemcpy(db, b.data(), 4 * b.size(), cudaMemcpyHostToDevice) != cudaSuccess) return MPCMD_ERR_CUDA;
-    }
+    const size_t hp = 4 * (size_t)ly.k_real, dp = 4 * (size_t)ly.k;
+    float* hw = host + off;
+    float* hb = hw + (int64_t)ly.n_real * ly.k_real;
+    const cudaError_t e1 = to_host ? cudaMemcpy2D(hw, hp, dw, dp, hp, ly.n_real, cudaMemcpyDeviceToHost)
+                                   : cudaMemcpy2D(dw, dp, hw, hp, hp, ly.n_real, cudaMemcpyHostToDevice);
+    const cudaError_t e2 = to_host ? cudaMemcpy(hb, db, 4 * (size_t)ly.n_real, cudaMemcpyDeviceToHost)
+                                   : cudaMemcpy(db, hb, 4 * (size_t)ly.n_real, cudaMemcpyHostToDevice);
+    if (e1 != cudaSuccess || e2 != cudaSuccess) return MPCMD_ERR_CUDA;
+    off += (int64_t)ly.n_real * ly.k_real + ly.n_real;
   }
   return MPCMD_OK;
 }
@@ -1306,30 +1545,37 @@ int mpcmd_mlp_create(const mpcmd_mlp_config* cfg, mpcmd_mlp** out) {
     m->layers.push_back(ly);
   }
   const int64_t BH = (int64_t)m->B * m->H;
-  s |= m->alloc(m->x0, (int64_t)m->B * m->kin);
   s |= m->alloc(m->x0t, (int64_t)m->B * m->kin);
-  m->h.resize(m->L); m->ht.resize(m->L); m->z.resize(m->L); m->dz.resize(m->L); m->dzt.resize(m->L);
+  m->ht.resize(m->L); m->zt.resize(m->L); m->dzt.resize(m->L);
   for (int l = 0; l < m->L && !s; ++l) {
-    s |= m->alloc(m->h[l], BH);
     s |= m->alloc(m->ht[l], BH);
-    s |= m->alloc(m->z[l], BH);
-    s |= m->alloc(m->dz[l], BH);
+    s |= m->alloc(m->zt[l], BH);
     s |= m->alloc(m->dzt[l], BH);
   }
+  s |= m->alloc(m->dz, BH);
   s |= m->alloc(m->dy, (int64_t)m->B * m->npad);
   s |= m->alloc(m->dyt, (int64_t)m->B * m->npad);
-  s |= m->alloc(m->yb, (int64_t)m->B * m->nout);
-  s |= m->alloc(m->dloss, 1);
-  if (s || cudaHostAlloc(reinterpret_cast<void**>(&m->err), sizeof(int), cudaHostAllocDefault) != cudaSuccess) {
+  if (s || cudaHostAlloc(reinterpret_cast<void**>(&m->err), sizeof(int), cudaHostAllocDefault) != cudaSuccess ||
+      cudaHostAlloc(reinterpret_cast<void**>(&m->loss), sizeof(double), cudaHostAllocDefault) != cudaSuccess) {
     delete m;
     return MPCMD_ERR_ALLOC;
   }
   *m->err = 0;
+  *m->loss = 0.0;
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess ||
-      cudaDeviceGetAttribute(&m->sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-      !allow_smem<256>() || !allow_smem<128>() || !allow_smem<64>() ||
-      !allow_infer<16>() || !allow_infer<8>() || !allow_infer<4>() || !make_infer_maps(m)) {
+      cudaDeviceGetAttribute(&m->sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
+    delete m;
+    return MPCMD_ERR_CUDA;
+  }
+  if (m->alloc(m->loss_part, (int64_t)std::max(m->sms, 2) * INF_EPI) != MPCMD_OK) {
+    delete m;
+    return MPCMD_ERR_ALLOC;
+  }
+  if (!allow_chain<INFER, 16>() || !allow_chain<INFER, 8>() || !allow_chain<INFER, 4>() ||
+      !allow_chain<FORWARD, 4>() || !allow_chain<BACKWARD, 4>() ||
+      cudaFuncSetAttribute(k_dx, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DxPipe::bytes(0)) != cudaSuccess ||
+      !allow_dw<true>() || !allow_dw<false>() || !make_infer_maps(m) || !make_train_maps(m)) {
     delete m;
     return MPCMD_ERR_CUDA;
   }
@@ -1359,6 +1605,10 @@ int mpcmd_mlp_get_params(mpcmd_mlp* m, float* host) {
 int mpcmd_mlp_set_params(mpcmd_mlp* m, const float* host) {
   if (!m || !host) return MPCMD_ERR_CONFIG;
   if (cudaStreamSynchronize(m->st) != cudaSuccess) return MPCMD_ERR_CUDA;
+  // (zero padding, whatever training left there: infinite activations make it NaN)
+  for (Layer& ly : m->layers)
+    if (cudaMemset(ly.w, 0, 4 * (size_t)ly.n * ly.k) != cudaSuccess || cudaMemset(ly.b, 0, 4 * (size_t)ly.n) != cudaSuccess)
+      return MPCMD_ERR_CUDA;
   int r = copy_params(m, const_cast<float*>(host), false, false);
   if (r) return r;
   for (Layer& ly : m->layers) {   // a new starting point: fresh moments
@@ -1381,31 +1631,25 @@ int mpcmd_mlp_forward(mpcmd_mlp* m, const float* x, int64_t rows, float* y) {
 
 int mpcmd_mlp_gradients(mpcmd_mlp* m, const float* x, const float* t, const float* w, float* grads, double* loss) {
   if (!m || !x || !t || !w) return MPCMD_ERR_CONFIG;
-  int r = backward(m, x, t, w);
+  int r = train_batch(m, x, t, w, nullptr);
   if (r) return r;
   if ((r = status_of(m))) return r;
-  if (loss && cudaMemcpy(loss, m->dloss, sizeof(double), cudaMemcpyDeviceToHost) != cudaSuccess) return MPCMD_ERR_CUDA;
+  if (loss) *loss = *m->loss;
   return grads ? copy_params(m, grads, true, true) : MPCMD_OK;
 }
 
 int mpcmd_mlp_train_step(mpcmd_mlp* m, const float* x, const float* t, const float* w, double* loss) {
   if (!m || !x || !t || !w) return MPCMD_ERR_CONFIG;
-  int r = backward(m, x, t, w);
+  AdamArgs a;
+  a.lr = (float)m->cfg.lr; a.b1 = (float)m->cfg.beta1; a.b2 = (float)m->cfg.beta2; a.eps = (float)m->cfg.eps;
+  a.c1 = (float)(1.0 - std::pow(m->cfg.beta1, (double)(m->step + 1)));
+  a.c2 = (float)(1.0 - std::pow(m->cfg.beta2, (double)(m->step + 1)));
+  int r = train_batch(m, x, t, w, &a);
   if (r) return r;
   m->step += 1;
-  const float b1 = (float)m->cfg.beta1, b2 = (float)m->cfg.beta2;
-  const float c1 = (float)(1.0 - std::pow(m->cfg.beta1, (double)m->step));
-  const float c2 = (float)(1.0 - std::pow(m->cfg.beta2, (double)m->step));
-  for (Layer& ly : m->layers) {
-    k_adam<<<512, 256, 0, m->st>>>(ly.w, ly.gw, ly.mw, ly.vw, (int64_t)ly.n * ly.k, ly.k, (float)m->cfg.lr, b1, b2,
-                                    (float)m->cfg.eps, c1, c2, ly.wb, ly.wt, ly.n);
-    k_adam<<<16, 256, 0, m->st>>>(ly.b, ly.gb, ly.mb, ly.vb, ly.n, 1, (float)m->cfg.lr, b1, b2, (float)m->cfg.eps,
-                                   c1, c2, nullptr, nullptr, ly.n);
-  }
-  if (cudaPeekAtLastError() != cudaSuccess) return MPCMD_ERR_CUDA;
   if (loss) {
     if ((r = status_of(m))) return r;
-    if (cudaMemcpy(loss, m->dloss, sizeof(double), cudaMemcpyDeviceToHost) != cudaSuccess) return MPCMD_ERR_CUDA;
+    *loss = *m->loss;
   }
   return MPCMD_OK;
 }
