@@ -137,9 +137,8 @@ struct EDev {
   int n_ctiles;
   STile* stile;            // shell tiles of every replica
   uint32_t* st_prefix;     // [R] first shell tile of each replica
-  uint32_t* rt_need;       // [R] rebuild tiles of each replica (0 when it does not rebuild)
-  uint32_t* rt_prefix;     // [R + 1] first rebuild tile of each replica (0 tiles when it does not rebuild)
-  int tile;                // particles per tile
+  uint32_t* rt_need;       // [R] rebuild units of each replica (0 when it does not rebuild)
+  uint32_t* rt_prefix;     // [R + 1] first rebuild unit of each replica
   // samples
   float* axes;             // [R * hist * 3]
   int hist;
@@ -410,13 +409,14 @@ __device__ __forceinline__ void block_scan(unsigned* part, unsigned v) {
   }
 }
 
-// Rebuild tiles of a replica of n particles.
+// A rebuild's work is dealt to the blocks in units of REB_UNIT particles.
+constexpr int REB_UNIT = 256;
 template <typename T>
-__device__ __forceinline__ uint32_t rebuild_tiles(const EDev<T>& d, const Rep<T>& R) {
-  return ((uint32_t)R.n + (uint32_t)d.tile - 1u) / (uint32_t)d.tile;
+__device__ __forceinline__ uint32_t rebuild_units(const Rep<T>& R) {
+  return ((uint32_t)R.n + (uint32_t)REB_UNIT - 1u) / (uint32_t)REB_UNIT;
 }
 
-// Plan of a rebuild: the tiles of the rebuilding replicas (rt_need) as a
+// Plan of a rebuild: the units of the rebuilding replicas (rt_need) as a
 // prefix over replicas (one block, at most 256 threads).  rt_need may have been
 // written by other blocks of this launch.
 template <typename T>
@@ -447,7 +447,7 @@ template <typename T>
 __global__ void k_ens_plan(EDev<T> d) {
   __shared__ unsigned part[256];
   for (int r = threadIdx.x; r < d.R; r += blockDim.x)
-    d.rt_need[r] = d.dyn[r].rebuild ? rebuild_tiles(d, d.rep[r]) : 0u;
+    d.rt_need[r] = d.dyn[r].rebuild ? rebuild_units(d.rep[r]) : 0u;
   __threadfence();
   __syncthreads();
   write_plan(d, part);
@@ -526,27 +526,60 @@ __device__ __forceinline__ void finish_rebuild(const EDev<T>& d, int shell_block
   write_shell_tiles(d, shell_block, part);
 }
 
+// A particle's state, loaded (zeros past the end) ahead of its use: the loops
+// below fetch the next particle while they work on one.
 template <typename T>
-__global__ void __launch_bounds__(MAX_BLOCK) k_ens_rebuild(EDev<T> d, int mode, int shell_block, int advance_step) {
+struct ParticleIn {
+  uint32_t cell;
+  T ox, oy, oz, vx, vy, vz;
+  uint8_t f;
+  __device__ __forceinline__ void load(const EDev<T>& d, int64_t i, int64_t hi) {
+    const bool ok = i < hi;
+    cell = ok ? d.cell[i] : 0u;
+    ox = ok ? d.ox[i] : (T)0; oy = ok ? d.oy[i] : (T)0; oz = ok ? d.oz[i] : (T)0;
+    vx = ok ? d.vx[i] : (T)0; vy = ok ? d.vy[i] : (T)0; vz = ok ? d.vz[i] : (T)0;
+    f = ok ? d.flag[i] : (uint8_t)0;
+  }
+};
+
+// Bound by the 46 bytes it reads and writes of a rebuilding replica's particles,
+// and by how evenly they are dealt: the blocks share the units of all rebuilding
+// replicas out in contiguous parts (tiles of 4,096 in turn left a third wave half
+// empty and cost a search, two barriers and an atomic each), fetch one particle
+// ahead and keep to the registers of four blocks an SM.  256 replicas, 10 of them
+// rebuilding in an MD step: 57 us a step on GB300 (65 before; tiles of 1,024: 90).
+template <typename T>
+__global__ void __launch_bounds__(MAX_BLOCK, sizeof(T) == 4 ? 4 : 1)
+    k_ens_rebuild(EDev<T> d, int mode, int shell_block, int advance_step) {
   __shared__ T red[32];
   __shared__ unsigned part[MAX_BLOCK];
-  const unsigned ntiles = d.rt_prefix[d.R];
+  const unsigned units = d.rt_prefix[d.R];
   if (advance_step && blockIdx.x == 0 && threadIdx.x == 0) d.g->cstep += 1;   // (nothing in this launch reads it)
-  for (unsigned t = blockIdx.x; t < ntiles; t += gridDim.x) {
-    const int r = tile_rep(d.rt_prefix, d.R, t);
+  unsigned u = (unsigned)((uint64_t)units * blockIdx.x / gridDim.x);
+  const unsigned u_end = (unsigned)((uint64_t)units * (blockIdx.x + 1) / gridDim.x);
+  const bool works = u < u_end;
+  while (u < u_end) {
+    // this block's part of one replica
+    const int r = tile_rep(d.rt_prefix, d.R, u);
     Dyn<T>& y = d.dyn[r];
     const Rep<T>& R = d.rep[r];
-    const int64_t tlo = R.poff + (int64_t)(t - d.rt_prefix[r]) * d.tile;
-    const int64_t thi = min(tlo + (int64_t)d.tile, R.poff + R.n);
+    const unsigned r0 = d.rt_prefix[r], v = min(u_end, d.rt_prefix[r + 1]);
+    const int64_t tlo = R.poff + (int64_t)(u - r0) * REB_UNIT;
+    const int64_t thi = min(R.poff + (int64_t)(v - r0) * REB_UNIT, R.poff + R.n);
+    u = v;
     const KParams<T>& kp = R.kp;
     const int tc = y.time_count;
     const SphereRel<T> sC = y.srel[0], sN = y.srel[1];
     T vmax = (T)0;
+    ParticleIn<T> next;
+    next.load(d, tlo + threadIdx.x, thi);
     for (int64_t i = tlo + threadIdx.x; i < thi; i += blockDim.x) {
-      uint32_t cell = d.cell[i];
-      T ox = d.ox[i], oy = d.oy[i], oz = d.oz[i];
-      T vx = d.vx[i], vy = d.vy[i], vz = d.vz[i];
-      uint8_t f = d.flag[i];
+      uint32_t cell = next.cell;
+      T ox = next.ox, oy = next.oy, oz = next.oz;
+      T vx = next.vx, vy = next.vy, vz = next.vz;
+      uint8_t f = next.f;
+      const uint8_t f0 = f;
+      next.load(d, i + blockDim.x, thi);
       if ((mode & M_LAZY) && !(f & E_IN) && tc > 0) {
         stream_one(kp, (const uint8_t*)nullptr, cell, ox, oy, oz, vx, vy, vz, f, true, tc);
         d.cell[i] = cell;
@@ -558,7 +591,7 @@ __global__ void __launch_bounds__(MAX_BLOCK) k_ens_rebuild(EDev<T> d, int mode, 
         const T dN = sep2(kp, cell, ox, oy, oz, sN, dx, dy, dz);
         const int mask = (dC <= kp.full2[0] ? 1 : 0) | (dN <= kp.full2[1] ? 2 : 0);
         f = mask ? (uint8_t)(f | E_IN) : (uint8_t)(f & ~E_IN);
-        d.flag[i] = f;
+        if (f != f0) d.flag[i] = f;
         vmax = fmax(vmax, vx * vx + vy * vy + vz * vz);
         if (mask) {
           cg::coalesced_group grp = cg::coalesced_threads();
@@ -587,7 +620,7 @@ __global__ void __launch_bounds__(MAX_BLOCK) k_ens_rebuild(EDev<T> d, int mode, 
   }
   // the last of the blocks that had work finishes the rebuild (most MD steps
   // rebuild no replica and end here)
-  if ((mode & M_LISTS) && blockIdx.x < ntiles && last_block(&d.g->arrived[1], min(ntiles, gridDim.x)))
+  if ((mode & M_LISTS) && works && last_block(&d.g->arrived[1], min(units, gridDim.x)))
     finish_rebuild(d, shell_block, part);
 }
 
@@ -853,7 +886,7 @@ __global__ void k_ens_dimer(EDev<T> d, int mode, int rattle_max) {
       const double thr = (double)kp.msd_thr;
       const bool rb = maxv > thr || tc == y.time_penetrate || step % (unsigned)d.mpc_every == 0u;
       y.maxmsd = 0ull;
-      d.rt_need[r] = rb ? rebuild_tiles(d, R) : 0u;
+      d.rt_need[r] = rb ? rebuild_units(R) : 0u;
       if (rb) {
         y.rebuild = 1;
         y.n_shell = 0;
@@ -869,12 +902,17 @@ __global__ void k_ens_dimer(EDev<T> d, int mode, int rattle_max) {
 }
 
 // ------------------------------------------------------------ collision ----
+// Bound by latency (31 warps an SM were 47 % busy): the next particle's 29 bytes
+// are on their way while the warp adds up its runs, and the sums stop at the
+// longest run of the warp.  133 million particles of 256 replicas: 1.48 ms on
+// GB300 (1.78 before; the 33 bytes a particle take 0.66).
 // mpc_rotation_mod.f95:110-160 (shifted cell of every particle, collision
 // sums) fused with distribute_mod.f95:95-182 (per-species counts and first
 // members on the unshifted cells, skipping the particles inside a sphere
 // cutoff; outside-list members order before inside-list members).
 template <typename T>
-__global__ void __launch_bounds__(MAX_BLOCK) k_ens_collide(EDev<T> d) {
+__global__ void __launch_bounds__(MAX_BLOCK, sizeof(T) == 4 ? 4 : 1)
+    k_ens_collide(EDev<T> d) {
   for (int t = blockIdx.x; t < d.n_ptiles; t += gridDim.x) {
     const uint32_t r = d.pt_rep[t];
     const Rep<T>& R = d.rep[r];
@@ -889,17 +927,21 @@ __global__ void __launch_bounds__(MAX_BLOCK) k_ens_collide(EDev<T> d) {
     // every lane of a warp takes part in every iteration (the run
     // aggregation shuffles over the whole warp); lanes past the tile end
     // carry a key of their own and nothing to add
-    for (int64_t i0 = d.pt_lo[t]; i0 < d.pt_hi[t]; i0 += blockDim.x) {
+    const int64_t hi = d.pt_hi[t];
+    ParticleIn<T> next;
+    next.load(d, d.pt_lo[t] + threadIdx.x, hi);
+    for (int64_t i0 = d.pt_lo[t]; i0 < hi; i0 += blockDim.x) {
       const int64_t i = i0 + threadIdx.x;
-      const bool valid = i < d.pt_hi[t];
+      const bool valid = i < hi;
+      const ParticleIn<T> me = next;
+      next.load(d, i + blockDim.x, hi);
       uint32_t key = 0xFFFFFFFFu - (uint32_t)lane, cid = 0xFFFFFFFFu - (uint32_t)lane;
-      T vx = (T)0, vy = (T)0, vz = (T)0;
-      unsigned cadd = 0u;
+      T vx = me.vx, vy = me.vy, vz = me.vz;
+      int sp = -1;
       if (valid) {
-        const uint32_t cell = d.cell[i];
-        const T ox = d.ox[i], oy = d.oy[i], oz = d.oz[i];
-        const uint8_t f = d.flag[i];
-        vx = d.vx[i]; vy = d.vy[i]; vz = d.vz[i];
+        const uint32_t cell = me.cell;
+        const T ox = me.ox, oy = me.oy, oz = me.oz;
+        const uint8_t f = me.f;
         key = shifted_key(kp, cell, ox, oy, oz, sx, sy, sz);
         d.pkey[i] = key;
         bool bulk = true;
@@ -910,9 +952,8 @@ __global__ void __launch_bounds__(MAX_BLOCK) k_ens_collide(EDev<T> d) {
             bulk = false;
         }
         if (bulk) {
-          const int sp = f & FLAG_SPECIES;
+          sp = f & FLAG_SPECIES;
           cid = unshifted_id(kp.lx, kp.ly, cell);
-          cadd = 1u << (8 * sp);
           // only the first B of a cell is ever relabelled (reaction_mod.f95:59)
           if (sp == 1) atomicMin(&d.dfirst[4 * (R.coff + cid) + 1], ((f & E_IN) ? 0x80000000u : 0u) | (uint32_t)i);
         }
@@ -924,7 +965,7 @@ __global__ void __launch_bounds__(MAX_BLOCK) k_ens_collide(EDev<T> d) {
         const unsigned heads = __ballot_sync(full, lane == 0 || prev != key);
         const int start = 31 - __clz(heads & (0xffffffffu >> (31 - lane)));
         T c = valid ? (T)1 : (T)0;
-        for (int o = 1; o < 32; o <<= 1) {
+        for (int o = 1; o < 32 && __any_sync(full, lane - o >= start); o <<= 1) {
           const T c2 = __shfl_up_sync(full, c, o), x2 = __shfl_up_sync(full, vx, o);
           const T y2 = __shfl_up_sync(full, vy, o), z2 = __shfl_up_sync(full, vz, o);
           if (lane - o >= start) { c += c2; vx += x2; vy += y2; vz += z2; }
@@ -945,12 +986,15 @@ __global__ void __launch_bounds__(MAX_BLOCK) k_ens_collide(EDev<T> d) {
         const uint32_t prev = __shfl_up_sync(full, cid, 1);
         const unsigned heads = __ballot_sync(full, lane == 0 || prev != cid);
         const int start = 31 - __clz(heads & (0xffffffffu >> (31 - lane)));
-        for (int o = 1; o < 32; o <<= 1) {
-          const unsigned a2 = __shfl_up_sync(full, cadd, o);
-          if (lane - o >= start) cadd += a2;
-        }
+        unsigned has[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) has[q] = __ballot_sync(full, sp == q);
         const bool tail = lane == 31 || ((heads >> (lane + 1)) & 1u);
-        if (tail && cadd) {
+        if (tail && sp >= 0) {   // (a run's members all count, or it is one lane past the end or inside a sphere)
+          const unsigned run = (0xffffffffu >> (31 - lane)) & (0xffffffffu << start);
+          unsigned cadd = 0u;
+#pragma unroll
+          for (int q = 0; q < 4; ++q) cadd |= (unsigned)__popc(has[q] & run) << (8 * q);
           const unsigned old = atomicAdd(&d.dcnt[R.coff + cid], cadd);
           for (int sp = 0; sp < 4; ++sp)
             if (((old >> (8 * sp)) & 255u) + ((cadd >> (8 * sp)) & 255u) > (unsigned)kp.cell_capacity)
@@ -1043,16 +1087,38 @@ __global__ void __launch_bounds__(MAX_BLOCK) k_ens_cells(EDev<T> d) {
 }
 
 // mpc_rotation_mod.f95:205-228: v <- v_cm + R (v - v_cm) about the cell's axis.
+// Bound by the latency of the cell's entry behind the particle's key: two
+// particles a thread in flight, entries read in pairs of values, all the blocks
+// that fit: 0.73 ms for 133 million particles on GB300 (1.13 with one particle
+// and six loads; four particles 0.75).
+constexpr int ROT_UNROLL = 2;   // particles per thread with their loads in flight together
 template <typename T>
 __global__ void __launch_bounds__(MAX_BLOCK) k_ens_rotate(EDev<T> d) {
   for (int t = blockIdx.x; t < d.n_ptiles; t += gridDim.x) {
     const uint32_t r = d.pt_rep[t];
     const Rep<T>& R = d.rep[r];
-    for (int64_t i = d.pt_lo[t] + threadIdx.x; i < d.pt_hi[t]; i += blockDim.x) {
-      const T* ro = d.rot + 6 * (R.coff + d.pkey[i]);
-      T vx = d.vx[i], vy = d.vy[i], vz = d.vz[i];
-      rotate_v(R.kp, ro, vx, vy, vz);
-      d.vx[i] = vx; d.vy[i] = vy; d.vz[i] = vz;
+    const int64_t hi = d.pt_hi[t];
+    const T* rot = d.rot + 6 * R.coff;
+    for (int64_t i0 = d.pt_lo[t] + threadIdx.x; i0 < hi; i0 += ROT_UNROLL * (int64_t)blockDim.x) {
+      uint32_t key[ROT_UNROLL];
+      T vx[ROT_UNROLL], vy[ROT_UNROLL], vz[ROT_UNROLL], ro[ROT_UNROLL][6];
+#pragma unroll
+      for (int u = 0; u < ROT_UNROLL; ++u) {
+        const int64_t i = i0 + u * (int64_t)blockDim.x;
+        const bool ok = i < hi;
+        key[u] = ok ? d.pkey[i] : 0u;
+        vx[u] = ok ? d.vx[i] : (T)0; vy[u] = ok ? d.vy[i] : (T)0; vz[u] = ok ? d.vz[i] : (T)0;
+      }
+#pragma unroll
+      for (int u = 0; u < ROT_UNROLL; ++u) load_rot(rot, key[u], ro[u]);
+#pragma unroll
+      for (int u = 0; u < ROT_UNROLL; ++u) {
+        const int64_t i = i0 + u * (int64_t)blockDim.x;
+        if (i < hi) {
+          rotate_v(R.kp, ro[u], vx[u], vy[u], vz[u]);
+          d.vx[i] = vx[u]; d.vy[i] = vy[u]; d.vz[i] = vz[u];
+        }
+      }
     }
   }
 }
@@ -1123,9 +1189,10 @@ __global__ void k_ens_sort_gather(EDev<T> d, int64_t ntot) {
 // particle cost some 25 instructions of the FP64 pipe, which set the time:
 // 3.6 ms for the 133 million particles of 256 replicas.  The four sums run
 // as PairSum (exact terms, about 2^-45 relative error) down to one value per
-// warp, the counts as integers, and only the warps' results are added in
-// FP64: 0.74 ms on GB300 (2.4 TB/s).
-constexpr int OBS_UNROLL = 4;   // particles per thread with their loads in flight together
+// warp, the counts as integers, and only the warps' results are added in FP64,
+// once for a block's part of a replica: 0.51 ms on GB300 (3.4 TB/s; 0.74 with
+// the sums closed after every tile and blocks for the rebuild's registers).
+constexpr int OBS_UNROLL = 2;   // particles per thread with their loads in flight together
 
 __device__ __forceinline__ void obs_tile_f32(const EDev<float>& d, int64_t lo, int64_t hi, const double* m,
                                              double* out) {
@@ -1201,9 +1268,18 @@ template <typename T>
 __global__ void __launch_bounds__(MAX_BLOCK) k_ens_observables(EDev<T> d, const double* mass /* [R * 4] */,
                                                                double* out) {
   if constexpr (sizeof(T) == 4) {
-    for (int t = blockIdx.x; t < d.n_ptiles; t += gridDim.x) {
-      const uint32_t r = d.pt_rep[t];
-      obs_tile_f32(d, d.pt_lo[t], d.pt_hi[t], mass + 4 * r, out + 8 * (size_t)r);
+    // neighbouring tiles to a block: one or two replicas' parts, each summed once
+    const int t0 = (int)((int64_t)d.n_ptiles * blockIdx.x / gridDim.x);
+    const int t1 = (int)((int64_t)d.n_ptiles * (blockIdx.x + 1) / gridDim.x);
+    if (t0 < t1) {
+      const int64_t end = d.pt_hi[t1 - 1];
+      uint32_t r = d.pt_rep[t0];
+      for (int64_t lo = d.pt_lo[t0]; lo < end; lo = d.rep[r].poff) {
+        const int64_t hi = min(end, d.rep[r].poff + d.rep[r].n);
+        obs_tile_f32(d, lo, hi, mass + 4 * r, out + 8 * (size_t)r);
+        if (hi == end) break;
+        ++r;
+      }
     }
   } else {
     __shared__ double red[8 * 32];

@@ -44,6 +44,7 @@ struct Ensemble : EnsembleBase {
   int64_t graph_launches = 0;
   int tile = 2048, block = 256, sblock = 256;
   int g_part = 0, g_shell = 0, nsm = 0;
+  int g_collide = 0, g_cells = 0, g_rotate = 0, g_obs = 0;
   int64_t cstep = 0;
   bool prepared = false, need_advance = true, vel_pending = false;
   int64_t launches = 0, replays = 0, field_samples = 0;
@@ -222,7 +223,6 @@ struct Ensemble : EnsembleBase {
     if (pt < 64 || pt > (1 << 20) || b < 32 || b > MAX_BLOCK || b % 32 || sb < 32 || sb > MAX_BLOCK || sb % 32)
       return MPCMD_ERR_CONFIG;
     tile = pt; block = b; sblock = sb;
-    d.tile = pt;
     std::vector<uint32_t> prep, crep;
     std::vector<int64_t> plo, phi, clo, chi;
     for (int r = 0; r < R; ++r) {
@@ -256,6 +256,17 @@ struct Ensemble : EnsembleBase {
     ECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_p, k_ens_rebuild<T>, b, 0));
     ECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_s, k_ens_force<T, M_FORCE | M_ADVANCE>, sb, 0));
     g_part = nsm * std::max(occ_p, 1);
+    // the collision's kernels need fewer registers than the rebuild, and are
+    // bound by latency: as many blocks as fit (their work is tiles in turn)
+    auto fit = [&](const void* k, int* g) {
+      int occ = 0;
+      if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k, b, 0) != cudaSuccess) return false;
+      *g = nsm * std::max(occ, 1);
+      return true;
+    };
+    if (!fit((const void*)k_ens_collide<T>, &g_collide) || !fit((const void*)k_ens_cells<T>, &g_cells) ||
+        !fit((const void*)k_ens_rotate<T>, &g_rotate) || !fit((const void*)k_ens_observables<T>, &g_obs))
+      return MPCMD_ERR_CUDA;
     g_shell = nsm * std::max(occ_s, 1);
     invalidate_graph();
     if (prepared) L_tiles();   // the lists' tiles follow the shell tile size
@@ -324,9 +335,9 @@ struct Ensemble : EnsembleBase {
     if (mpc) {
       L_force(M_FORCE);
       L_dimer(M_VEL);
-      k_ens_collide<T><<<g_part, block, 0, st>>>(d);
-      k_ens_cells<T><<<g_part, block, 0, st>>>(d);
-      k_ens_rotate<T><<<g_part, block, 0, st>>>(d);
+      k_ens_collide<T><<<g_collide, block, 0, st>>>(d);
+      k_ens_cells<T><<<g_cells, block, 0, st>>>(d);
+      k_ens_rotate<T><<<g_rotate, block, 0, st>>>(d);
       launches += 3;
       need_advance = true;
     } else if (last) {
@@ -543,7 +554,7 @@ struct Ensemble : EnsembleBase {
   int observables(mpcmd_obs* out) override {
     if (!out) return MPCMD_ERR_CONFIG;
     ECK(cudaMemsetAsync(d_obs, 0, 8 * 8 * (size_t)R, st));
-    k_ens_observables<T><<<g_part, block, 0, st>>>(d, d_mass, d_obs);
+    k_ens_observables<T><<<g_obs, block, 0, st>>>(d, d_mass, d_obs);
     ++launches;
     std::vector<double> o(8 * (size_t)R);
     ECK(cudaMemcpyAsync(o.data(), d_obs, 8 * o.size(), cudaMemcpyDeviceToHost, st));
