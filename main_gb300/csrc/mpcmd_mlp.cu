@@ -18,7 +18,8 @@
 //                      depend on one another, with Adam in the epilogue.
 // (A step of 256 rows through four hidden layers of 256 to 2,050 outputs: 87 us
 // a call, about 60 of them kernels, where 31 launches through memory took 305.
-// All of it is latency: a contraction's MMAs wait for one another.)
+// All of it is latency: a contraction's MMAs wait for one another.  Each kernel
+// starts while the one before it runs; 97 us without that.)
 // Every contraction is C[M, N] = A[M, K] . B[N, K]^T with both operands BF16
 // and K-major.
 //
@@ -372,13 +373,6 @@ __device__ __forceinline__ void copy_async(void* dst, const void* src) {
   else asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
 }
 
-// A training step's kernels are launched early (programmatic dependent launch):
-// a kernel lets the next one start once it holds its tensor memory, and the next
-// one sets itself up, then waits until the kernel before it has ended with its
-// results visible.
-__device__ __forceinline__ void let_next_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-
 // Consecutive columns of a lane's row, packed in pairs, as a column each of a
 // transposed matrix (consecutive lanes: consecutive rows).
 template <int N>
@@ -475,8 +469,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(INF_THREADS, 1)
   cluster_sync();   // both CTAs' barriers exist before either signals them
   tmem_fence_after();
   const uint32_t tmem = *tmem_slot;
-  if constexpr (MODE != INFER) let_next_start();
-  if constexpr (MODE == BACKWARD) wait_for_previous();
+  if constexpr (MODE != INFER) mpcmd::let_next_start();
+  if constexpr (MODE == BACKWARD) mpcmd::wait_for_previous();
 
   if (warp == 0) {
     if (lane == 0) {
@@ -993,8 +987,8 @@ __global__ void __launch_bounds__(DxPipe::THREADS, 1)
   __shared__ int issued;
   DxPipe p;
   p.open(smem_raw, &bail, &issued, a.err);
-  let_next_start();
-  wait_for_previous();
+  mpcmd::let_next_start();
+  mpcmd::wait_for_previous();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int tiles_n = a.H / 32, units = (a.rows / BM) * tiles_n;
   if (warp == 0) {
@@ -1108,7 +1102,7 @@ __global__ void __launch_bounds__(DwPipe::THREADS, 1)
   };
   if (warp == 0) {
     if (lane == 0) {
-      wait_for_previous();
+      mpcmd::wait_for_previous();
       int g = 0, l, mt, nt;
       for (int u = blockIdx.x; u < a.tiles && !bail; u += gridDim.x) {
         tile_of(u, l, mt, nt);
@@ -1197,7 +1191,7 @@ __global__ void __launch_bounds__(DwPipe::THREADS, 1)
         const int n0 = (u - ly.first_bias) * 64 + 4 * ew, n = n0 + (lane & 3);
         float b = 0.f, m1 = 0.f, m2 = 0.f;
         if constexpr (UPDATE) { b = ly.bw[n]; m1 = ly.bm[n]; m2 = ly.bv[n]; }
-        wait_for_previous();
+        mpcmd::wait_for_previous();
         float s[4] = {};
         const __nv_bfloat16* zp = ly.dzt + (size_t)n0 * a.rows + lane;
 #pragma unroll 4
@@ -1320,23 +1314,6 @@ int status_of(mpcmd_mlp* m) {
   return *reinterpret_cast<volatile int*>(m->err) ? MPCMD_ERR_CUDA : MPCMD_OK;
 }
 
-// A kernel that sets itself up while the one before it in the stream still runs
-// (it calls wait_for_previous; a step of 256 rows takes 87 us instead of 97).
-template <typename... P, typename... A>
-void launch_early(void (*kernel)(P...), int grid, int threads, size_t smem, cudaStream_t st, const A&... args) {
-  cudaLaunchAttribute at{};
-  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at.val.programmaticStreamSerializationAllowed = 1;
-  cudaLaunchConfig_t c{};
-  c.gridDim = dim3((unsigned)grid);
-  c.blockDim = dim3((unsigned)threads);
-  c.dynamicSmemBytes = smem;
-  c.stream = st;
-  c.attrs = &at;
-  c.numAttrs = 1;
-  cudaLaunchKernelEx(&c, kernel, args...);
-}
-
 template <int MODE, int VB>
 bool allow_chain() {
   return cudaFuncSetAttribute(k_chain<MODE, VB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)INF_SMEM) ==
@@ -1440,20 +1417,20 @@ int train_batch(mpcmd_mlp* m, const float* x, const float* t, const float* w, co
   d.zt = m->zt[L - 1]; d.dz = m->dz; d.dzt = m->dzt[L - 1];
   d.loss = m->loss_part; d.n_loss = grid * INF_EPI; d.loss_out = m->loss;
   d.err = m->err;
-  launch_early(k_dx, std::min((B / BM) * (m->H / 32), m->sms), DxPipe::THREADS, DxPipe::bytes(0), m->st, m->dx_a, m->dx_b,
-               d);
+  mpcmd::launch_next_smem(k_dx, std::min((B / BM) * (m->H / 32), m->sms), DxPipe::THREADS, DxPipe::bytes(0), m->st,
+                          m->dx_a, m->dx_b, d);
   if (L > 1) {
     InferArgs r{};
     r.layers = L - 1; r.H = m->H; r.rows = B;
     r.dz = m->dz; r.err = m->err;
     for (int j = 0; j + 1 < L; ++j) { r.zt[j] = m->zt[L - 2 - j]; r.at[j] = m->dzt[L - 2 - j]; }
     const int rg = chain_grid(m, B, r);
-    launch_early(k_chain<BACKWARD, 4>, rg, INF_THREADS, INF_SMEM, m->st, m->back, r);
+    mpcmd::launch_next_smem(k_chain<BACKWARD, 4>, rg, INF_THREADS, INF_SMEM, m->st, m->back, r);
   }
   DwArgs g = m->dw;
   if (adam) g.adam = *adam;
   const int dg = std::min(g.units, m->sms);
-  launch_early(adam ? k_dw<true> : k_dw<false>, dg, DwPipe::THREADS, DW_SMEM, m->st, m->dw_maps, g);
+  mpcmd::launch_next_smem(adam ? k_dw<true> : k_dw<false>, dg, DwPipe::THREADS, DW_SMEM, m->st, m->dw_maps, g);
   return cudaPeekAtLastError() == cudaSuccess ? MPCMD_OK : MPCMD_ERR_CUDA;
 }
 

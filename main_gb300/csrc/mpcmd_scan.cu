@@ -26,6 +26,7 @@ int debug_sync(cudaStream_t st, const char* where, int line) {
 constexpr int SCAN_TILE = 4 * TPB;
 
 __global__ void k_scan_tiles(const uint32_t* in, int64_t n, uint32_t* tile_sums) {
+  after_previous();
   __shared__ uint32_t sh[TPB / 32];
   int64_t base = (int64_t)blockIdx.x * SCAN_TILE;
   uint32_t s = 0;
@@ -69,6 +70,7 @@ __device__ uint32_t block_exclusive_scan(uint32_t v, uint32_t* total) {
 }
 
 __global__ void k_scan_apply(const uint32_t* in, uint32_t* out, int64_t n, const uint32_t* tile_offsets) {
+  after_previous();
   int64_t base = (int64_t)blockIdx.x * SCAN_TILE;
   uint32_t carry = tile_offsets[blockIdx.x];
   for (int k = 0; k < 4; ++k) {
@@ -95,16 +97,16 @@ void scan_u32(const uint32_t* in, uint32_t* out, int64_t n, uint32_t* tmp, cudaS
   int64_t tiles = (n + SCAN_TILE - 1) / SCAN_TILE;
   if (tiles <= 1) {
     cudaMemsetAsync(tmp, 0, sizeof(uint32_t), st);
-    k_scan_apply<<<1, TPB, 0, st>>>(in, out, n, tmp);
+    launch_next(k_scan_apply, 1, TPB, st, in, out, n, tmp);
     LAUNCH_COUNT();
     return;
   }
   uint32_t* sums = tmp;
   uint32_t* offs = tmp + tiles + 4;
-  k_scan_tiles<<<(unsigned)tiles, TPB, 0, st>>>(in, n, sums);
+  launch_next(k_scan_tiles, (unsigned)tiles, TPB, st, in, n, sums);
   LAUNCH_COUNT();
   scan_u32(sums, offs, tiles, offs + tiles + 4, st);
-  k_scan_apply<<<(unsigned)tiles, TPB, 0, st>>>(in, out, n, offs);
+  launch_next(k_scan_apply, (unsigned)tiles, TPB, st, in, out, n, offs);
   LAUNCH_COUNT();
 }
 
