@@ -336,7 +336,10 @@ void Launch<T>::download_convert(const Dev<T>& d, const KParams<T>& kp, double* 
 // division per coordinate, which set the time before (831 us for 2.1e7
 // particles), are taken in FP32 and repeated in FP64 only inside the error
 // band of the FP32 result, so the counts are those of the FP64 arithmetic.
-// The fields, series and axes of that box take 0.69 ms instead of 1.77.
+// The next four particles' loads are in flight meanwhile, and the few particles
+// that reach a slab are binned a full warp at a time: 99 us instead of 206 when
+// a lane that found one held its warp up.  The fields, series and axes of that
+// box take 0.57 ms instead of 1.77.
 
 // Bin of a coordinate: ceil(u / w) clamped to [1, nb], 0-based.  t = uf * iwf
 // has relative error below 3 * 2^-24 of u / w (uf, iwf and the product
@@ -371,20 +374,25 @@ __global__ void __launch_bounds__(TPB) k_concentration(Particles<T> p, KParams<T
   unsigned int na = 0u, nb = 0u;
   const float lof[3] = {(float)c.lo[0], (float)c.lo[1], (float)c.lo[2]};
   const float hif[3] = {(float)c.hi[0], (float)c.hi[1], (float)c.hi[2]};
-  auto count = [&](int64_t i, uint8_t f, uint32_t cl) {
+  auto lag_of = [&](uint8_t f) {
+    if (f & FLAG_PASSIVE) return tc;
+    return !(f & (FLAG_INLIST | FLAG_FRESH | FLAG_HOME_SHELL)) ? tc_defer : 0;
+  };
+  // Counts particle i of species 0 or 1 in the totals; whether it may lie in a slab.
+  auto reaches = [&](uint8_t f, uint32_t cl) {
     const int sp = f & FLAG_SPECIES;
-    if (sp > 1) return;
+    if (sp > 1) return false;
     if (sp == 0) ++na; else ++nb;
-    int lag = 0;
-    if (f & FLAG_PASSIVE) lag = tc;
-    else if (!(f & (FLAG_INLIST | FLAG_FRESH | FLAG_HOME_SHELL))) lag = tc_defer;
-    if (lag == 0) {
-      bool reach = false;
-      const int q[3] = {cell_x(cl), cell_y(cl), cell_z(cl)};
+    bool reach = lag_of(f) > 0;
+    const int q[3] = {cell_x(cl), cell_y(cl), cell_z(cl)};
 #pragma unroll
-      for (int k = 0; k < 3; ++k) reach |= q[k] >= c.clo[k] && q[k] <= c.chi[k];
-      if (!reach) return;
-    }
+    for (int k = 0; k < 3; ++k) reach |= q[k] >= c.clo[k] && q[k] <= c.chi[k];
+    return reach;
+  };
+  auto bin = [&](int64_t i) {
+    const uint8_t f = p.flag[i];
+    uint32_t cl = p.cell[i];
+    const int sp = f & FLAG_SPECIES, lag = lag_of(f);
     T ox = p.ox[i], oy = p.oy[i], oz = p.oz[i];
     if (lag > 0) {
       T vx = p.vx[i], vy = p.vy[i], vz = p.vz[i];
@@ -407,20 +415,53 @@ __global__ void __launch_bounds__(TPB) k_concentration(Particles<T> p, KParams<T
     if (sy) atomicAdd(&c.xz[sp][jx + (size_t)c.nx * jz], 1u);
     if (sx) atomicAdd(&c.yz[sp][jy + (size_t)c.ny * jz], 1u);
   };
+  // The few particles that reach a slab wait in a queue per warp until there is
+  // one for every lane (particle indices are below 2^31).
+  __shared__ uint32_t queues[TPB / 32][32 + 4 * 32];
+  uint32_t* queue = queues[threadIdx.x >> 5];
+  const int lane = threadIdx.x & 31;
+  const unsigned below = (1u << lane) - 1u;
+  int waiting = 0;
+  auto push = [&](bool want, int64_t i) {
+    const unsigned m = __ballot_sync(0xffffffffu, want);
+    if (want) queue[waiting + __popc(m & below)] = (uint32_t)i;
+    waiting += __popc(m);
+  };
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   const int64_t t0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, n4 = kp.n >> 2;
-  for (int64_t q = t0; q < n4; q += stride) {
+  uchar4 f_next = make_uchar4(3, 3, 3, 3);   // (a species that is not counted)
+  uint4 cl_next = make_uint4(0u, 0u, 0u, 0u);
+  auto fetch = [&](int64_t q) {
+    f_next = make_uchar4(3, 3, 3, 3);
+    if (q < n4) {
+      f_next = load4(p.flag, q << 2);
+      cl_next = *reinterpret_cast<const uint4*>(p.cell + (q << 2));
+    }
+  };
+  fetch(t0);
+  for (int64_t q = t0; q - lane < n4; q += stride) {
+    const uchar4 f = f_next;
+    const uint4 cl = cl_next;
     const int64_t i = q << 2;
-    const uchar4 f = load4(p.flag, i);
-    const uint4 cl = *reinterpret_cast<const uint4*>(p.cell + i);
-    count(i, f.x, cl.x);
-    count(i + 1, f.y, cl.y);
-    count(i + 2, f.z, cl.z);
-    count(i + 3, f.w, cl.w);
+    fetch(q + stride);
+    push(reaches(f.x, cl.x), i);
+    push(reaches(f.y, cl.y), i + 1);
+    push(reaches(f.z, cl.z), i + 2);
+    push(reaches(f.w, cl.w), i + 3);
+    if (waiting >= 32) {
+      __syncwarp();
+      do {
+        waiting -= 32;
+        bin(queue[waiting + lane]);
+      } while (waiting >= 32);
+      __syncwarp();
+    }
   }
+  __syncwarp();
+  if (lane < waiting) bin(queue[lane]);
   if (t0 < (kp.n & 3)) {
     const int64_t i = (n4 << 2) + t0;
-    count(i, p.flag[i], p.cell[i]);
+    if (reaches(p.flag[i], p.cell[i])) bin(i);
   }
   na = __reduce_add_sync(0xffffffffu, na);
   nb = __reduce_add_sync(0xffffffffu, nb);
