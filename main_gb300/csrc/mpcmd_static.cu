@@ -93,6 +93,7 @@ __device__ __forceinline__ uint32_t static_key(const KParams<double>& kp, double
 }
 
 __global__ void k_static_clear(double* acc, int64_t ncell) {
+  let_next_start();
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < ncell; c += stride) {
     double2* a = reinterpret_cast<double2*>(acc + kRec * (size_t)c);
@@ -140,6 +141,7 @@ __device__ __forceinline__ uint32_t fast_key(const KParams<double>& kp, double x
 __global__ void __launch_bounds__(kThreads) k_static_accumulate(KParams<double> kp, const double* x, const double* y,
                                                                 const double* z, const double* vx, const double* vy,
                                                                 const double* vz, int64_t n, Shift s, double* acc) {
+  after_previous();
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += stride) {
     uint32_t key = fast_key(kp, x[i], y[i], z[i], s);
@@ -185,6 +187,7 @@ __device__ __forceinline__ bool cell_map(const KParams<double>& kp, uint32_t cel
 }
 
 __global__ void __launch_bounds__(kThreads) k_static_cells(KParams<double> kp, uint32_t step, double* acc) {
+  after_previous();
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < kp.ncell_shift; i += stride) {
     double2* a = reinterpret_cast<double2*>(acc + kRec * (size_t)i);
@@ -204,6 +207,7 @@ template <bool OWN_MAP>
 __global__ void __launch_bounds__(kThreads) k_static_rotate(KParams<double> kp, const double* x, const double* y,
                                                             const double* z, double* vx, double* vy, double* vz,
                                                             int64_t n, Shift s, uint32_t step, const double* acc) {
+  wait_for_previous();   // (what follows is the caller's)
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += stride) {
     uint32_t key = fast_key(kp, x[i], y[i], z[i], s);
@@ -283,12 +287,21 @@ extern "C" int mpcmd_collide_static(const double* x, const double* y, const doub
   const int grid = (int)std::min<int64_t>(want, (int64_t)nsm * 8);
   const int tgrid = (int)std::min<int64_t>((ncs + kThreads - 1) / kThreads, (int64_t)nsm * 8);
   k_static_clear<<<tgrid, kThreads, 0, st>>>(acc, ncs);
-  k_static_accumulate<<<grid, kThreads, 0, st>>>(kp, x, y, z, vx, vy, vz, n, s, acc);
+  // Up to three blocks an SM each kernel starts while the one before it ends (1,536
+  // to 8,192 particles 14.8 us instead of 20.5, 80,000 23.6 instead of 26.7).
+  // Past that the early blocks crowd the first SMs that fall free, where they
+  // share the FP64 pipe (270,000 particles: 43.7 us instead of 33.7).
+  const bool early = grid <= 3 * nsm;
+  auto next = [&](auto kernel, int blocks, auto... args) {
+    if (early) launch_next(kernel, blocks, kThreads, st, args...);
+    else kernel<<<blocks, kThreads, 0, st>>>(args...);
+  };
+  next(k_static_accumulate, grid, kp, x, y, z, vx, vy, vz, n, s, acc);
   if (n <= kOwnMap) {
-    k_static_rotate<true><<<grid, kThreads, 0, st>>>(kp, x, y, z, vx, vy, vz, n, s, (uint32_t)step, acc);
+    next(k_static_rotate<true>, grid, kp, x, y, z, vx, vy, vz, n, s, (uint32_t)step, acc);
   } else {
-    k_static_cells<<<tgrid, kThreads, 0, st>>>(kp, (uint32_t)step, acc);
-    k_static_rotate<false><<<grid, kThreads, 0, st>>>(kp, x, y, z, vx, vy, vz, n, s, (uint32_t)step, acc);
+    next(k_static_cells, tgrid, kp, (uint32_t)step, acc);
+    next(k_static_rotate<false>, grid, kp, x, y, z, vx, vy, vz, n, s, (uint32_t)step, acc);
   }
   if (cudaPeekAtLastError() != cudaSuccess) return MPCMD_ERR_CUDA;
   return MPCMD_OK;
