@@ -881,6 +881,7 @@ struct Engine : EngineBase {
     if (nsteps <= 0) return MPCMD_OK;
     regather_shell();
     const int64_t target = cstep + nsteps;
+    bool after_dimer = false;   // the last kernel issued is the dimer step
     while (cstep < target) {
       const int64_t n = cstep + 1;
       const bool last = (n == target);
@@ -895,6 +896,7 @@ struct Engine : EngineBase {
           if (kp.ns == 0) std::swap(d.sh, d.sh2);
         }
         pb(PROF_DIMER); Launch<T>::dimer(d, kp, a, 2, w3, cfg.rattle_max_iter, st); pe();
+        after_dimer = kp.nd > 0;
         advanced = true;
       }
       time_count += 1;
@@ -918,11 +920,13 @@ struct Engine : EngineBase {
       a.mpc = mpc ? 1 : 0;
       a.rebuilt = rebuild ? 1 : 0;
       a.advance = last ? 0 : 1;
+      a.after_dimer = after_dimer && !rebuild ? 1 : 0;
       pb(PROF_FORCE); Launch<T>::force(d, kp, a, st); pe();
       if (mpc && kp.kinetics == MPCMD_KIN_SELKOV && kp.exclusion == MPCMD_EXCL_CELLS) {
         pb(PROF_AFFECTED); Launch<T>::affected(d, kp, a, st); pe();
       }
       pb(PROF_DIMER); Launch<T>::dimer(d, kp, a, 1 | (last ? 0 : 2), w3, cfg.rattle_max_iter, st); pe();
+      after_dimer = kp.nd > 0 && !mpc;
       if (mpc) {
         pb(PROF_CELLS); Launch<T>::cells(d, kp, a, 1 | (kp.kinetics ? 2 : 0), st); pe();
         // the rotated velocities hold until the next collision: the particles

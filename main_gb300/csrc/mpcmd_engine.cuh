@@ -158,6 +158,7 @@ struct StepArgs {
   int rebuilt;         // a rebuild ran in this step
   int forces_only;     // k_force: pair forces, catalysis and sphere sums without the kicks (a restart)
   int merge_only;      // rebuild pass: lazy-stream and merge only, no lists
+  int after_dimer;     // k_force: the kernel right before it in the stream is the dimer step
   int grid;            // persistent grid size of the light kernels
   int g_rebuild;       // SMs x resident blocks of k_rebuild, k_force, k_rotate_main
   int g_force;

@@ -1207,6 +1207,36 @@ constexpr int SPH_PER_BLOCK = (TPB / 32) / SPH_WARPS;
 // OWN: the owner-tag form (a template flag: the common form keeps no tag state)
 template <typename T, bool OWN>
 __global__ void __launch_bounds__(TPB, sizeof(T) == 4 ? 5 : 1) k_force(Dev<T> d, KParams<T> kp, StepArgs a) {
+  // The entry's state; after the dimer step, which writes none of it, the first
+  // entry's arrives while that ends (a period of 64 dimers between walls 1.34 ->
+  // 1.28 ms).
+  uint32_t cell = 0, idx = 0;
+  T ox = 0, oy = 0, oz = 0, vx = 0, vy = 0, vz = 0;
+  T msd0 = (T)0;   // loaded with the rest: its use at the end would wait on it
+  uint8_t fl = 0;
+  int np = 0;
+  uint4 packed = make_uint4(0u, 0u, 0u, 0u);
+  auto load = [&](int64_t j, int64_t nin) {
+    cell = 0; idx = 0; fl = 0; np = 0;
+    ox = oy = oz = vx = vy = vz = msd0 = (T)0;
+    if (j >= nin) return;
+    if (a.advance && !a.mpc) msd0 = d.sh.msd[j];
+    cell = d.sh.cell[j];
+    ox = d.sh.ox[j]; oy = d.sh.oy[j]; oz = d.sh.oz[j];
+    vx = d.sh.vx[j]; vy = d.sh.vy[j]; vz = d.sh.vz[j];
+    fl = d.sh.flag[j];
+    np = d.sh.np[j];
+    // the main index keys the catalysis draws and orders the species lists;
+    // without owner tags or the on-exit record nothing here needs the slot,
+    // so after a re-sort the entry's main index replaces it
+    idx = (d.lid && !OWN && !d.inc) ? d.sh.mid[j] : d.sh.idx[j];
+    packed = *reinterpret_cast<const uint4*>(d.sh.sph + (size_t)j * PAIRMAX);
+  };
+  bool loaded = a.after_dimer && (int)blockIdx.x < a.g_force;
+  if (loaded) {
+    const unsigned int nin = d.ctr->n_inside;
+    load(wave_first(nin, a.g_force), nin);
+  }
   after_previous();
   if (d.ctr->abort_step) return;
   if (!a.rebuilt) {
@@ -1294,29 +1324,12 @@ __global__ void __launch_bounds__(TPB, sizeof(T) == 4 ? 5 : 1) k_force(Dev<T> d,
   for (int64_t base = wave_first(nin, a.g_force) - lane; base < (int64_t)nin; base += stride) {
     const int64_t j = base + lane;
     const bool act = j < (int64_t)nin;
-    uint32_t cell = 0, idx = 0;
-    T ox = 0, oy = 0, oz = 0, vx = 0, vy = 0, vz = 0;
-    T msd0 = (T)0;   // loaded with the rest: its use at the end would wait on it
-    uint8_t fl = 0;
-    int np = 0;
-    uint16_t sphl[PAIRMAX];
-    if (act) {
-      if (a.advance && !a.mpc) msd0 = d.sh.msd[j];
-      cell = d.sh.cell[j];
-      ox = d.sh.ox[j]; oy = d.sh.oy[j]; oz = d.sh.oz[j];
-      vx = d.sh.vx[j]; vy = d.sh.vy[j]; vz = d.sh.vz[j];
-      fl = d.sh.flag[j];
-      np = d.sh.np[j];
-      // the main index keys the catalysis draws and orders the species lists;
-      // without owner tags or the on-exit record nothing here needs the slot,
-      // so after a re-sort the entry's main index replaces it
-      idx = (d.lid && !OWN && !d.inc) ? d.sh.mid[j] : d.sh.idx[j];
-      const uint4 packed = *reinterpret_cast<const uint4*>(d.sh.sph + (size_t)j * PAIRMAX);
-      sphl[0] = (uint16_t)(packed.x & 0xFFFFu); sphl[1] = (uint16_t)(packed.x >> 16);
-      sphl[2] = (uint16_t)(packed.y & 0xFFFFu); sphl[3] = (uint16_t)(packed.y >> 16);
-      sphl[4] = (uint16_t)(packed.z & 0xFFFFu); sphl[5] = (uint16_t)(packed.z >> 16);
-      sphl[6] = (uint16_t)(packed.w & 0xFFFFu); sphl[7] = (uint16_t)(packed.w >> 16);
-    }
+    if (!loaded) load(j, nin);
+    loaded = false;
+    const uint16_t sphl[PAIRMAX] = {(uint16_t)(packed.x & 0xFFFFu), (uint16_t)(packed.x >> 16),
+                                    (uint16_t)(packed.y & 0xFFFFu), (uint16_t)(packed.y >> 16),
+                                    (uint16_t)(packed.z & 0xFFFFu), (uint16_t)(packed.z >> 16),
+                                    (uint16_t)(packed.w & 0xFFFFu), (uint16_t)(packed.w >> 16)};
     // owner tag (type_B) of the particle, with owner_tags
     uint32_t own = 0, own0 = 0;
     if (OWN && act) own = own0 = d.owner[idx];
@@ -1780,8 +1793,6 @@ __device__ __forceinline__ double wrap_box(double X, double L) {
 // 7.2 us with the divisions by constants through div_const and wrap_box.
 template <typename T>
 __global__ void k_dimer_split(Dev<T> d, KParams<T> kp, StepArgs a, int mode, double w3, int rattle_max) {
-  after_previous();
-  if (d.ctr->abort_step) return;
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   const int k = t >> 2, c = t & 3;
   const unsigned gmask = 0xFu << (threadIdx.x & 28);   // this group's four lanes
@@ -1801,16 +1812,22 @@ __global__ void k_dimer_split(Dev<T> d, KParams<T> kp, StepArgs a, int mode, dou
   if (live && comp) {
     X1 = d.dpos[3 * s1 + c]; X2 = d.dpos[3 * s2 + c];
     V1 = d.dvel[3 * s1 + c]; V2 = d.dvel[3 * s2 + c];
-    F1 = d.dfrc[3 * s1 + c]; F2 = d.dfrc[3 * s2 + c];
     Q1 = d.dq[3 * s1 + c]; Q2 = d.dq[3 * s2 + c];
   }
+  double fw1 = 0., pw1 = 0., fw2 = 0., pw2 = 0.;
+  if ((mode & 1) && live && c == 2 && !per) {
+    lj_wall(kp, X1, kp.rwc, w3, fw1, pw1);
+    lj_wall(kp, X2, kp.rwn, w3, fw2, pw2);
+  }
+  double dX = X1 - X2;   // of this step's positions
+  if (wrapc) dX = dmin_image(dX, L);
+  // (only the dimer step before wrote the state used so far: it arrives, and the
+  // walls' forces are formed, while the force kernel ends)
+  after_previous();
+  if (d.ctr->abort_step) return;
+  if (!(mode & 1) && live && comp) { F1 = d.dfrc[3 * s1 + c]; F2 = d.dfrc[3 * s2 + c]; }
   unsigned long long iters = 0;
   if (mode & 1) {
-    double fw1 = 0., pw1 = 0., fw2 = 0., pw2 = 0.;
-    if (live && c == 2 && !per) {
-      lj_wall(kp, X1, kp.rwc, w3, fw1, pw1);
-      lj_wall(kp, X2, kp.rwn, w3, fw2, pw2);
-    }
     // the wall energies travel from the z lane to the energy lane
     const int zl = (threadIdx.x & 31 & ~3) | 2;
     const double p1 = __shfl_sync(gmask, pw1, zl), p2 = __shfl_sync(gmask, pw2, zl);
@@ -1829,8 +1846,7 @@ __global__ void k_dimer_split(Dev<T> d, KParams<T> kp, StepArgs a, int mode, dou
     if (comp) { V1 = Q1 + hIMc * F1; V2 = Q2 + hIMn * F2; }
     int acc = 0;
     for (;;) {
-      double dd = X1 - X2;
-      if (wrapc) dd = dmin_image(dd, L);
+      const double dd = dX;
       const double Con2diff = 2.0 * group4_sum(gmask, (V1 - V2) * dd);
       if (!live || fabs(Con2diff) < 1.e-8) break;
       if (acc == rattle_max) { if (c == 0) atomicOr(&d.ctr->status, DEV_ERR_RATTLE); break; }
@@ -1852,10 +1868,7 @@ __global__ void k_dimer_split(Dev<T> d, KParams<T> kp, StepArgs a, int mode, dou
     }
   }
   if (mode & 2) {
-    const double pr1 = X1, pr2 = X2;
-    double dP = X1 - X2;
-    if (wrapc) dP = dmin_image(dP, L);
-    if (!comp) dP = 0.;
+    const double pr1 = X1, pr2 = X2, dP = comp ? dX : 0.;
     Q1 = V1 + hIMc * F1; Q2 = V2 + hIMn * F2;
     X1 = X1 + dt * Q1; X2 = X2 + dt * Q2;
     if (!fast && wrapc) { X1 = wrap_box(X1, L); X2 = wrap_box(X2, L); }
@@ -1954,8 +1967,6 @@ void Launch<T>::sphere_totals(const Dev<T>& d, const KParams<T>& kp, double w3, 
 // by reciprocals.
 template <typename T>
 __global__ void k_rotor_split(Dev<T> d, KParams<T> kp, StepArgs a, int mode, int rattle_max) {
-  after_previous();
-  if (d.ctr->abort_step) return;
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   const int k = t >> 2, c = t & 3;
   const unsigned gmask = 0xFu << (threadIdx.x & 28);   // this group's four lanes
@@ -1975,10 +1986,13 @@ __global__ void k_rotor_split(Dev<T> d, KParams<T> kp, StepArgs a, int mode, int
   if (live && comp) {
     X1 = d.dpos[3 * s1 + c]; X2 = d.dpos[3 * s2 + c];
     V1 = d.dvel[3 * s1 + c]; V2 = d.dvel[3 * s2 + c];
-    F1 = d.dfrc[3 * s1 + c]; F2 = d.dfrc[3 * s2 + c];
     Q1 = d.dq[3 * s1 + c]; Q2 = d.dq[3 * s2 + c];
     A = d.anchor[3 * kk + c];
   }
+  // (only the dimer step before wrote the state read so far)
+  after_previous();
+  if (d.ctr->abort_step) return;
+  if (!(mode & 1) && live && comp) { F1 = d.dfrc[3 * s1 + c]; F2 = d.dfrc[3 * s2 + c]; }
   unsigned long long iters = 0;
   if (mode & 1) {
     double fw1 = 0., pw1 = 0., fw2 = 0., pw2 = 0.;
