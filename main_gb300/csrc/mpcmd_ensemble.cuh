@@ -549,7 +549,7 @@ struct ParticleIn {
 // ahead and keep to the registers of four blocks an SM.  256 replicas, 10 of them
 // rebuilding in an MD step: 57 us a step on GB300 (65 before; tiles of 1,024: 90).
 template <typename T>
-__global__ void __launch_bounds__(MAX_BLOCK, sizeof(T) == 4 ? 4 : 1)
+__global__ void __launch_bounds__(MAX_BLOCK, sizeof(T) == 4 ? 4 : 0)
     k_ens_rebuild(EDev<T> d, int mode, int shell_block, int advance_step) {
   __shared__ T red[32];
   __shared__ unsigned part[MAX_BLOCK];
@@ -911,7 +911,7 @@ __global__ void k_ens_dimer(EDev<T> d, int mode, int rattle_max) {
 // members on the unshifted cells, skipping the particles inside a sphere
 // cutoff; outside-list members order before inside-list members).
 template <typename T>
-__global__ void __launch_bounds__(MAX_BLOCK, sizeof(T) == 4 ? 4 : 1)
+__global__ void __launch_bounds__(MAX_BLOCK, sizeof(T) == 4 ? 4 : 0)
     k_ens_collide(EDev<T> d) {
   for (int t = blockIdx.x; t < d.n_ptiles; t += gridDim.x) {
     const uint32_t r = d.pt_rep[t];

@@ -2503,8 +2503,12 @@ __device__ __forceinline__ bool watch_test(const KParams<T>& kp, T gap, uint32_t
   return false;
 }
 
+// Bound by the latency of the cell's entry behind the particle's key and by the
+// 33 bytes it moves a particle.  FP32: kept to the registers of six blocks an SM
+// (168 million particles: 1.26 ms on GB300; five blocks 1.31, seven 1.39, eight
+// 1.41).
 template <typename T>
-__global__ void __launch_bounds__(TPB) k_rotate_main(Dev<T> d, KParams<T> kp, StepArgs a) {
+__global__ void __launch_bounds__(TPB, sizeof(T) == 4 ? 6 : 0) k_rotate_main(Dev<T> d, KParams<T> kp, StepArgs a) {
   after_previous();
   if (d.ctr->abort_step) return;
   // two particles per thread and iteration: all loads and both table gathers
