@@ -633,14 +633,15 @@ __global__ void __launch_bounds__(MAX_BLOCK, sizeof(T) == 4 ? 4 : 0)
 // [M_ADVANCE].  The kicks add the C pair force, then the N pair force
 // (kick_lists order); the FP32 build adds their sum.
 //
-// Bound by the entries' gathered states (67 bytes an entry read and written)
-// and, for few replicas, by the chain of dependent loads in front of them: a
+// Bound by the entries' gathered states (37 bytes an entry read, and 16 to 33
+// written: an entry beyond the cutoffs keeps its velocity, and few change cell or
+// species in a step; writing only what changed took 54 us to 44) and, for few replicas, by the chain of dependent loads in front of them: a
 // tile's descriptor gives its replica and entries in one load (a binary search
 // over the tile prefix was four to eight).  The pair forces pass through
 // memory only from a step that ends a call or a period (M_FORCE alone) to the
 // M_ADVANCE that opens the next; a fused step neither reads nor keeps them,
-// which was 48 bytes an entry: 54 us per MD step for 256 replicas against 83,
-// 5.5 us against 7.7 for 16.
+// which was 48 bytes an entry (83 us to 54 per MD step of 256 replicas).  With
+// all of it 44 us per MD step for 256 replicas, 4.8 us for 16.
 template <typename T, int MODE>
 __global__ void __launch_bounds__(MAX_BLOCK) k_ens_force(EDev<T> d) {
   constexpr bool FORCE = (MODE & M_FORCE) != 0, ADVANCE = (MODE & M_ADVANCE) != 0;
@@ -664,6 +665,9 @@ __global__ void __launch_bounds__(MAX_BLOCK) k_ens_force(EDev<T> d) {
       T ox = d.ox[i], oy = d.oy[i], oz = d.oz[i];
       T vx = d.vx[i], vy = d.vy[i], vz = d.vz[i];
       uint8_t f = d.flag[i];
+      const uint32_t cell0 = cell;
+      const uint8_t f0 = f;
+      const T vx0 = vx, vy0 = vy, vz0 = vz;
       T fp[6];
 #pragma unroll
       for (int q = 0; q < 6; ++q) fp[q] = FORCE ? (T)0 : d.sh_fp[6 * e + q];
@@ -699,11 +703,12 @@ __global__ void __launch_bounds__(MAX_BLOCK) k_ens_force(EDev<T> d) {
         stream_one(kp, (const uint8_t*)nullptr, cell, ox, oy, oz, vx, vy, vz, f, false, 0);
         msd = msd0 + (vx * vx + vy * vy + vz * vz) * (kp.dt * kp.dt);
         d.sh_msd[e] = msd;
-        d.cell[i] = cell;
+        if (cell != cell0) d.cell[i] = cell;   // (few leave their cell in a step)
         d.ox[i] = ox; d.oy[i] = oy; d.oz[i] = oz;
       }
-      d.vx[i] = vx; d.vy[i] = vy; d.vz[i] = vz;
-      if (FORCE) d.flag[i] = f;
+      // (most entries are beyond the cutoff and keep their velocity)
+      if (vx != vx0 || vy != vy0 || vz != vz0) { d.vx[i] = vx; d.vy[i] = vy; d.vz[i] = vz; }
+      if (FORCE && f != f0) d.flag[i] = f;
       if (FORCE && !ADVANCE) {
 #pragma unroll
         for (int q = 0; q < 6; ++q) d.sh_fp[6 * e + q] = fp[q];

@@ -1330,6 +1330,9 @@ __global__ void __launch_bounds__(TPB, sizeof(T) == 4 ? 5 : 1) k_force(Dev<T> d,
                                     (uint16_t)(packed.y & 0xFFFFu), (uint16_t)(packed.y >> 16),
                                     (uint16_t)(packed.z & 0xFFFFu), (uint16_t)(packed.z >> 16),
                                     (uint16_t)(packed.w & 0xFFFFu), (uint16_t)(packed.w >> 16)};
+    const uint32_t cell0 = cell;
+    const uint8_t fl0 = fl;
+    const T vx0 = vx, vy0 = vy, vz0 = vz;
     // owner tag (type_B) of the particle, with owner_tags
     uint32_t own = 0, own0 = 0;
     if (OWN && act) own = own0 = d.owner[idx];
@@ -1437,7 +1440,7 @@ __global__ void __launch_bounds__(TPB, sizeof(T) == 4 ? 5 : 1) k_force(Dev<T> d,
         T msd = msd0 + (vx * vx + vy * vy + vz * vz) * (kp.dt * kp.dt);
         d.sh.msd[j] = msd;
         msdmax = msd > msdmax ? msd : msdmax;
-        d.sh.cell[j] = cell;
+        if (cell != cell0) d.sh.cell[j] = cell;   // (few leave their cell in a step)
         d.sh.ox[j] = ox; d.sh.oy[j] = oy; d.sh.oz[j] = oz;
       } else if (!SUMK) {
 #pragma unroll
@@ -1447,8 +1450,8 @@ __global__ void __launch_bounds__(TPB, sizeof(T) == 4 ? 5 : 1) k_force(Dev<T> d,
           d.sh.pf[bq] = fpx[q]; d.sh.pf[bq + 1] = fpy[q]; d.sh.pf[bq + 2] = fpz[q];
         }
       }
-      d.sh.vx[j] = vx; d.sh.vy[j] = vy; d.sh.vz[j] = vz;
-      d.sh.flag[j] = fl;
+      if (vx != vx0 || vy != vy0 || vz != vz0) { d.sh.vx[j] = vx; d.sh.vy[j] = vy; d.sh.vz[j] = vz; }
+      if (fl != fl0) d.sh.flag[j] = fl;
       if (OWN && own != own0) d.owner[idx] = (uint16_t)own;
     }
   }
