@@ -288,9 +288,12 @@ struct Ensemble : EnsembleBase {
   }
   void L_tiles() { k_ens_tiles<T><<<1, 256, 0, st>>>(d, sblock); ++launches; }
   void L_dimer(int mode) {
-    // four lanes per replica; blocks of eight replicas spread over the SMs (of
-    // 64 for thousands of replicas, whose plan one block writes)
-    const int tpb = R <= 2048 ? 32 : 256;
+    // Four lanes per replica.  Up to 32 replicas in one block, which plans the
+    // rebuild without waiting for others (its four warps keep one FP64 pipe busy:
+    // a period of 16 replicas 1.09 ms against 1.15 in blocks of eight replicas, of
+    // 32 1.41 against 1.45, of 48 1.72 against 1.67); then blocks of eight spread
+    // over the SMs (of 64 for thousands of replicas, whose plan one block writes).
+    const int tpb = R <= 32 ? (4 * R + 31) / 32 * 32 : (R <= 2048 ? 32 : 256);
     k_ens_dimer<T><<<(4 * R + tpb - 1) / tpb, tpb, 0, st>>>(d, mode, rattle_max);
     ++launches;
   }

@@ -1,4 +1,5 @@
-"""Hundreds of replicas of a few hundred particles: a block's share of a
+"""Replica counts around the one block of 32 replicas that takes the dimer step
+of small ensembles, and hundreds of replicas of a few hundred particles: a block's share of a
 rebuild (units of 256 particles) and of the observables (neighbouring work
 tiles) then begins and ends inside replicas and covers several of them.
 
@@ -40,6 +41,28 @@ def test_fp64_follows_single_contexts():
     for chunk in (50, 20):
         ens.run(chunk)
         for r, (cfg, e) in engines.items():
+            e.run(chunk)
+            assert_close(ens.download(r), e.download_state(), cfg, pos=1e-9, vel=1e-9, flags=1.0, dimer=1e-9)
+    ens.close()
+
+
+@pytest.mark.parametrize("count", [1, 7, 8, 31, 32, 33])
+def test_fp64_dimer_blocks(count):
+    reps = replicas(count)
+    ens = E.Ensemble(reps, precision=64)
+    ens.initial()
+    engines = []
+    for r in sorted({0, count // 2, count - 1}):
+        cfg = E.config_of_replica(reps[r], precision=64)
+        e = Engine(cfg)
+        e.initial()
+        ens.upload(r, e.download_state())
+        e.prepare()
+        engines.append((r, cfg, e))
+    ens.prepare()
+    for chunk in (50, 20, 3):
+        ens.run(chunk)
+        for r, cfg, e in engines:
             e.run(chunk)
             assert_close(ens.download(r), e.download_state(), cfg, pos=1e-9, vel=1e-9, flags=1.0, dimer=1e-9)
     ens.close()
