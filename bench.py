@@ -555,11 +555,11 @@ def main_surrogate(args, ws, rk, lr):
             # cores need time for (the FP32 output alone is 537 MB at 65,536
             # points): its binding roofline is HBM; the tensor fraction is
             # given beside it
-            "roofline": {"bound": "hbm", "kernel": "k_gemm (forward of %d points, five launches)" % inf["points"],
+            "roofline": {"bound": "hbm", "kernel": "k_chain (forward of %d points, one launch)" % inf["points"],
                          "achieved": round(inf["gbs"], 1), "peak": hbm, "peak_source": peak_kind,
                          "unit": "GB/s", "frac": round(inf["gbs"] / hbm, 4), "traffic": None,
                          "algorithmic_bytes_per_launch": int(inf["bytes"]),
-                         "what": "inputs, BF16 activations written and read once, weights, FP32 outputs",
+                         "what": "inputs, BF16 weights, FP32 outputs",
                          "tensor": {"achieved": round(inf["tflops"], 2), "peak": peak, "unit": "TFLOP/s",
                                     "frac": round(inf["tflops"] / peak, 4)}},
             "surrogate": out}
