@@ -317,7 +317,7 @@ struct Engine : EngineBase {
     CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
     grid = nsm * 8;
     // the heavy persistent kernels run exactly one wave: SMs x resident blocks
-    int occ[6];
+    int occ[OCC_KERNELS];
     Launch<T>::occupancy(occ);
     CK(cudaGetLastError());
     g_rebuild = nsm * std::max(occ[0], 1);
@@ -326,6 +326,10 @@ struct Engine : EngineBase {
     g_far = nsm * std::max(occ[3], 1);
     g_cells = nsm * std::max(occ[4], 1);
     g_shell = nsm * std::max(occ[5], 1);
+    kp.g_obs = nsm * std::max(occ[6], 1);
+    kp.g_conc = nsm * std::max(occ[7], 1);
+    kp.g_gather = nsm * std::max(occ[8], 1);
+    kp.g_scatter = nsm * std::max(occ[9], 1);
     CK(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
     CK(cudaStreamCreateWithFlags(&cst, cudaStreamNonBlocking));
     for (cudaEvent_t& e : xev) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
@@ -1128,7 +1132,7 @@ struct Engine : EngineBase {
   int observables(mpcmd_obs* o) override {
     std::memset(o, 0, sizeof(*o));
     CK(cudaMemsetAsync(d.ctr->sums, 0, 8 * sizeof(double), st));
-    Launch<T>::observables(d, kp, cfg.mass, grid, st);
+    Launch<T>::observables(d, kp, cfg.mass, st);
     Counters h;
     int r = read_counters(h);
     if (r) return r;

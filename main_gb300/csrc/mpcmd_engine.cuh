@@ -177,6 +177,8 @@ struct StepArgs {
   float shf[3];        // the same rounded to float (FP32 kernels)
 };
 
+constexpr int OCC_KERNELS = 10;   // kernels whose grids are one wave
+
 template <typename T>
 struct Launch {
   // conversion of one uploaded FP64 component (0-2 positions, 3-5
@@ -224,7 +226,7 @@ struct Launch {
   // cell (any order inside a cell), main indices kept in lid / lpos; the
   // caller provides lid2 and lpos and swaps nothing
   static void resort(Dev<T>& d, const KParams<T>& kp, int tc, int tc_full, cudaStream_t st);
-  static void observables(const Dev<T>& d, const KParams<T>& kp, const double* mass, int grid, cudaStream_t st);
+  static void observables(const Dev<T>& d, const KParams<T>& kp, const double* mass, cudaStream_t st);
   // counts into c's arrays (zeroed by the caller)
   static void concentration(const Dev<T>& d, const KParams<T>& kp, int tc, int tc_defer, const ConcArgs& c,
                             cudaStream_t st);
@@ -232,7 +234,7 @@ struct Launch {
   static void conc_scale(const uint32_t* cnt, double* out, const ConcScale& s, int64_t lo, int64_t hi,
                          cudaStream_t st);
   // resident blocks per SM of the persistent kernels (rebuild, force, rotate)
-  static void occupancy(int* blocks);
+  static void occupancy(int* blocks /* [OCC_KERNELS] */);
   static void init_solvent(const Dev<T>& d, const KParams<T>& kp, const int64_t* bounds, double kT,
                            const double* mass, cudaStream_t st);
 };

@@ -337,9 +337,9 @@ void Launch<T>::download_convert(const Dev<T>& d, const KParams<T>& kp, double* 
 // particles), are taken in FP32 and repeated in FP64 only inside the error
 // band of the FP32 result, so the counts are those of the FP64 arithmetic.
 // The next four particles' loads are in flight meanwhile, and the few particles
-// that reach a slab are binned a full warp at a time: 99 us instead of 206 when
+// that reach a slab are binned a full warp at a time: 86 us instead of 206 when
 // a lane that found one held its warp up.  The fields, series and axes of that
-// box take 0.57 ms instead of 1.77.
+// box take 0.55 ms instead of 1.77.
 
 // Bin of a coordinate: ceil(u / w) clamped to [1, nb], 0-based.  t = uf * iwf
 // has relative error below 3 * 2^-24 of u / w (uf, iwf and the product
@@ -500,7 +500,7 @@ __global__ void k_conc_scale(const uint32_t* cnt, double* out, ConcScale s, int6
 template <typename T>
 void Launch<T>::concentration(const Dev<T>& d, const KParams<T>& kp, int tc, int tc_defer, const ConcArgs& c,
                               cudaStream_t st) {
-  k_concentration<T><<<1024, TPB, 0, st>>>(d.p, kp, d.react_box, tc, tc_defer, c);
+  k_concentration<T><<<kp.g_conc, TPB, 0, st>>>(d.p, kp, d.react_box, tc, tc_defer, c);
   // (the row blocks in y stay below 65,536: ny <= 2^20)
   k_conc_rows<T><<<dim3((c.nx + 127) / 128, (c.ny + CONC_ROWS - 1) / CONC_ROWS), 128, 0, st>>>(c);
   LAUNCH_COUNT(); LAUNCH_COUNT();
@@ -1707,7 +1707,7 @@ void Launch<T>::sort_shell(const Dev<T>& d, const KParams<T>& kp, cudaStream_t s
   launch_next(k_shell_clear_counts<T>, (kp.ns * SHELL_CLASSES + TPB - 1) / TPB, TPB, st, d, kp);
   launch_next(k_shell_hist<T>, 1024, TPB, st, d, kp);
   launch_next(k_shell_scan<T>, 1, TPB, st, d, kp);
-  launch_next(k_shell_scatter<T>, 1024, TPB, st, d, kp);
+  launch_next(k_shell_scatter<T>, kp.g_scatter, TPB, st, d, kp);
   LAUNCH_COUNT(); LAUNCH_COUNT(); LAUNCH_COUNT(); LAUNCH_COUNT();
 }
 
@@ -2607,17 +2607,6 @@ void Launch<T>::rotate_main(const Dev<T>& d, const KParams<T>& kp, const StepArg
   LAUNCH_COUNT();
 }
 
-template <typename T>
-void Launch<T>::occupancy(int* blocks) {
-  blocks[0] = blocks[1] = blocks[2] = blocks[3] = blocks[4] = blocks[5] = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks[0], k_rebuild<T>, TPB, 0);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks[1], k_force<T, false>, TPB, 0);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks[2], k_rotate_main<T>, TPB, 0);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks[3], k_rebuild_far<T>, TPB, 0);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks[4], k_cells<T>, TPB, 0);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks[5], k_shell_advance<T>, TPB, 0);
-}
-
 // ---------------------------------------------------- shell home moves ----
 template <typename T>
 __global__ void k_flush(Dev<T> d, KParams<T> kp) {
@@ -2985,7 +2974,7 @@ void Launch<T>::sort(Dev<T>& d, const KParams<T>& kp, cudaStream_t st) {
   scan_u32(d.scnt, d.sstart, kp.ncell, d.scan_tmp, st);
   launch_next(k_sort_fill<T>, 1024, TPB, st, d, kp);
   launch_next(k_sort_segments<T>, 1024, TPB, st, d, kp);
-  launch_next(k_sort_gather<T>, 1024, TPB, st, d, kp);
+  launch_next(k_sort_gather<T>, kp.g_gather, TPB, st, d, kp);
   LAUNCH_COUNT(); LAUNCH_COUNT(); LAUNCH_COUNT(); LAUNCH_COUNT();
   Particles<T> t = d.p; d.p = d.p2; d.p2 = t;
   uint16_t* o = d.owner; d.owner = d.owner2; d.owner2 = o;
@@ -3001,9 +2990,10 @@ void Launch<T>::sort(Dev<T>& d, const KParams<T>& kp, cudaStream_t st) {
 // FP32 build: PairSum sums per thread (exact products of the masses and the
 // FP32 velocities), widened to FP64 for the reduction; FP64 arithmetic per
 // particle would run at the part's FP64 rate.  Bound by the 13 bytes a
-// particle it reads: four particles per thread and iteration in 16-byte
-// (flags: 4-byte) loads keep enough of them in flight.  2.1e7 particles: 84 us
-// against 160 with one particle per iteration; 1.7e8: 549 against 712 us.
+// particle it reads and 50 instructions of float pairs: four particles per thread
+// and iteration in 16-byte (flags: 4-byte) loads, the species counted a byte each,
+// one wave of blocks.  2.1e7 particles: 72 us against 160 with one particle per
+// iteration; 1.7e8: 514 against 712 us.
 template <typename T>
 __global__ void __launch_bounds__(TPB) k_observables(Dev<T> d, KParams<T> kp, double m0, double m1, double m2,
                                                      double m3) {
@@ -3020,7 +3010,7 @@ __global__ void __launch_bounds__(TPB) k_observables(Dev<T> d, KParams<T> kp, do
     // species of one mass (every input deck's) are weighted once, after the sum
     const bool one_mass = m0 == m1 && m0 == m2 && m0 == m3;
     PairSum sum[4] = {{0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}};   // momentum, twice the kinetic energy
-    uint32_t cnt[4] = {0u, 0u, 0u, 0u};
+    uint32_t cnt[4] = {0u, 0u, 0u, 0u}, four = 0u;   // four: up to four particles' species, a byte each
     auto add = [&](int64_t i, uint8_t f, float vx, float vy, float vz) {
       int sp = f & FLAG_SPECIES;
       if (f & FLAG_HOME_SHELL) {
@@ -3042,7 +3032,12 @@ __global__ void __launch_bounds__(TPB) k_observables(Dev<T> d, KParams<T> kp, do
           pair_add_prod(sum[3], wh, wl, p, __fmaf_rn(v[k], v[k], -p));
         }
       }
-      cnt[0] += sp == 0; cnt[1] += sp == 1; cnt[2] += sp == 2; cnt[3] += sp == 3;
+      four += 1u << (8 * sp);
+    };
+    auto count = [&]() {
+#pragma unroll
+      for (int k = 0; k < 4; ++k) cnt[k] += (four >> (8 * k)) & 255u;
+      four = 0u;
     };
     const int64_t n4 = kp.n >> 2;
     const int64_t t0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -3054,10 +3049,12 @@ __global__ void __launch_bounds__(TPB) k_observables(Dev<T> d, KParams<T> kp, do
       add(i + 1, f.y, vx.y, vy.y, vz.y);
       add(i + 2, f.z, vx.z, vy.z, vz.z);
       add(i + 3, f.w, vx.w, vy.w, vz.w);
+      count();
     }
     if (t0 < (kp.n & 3)) {
       const int64_t i = (n4 << 2) + t0;
       add(i, d.p.flag[i], d.p.vx[i], d.p.vy[i], d.p.vz[i]);
+      count();
     }
     // one FP64 atomic per value and block
     __shared__ double s_part[TPB / 32][8];
@@ -3110,9 +3107,24 @@ __global__ void __launch_bounds__(TPB) k_observables(Dev<T> d, KParams<T> kp, do
 }
 
 template <typename T>
-void Launch<T>::observables(const Dev<T>& d, const KParams<T>& kp, const double* mass, int grid, cudaStream_t st) {
-  launch_next(k_observables<T>, grid, TPB, st, d, kp, mass[0], mass[1], mass[2], mass[3]);
+void Launch<T>::observables(const Dev<T>& d, const KParams<T>& kp, const double* mass, cudaStream_t st) {
+  launch_next(k_observables<T>, kp.g_obs, TPB, st, d, kp, mass[0], mass[1], mass[2], mass[3]);
   LAUNCH_COUNT();
+}
+
+template <typename T>
+void Launch<T>::occupancy(int* blocks) {
+  for (int i = 0; i < OCC_KERNELS; ++i) blocks[i] = 0;
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks[0], k_rebuild<T>, TPB, 0);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks[1], k_force<T, false>, TPB, 0);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks[2], k_rotate_main<T>, TPB, 0);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks[3], k_rebuild_far<T>, TPB, 0);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks[4], k_cells<T>, TPB, 0);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks[5], k_shell_advance<T>, TPB, 0);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks[6], k_observables<T>, TPB, 0);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks[7], k_concentration<T>, TPB, 0);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks[8], k_sort_gather<T>, TPB, 0);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks[9], k_shell_scatter<T>, TPB, 0);
 }
 
 // ------------------------------------------------------------------ init ----
