@@ -145,9 +145,10 @@ struct KParams {
   double hIMc, hIMn, IIM;          // (dt/2)/Mc, (dt/2)/Mn, 1/(1/Mc + 1/Mn)
   double iMc, iMn, iD2, iMcdt, iMndt;   // 1/Mc, 1/Mn, 1/Dcn^2, 1/(Mc dt), 1/(Mn dt)
   T cut2_strict[2];      // (R * 2^(1/6))^2 for the initial placement test
-  // launches of one wave (engine; SMs x resident blocks; more blocks than fit run
-  // a second, partly filled one)
-  int g_obs, g_conc, g_gather, g_scatter;
+  // blocks of one wave (engine; SMs x resident blocks): with a number between one
+  // wave and two, the second runs partly filled.  Two waves where a second block
+  // hides the first one's latency (k_resort_count, k_accumulate_main).
+  int g_obs, g_conc, g_gather, g_scatter, g_rcount, g_rbin, g_accum;
 };
 
 // Sphere position as cell + offset in T (written whenever a sphere moves).

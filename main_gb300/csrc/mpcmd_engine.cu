@@ -330,6 +330,9 @@ struct Engine : EngineBase {
     kp.g_conc = nsm * std::max(occ[7], 1);
     kp.g_gather = nsm * std::max(occ[8], 1);
     kp.g_scatter = nsm * std::max(occ[9], 1);
+    kp.g_rcount = nsm * std::max(occ[10], 1);
+    kp.g_rbin = nsm * std::max(occ[11], 1);
+    kp.g_accum = nsm * std::max(occ[12], 1);
     CK(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
     CK(cudaStreamCreateWithFlags(&cst, cudaStreamNonBlocking));
     for (cudaEvent_t& e : xev) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));

@@ -177,7 +177,7 @@ struct StepArgs {
   float shf[3];        // the same rounded to float (FP32 kernels)
 };
 
-constexpr int OCC_KERNELS = 10;   // kernels whose grids are one wave
+constexpr int OCC_KERNELS = 13;   // kernels whose grids are one wave
 
 template <typename T>
 struct Launch {

@@ -2220,7 +2220,7 @@ __global__ void __launch_bounds__(TPB) k_accumulate_main(Dev<T> d, KParams<T> kp
 
 template <typename T>
 void Launch<T>::accumulate_main(const Dev<T>& d, const KParams<T>& kp, const StepArgs& a, int what, cudaStream_t st) {
-  launch_next(k_accumulate_main<T>, a.grid, TPB, st, d, kp, a, what);
+  launch_next(k_accumulate_main<T>, 2 * kp.g_accum, TPB, st, d, kp, a, what);
   LAUNCH_COUNT();
 }
 
@@ -2955,9 +2955,9 @@ void Launch<T>::resort(Dev<T>& d, const KParams<T>& kp, int tc, int tc_full, cud
   const int nbins = (int)((kp.ncell + (1 << bits) - 1) >> bits);
   cudaMemsetAsync(d.scnt, 0, sizeof(uint32_t) * nbins, st);
   cudaMemsetAsync(d.sfill, 0, sizeof(uint32_t) * nbins, st);
-  launch_next(k_resort_count<T>, 1024, TPB, st, d, kp, bits, tc, tc_full);
+  launch_next(k_resort_count<T>, 2 * kp.g_rcount, TPB, st, d, kp, bits, tc, tc_full);
   scan_u32(d.scnt, d.sstart, nbins, d.scan_tmp, st);
-  launch_next(k_resort_bin<T>, 1024, TPB, st, d, kp, bits);
+  launch_next(k_resort_bin<T>, kp.g_rbin, TPB, st, d, kp, bits);
   launch_next(k_resort_fine<T>, nbins < 65535 ? nbins : 65535, TPB, st, d, kp, bits, nbins);
   LAUNCH_COUNT(); LAUNCH_COUNT(); LAUNCH_COUNT();
   Particles<T> t = d.p; d.p = d.p2; d.p2 = t;
@@ -3125,6 +3125,9 @@ void Launch<T>::occupancy(int* blocks) {
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks[7], k_concentration<T>, TPB, 0);
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks[8], k_sort_gather<T>, TPB, 0);
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks[9], k_shell_scatter<T>, TPB, 0);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks[10], k_resort_count<T>, TPB, 0);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks[11], k_resort_bin<T>, TPB, 0);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks[12], k_accumulate_main<T>, TPB, 0);
 }
 
 // ------------------------------------------------------------------ init ----
