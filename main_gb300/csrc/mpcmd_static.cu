@@ -162,6 +162,12 @@ __global__ void __launch_bounds__(kThreads) k_static_accumulate(KParams<double> 
 struct Map {
   double M[3][3], b[3];
 };
+// sum / n for a count n with rn = 1 / n rounded to nearest, rounded as the
+// division (div_const); an infinite or undefined sum stays what it is.
+__device__ __forceinline__ double mean_of(double sum, double n, double rn) {
+  const double q = div_const(sum, n, rn);
+  return (__double2hiint(q) & 0x7FF00000) != 0x7FF00000 ? q : sum * rn;
+}
 __device__ __forceinline__ bool cell_map(const KParams<double>& kp, uint32_t cell, uint32_t step, double2 a0, double2 a1,
                                          Map& w) {
   const double pi = 3.141592653589793;
@@ -169,7 +175,8 @@ __device__ __forceinline__ bool cell_map(const KParams<double>& kp, uint32_t cel
   const unsigned int cnt = (unsigned int)__double2loint(a0.x);
   if (cnt == 0u) return false;
   const double n = (double)cnt;
-  const double m[3] = {a0.y / n, a1.x / n, a1.y / n};
+  const double rn = 1.0 / n;
+  const double m[3] = {mean_of(a0.y, n, rn), mean_of(a1.x, n, rn), mean_of(a1.y, n, rn)};
   double u1, u2, sp, cp;
   contract_pair(kp.seed, TAG_AXIS, cell, 0, step, u1, u2);
   sincos(2.0 * pi * u1, &sp, &cp);
