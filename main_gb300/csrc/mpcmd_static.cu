@@ -35,10 +35,10 @@
 // root) is drawn once per cell instead of once per particle, the shifted cell
 // comes from 32.32 fixed-point integers, and the rotation about the centre of
 // mass is one affine map, nine fused multiply-adds a particle.  5.1 million
-// unsorted particles in 80^3 cells: 367 us against 1615 with the axis drawn
+// unsorted particles in 80^3 cells: 348 us against 1615 with the axis drawn
 // and the rotation evaluated per particle (450 with 22 FP64 instructions a
 // particle from the centre of mass and the axis); the atomics take 124 us,
-// the cells 102, the rotation 126.
+// the cells 83 (102 with three divisions and unfused products), the rotation 123.
 #include <algorithm>
 #include <cmath>
 #include <mutex>
@@ -180,16 +180,15 @@ __device__ __forceinline__ bool cell_map(const KParams<double>& kp, uint32_t cel
   double u1, u2, sp, cp;
   contract_pair(kp.seed, TAG_AXIS, cell, 0, step, u1, u2);
   sincos(2.0 * pi * u1, &sp, &cp);
-  const double theta = 2.0 * u2 - 1.0, r = sqrt(1.0 - theta * theta);
+  const double theta = fma(2.0, u2, -1.0), r = sqrt(1.0 - theta * theta);
   const double u[3] = {r * cp, r * sp, theta};
   const double su[3] = {sn * u[0], sn * u[1], sn * u[2]};
-  const double xy = c1 * u[0] * u[1], xz = c1 * u[0] * u[2], yz = c1 * u[1] * u[2];
-  w.M[0][0] = fma(c1 * u[0], u[0], c); w.M[0][1] = xy - su[2]; w.M[0][2] = xz + su[1];
-  w.M[1][0] = xy + su[2]; w.M[1][1] = fma(c1 * u[1], u[1], c); w.M[1][2] = yz - su[0];
-  w.M[2][0] = xz - su[1]; w.M[2][1] = yz + su[0]; w.M[2][2] = fma(c1 * u[2], u[2], c);
+  const double k0 = c1 * u[0], k1 = c1 * u[1], k2 = c1 * u[2];
+  w.M[0][0] = fma(k0, u[0], c); w.M[0][1] = fma(k0, u[1], -su[2]); w.M[0][2] = fma(k0, u[2], su[1]);
+  w.M[1][0] = fma(k0, u[1], su[2]); w.M[1][1] = fma(k1, u[1], c); w.M[1][2] = fma(k1, u[2], -su[0]);
+  w.M[2][0] = fma(k0, u[2], -su[1]); w.M[2][1] = fma(k1, u[2], su[0]); w.M[2][2] = fma(k2, u[2], c);
 #pragma unroll
-  for (int q = 0; q < 3; ++q)
-    w.b[q] = m[q] - fma(w.M[q][2], m[2], fma(w.M[q][1], m[1], w.M[q][0] * m[0]));
+  for (int q = 0; q < 3; ++q) w.b[q] = fma(-w.M[q][2], m[2], fma(-w.M[q][1], m[1], fma(-w.M[q][0], m[0], m[q])));
   return true;
 }
 
@@ -295,7 +294,7 @@ extern "C" int mpcmd_collide_static(const double* x, const double* y, const doub
   const int tgrid = (int)std::min<int64_t>((ncs + kThreads - 1) / kThreads, (int64_t)nsm * 8);
   k_static_clear<<<tgrid, kThreads, 0, st>>>(acc, ncs);
   // Up to three blocks an SM each kernel starts while the one before it ends (1,536
-  // to 8,192 particles 14.8 us instead of 20.5, 80,000 23.6 instead of 26.7).
+  // to 8,192 particles 14.4 us instead of 20.5, 80,000 22 instead of 26.7).
   // Past that the early blocks crowd the first SMs that fall free, where they
   // share the FP64 pipe (270,000 particles: 43.7 us instead of 33.7).
   const bool early = grid <= 3 * nsm;
