@@ -1149,6 +1149,8 @@ inline int tile_steps(int64_t n, int grid, int most) {
 
 template <typename T>
 void Launch<T>::rebuild_split(const Dev<T>& d, const KParams<T>& kp, const StepArgs& a, cudaStream_t st) {
+  // (the memset also keeps the far pass from starting early, before the SMs are
+  // free for one wave of it: 1 % of a period at 256^3)
   cudaMemsetAsync(&d.ctr->n_near, 0, sizeof(unsigned int), st);
   StepArgs b = a;
   b.far_steps = tile_steps(kp.n, a.g_far, FAR_STEPS_MAX);
