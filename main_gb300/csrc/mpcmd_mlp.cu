@@ -148,30 +148,6 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16
 }
 __device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
-// The same box for both CTAs of a pair: the data and the byte count arrive at
-// the same shared-memory offsets in each.
-__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap* map, uint32_t bar, int x, int y) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes.multicast::cluster [%0], [%1, {%3, "
-      "%4}], [%2], %5;" ::"r"(dst),
-      "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(x), "r"(y), "h"((uint16_t)3)
-      : "memory");
-}
-// tcgen05.commit to the barriers at this offset in both CTAs of a pair.
-__device__ __forceinline__ void mma_commit_pair(uint32_t bar) {
-  asm volatile(
-      "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar),
-      "h"((uint16_t)3)
-      : "memory");
-}
-__device__ __forceinline__ uint32_t cluster_rank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ void cluster_sync() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
 __device__ __forceinline__ void mma_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
@@ -281,19 +257,17 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
 //   * shared memory is left to the weights and the stores: one producer thread
 //     walks the weight boxes of all layers in order (64 columns of K by the
 //     layer's width, or two boxes by 128 output columns) through a ring of
-//     32 KB stages, running ahead across layers and row tiles;
-//   * two CTAs form a pair that walks the same boxes for two row tiles: each
-//     loads half of every box and multicasts it to both, which halves the reads
-//     from L2;
+//     32 KB stages, running ahead across layers and row tiles (one load of each
+//     box for two CTAs, by multicast, gained nothing: a call of 65,536 points took
+//     192.8 us with it and 192.5 without, of 64 points 40.2 and 38.7);
 //   * tensor memory holds A (128 columns) and three 128-column accumulators;
 //     a hidden layer uses the first two.  Three groups of four epilogue warps
 //     (one warp per lane quarter) take the output tiles in turn, so that the
 //     stores of three tiles and the MMAs of the next overlap, and the next row
 //     tile enters while the last ones are stored;
-//   * pairs of row tiles that do not fill a wave are split over several pairs
-//     of CTAs by output columns, each repeating the (much cheaper) hidden
-//     layers: with fewer row tiles than SMs all of them, else the last partial
-//     wave.
+//   * row tiles that do not fill a wave are split over several CTAs by output
+//     columns, each repeating the (much cheaper) hidden layers: with fewer row
+//     tiles than SMs all of them, else the last partial wave.
 // Inference: one launch instead of six (one conversion and five GEMMs with the
 // activations through L2): with the call's own cost, 64 points take 43 us against 80, 65,536
 // points 196 against 283.  A hidden layer takes 3 us (1 us of MMAs, then its
@@ -312,7 +286,7 @@ constexpr uint32_t TM_ACC = 128;                   // first accumulator column (
 
 enum ChainMode : int { INFER = 0, FORWARD = 1, BACKWARD = 2 };
 
-struct InferMaps {             // (boxes of half the rows: one CTA's share)
+struct InferMaps {
   CUtensorMap w[MAX_HIDDEN];   // hidden layer l: 64 x H
   CUtensorMap out, tail;       // output layer: 64 x 128 and 64 x tail_n
 };
@@ -320,7 +294,7 @@ struct InferArgs {
   int layers, H, n_in, rows;   // layers of the chain (BACKWARD: all hidden ones but the last)
   int tiles;            // output jobs per row tile (BACKWARD: none)
   int tail_n;           // width of the last output job (a multiple of 16)
-  int whole, part, split;   // rounds of whole row-tile pairs; pairs left over, each split this many ways
+  int whole, part, split;   // rounds of whole row tiles; row tiles left over, each split this many ways
   int n_out;
   const float* x;       // [rows, n_in]
   const float* bias[MAX_HIDDEN];
@@ -346,14 +320,13 @@ constexpr size_t INF_SMEM = 1024 + (size_t)INF_STAGES * INF_STAGE + (size_t)INF_
                             (2 * INF_STAGES + 2 * INF_GROUPS + 3) * 8 + 16;
 static_assert(INF_SMEM <= 232448, "shared memory of one CTA");
 
-// Work item v of this CTA: its row tile (the CTAs of a pair take neighbouring
-// ones) and its output jobs [t0, t1).
+// Work item v of this CTA: its row tile and its output jobs [t0, t1).
 __device__ __forceinline__ bool infer_item(const InferArgs& a, int v, int& mt, int& t0, int& t1) {
-  const int g = (int)gridDim.x >> 1, b = (int)blockIdx.x >> 1, r = (int)blockIdx.x & 1;
-  if (v < a.whole) { mt = 2 * (v * g + b) + r; t0 = 0; t1 = a.tiles; return true; }
+  const int g = (int)gridDim.x, b = (int)blockIdx.x;
+  if (v < a.whole) { mt = v * g + b; t0 = 0; t1 = a.tiles; return true; }
   if (v > a.whole || a.part == 0 || b >= a.part * a.split) return false;
-  const int q = b % a.split;
-  mt = 2 * (a.whole * g + b / a.split) + r;
+  const int q = b / a.part;
+  mt = a.whole * g + b % a.part;
   t0 = a.tiles * q / a.split;
   t1 = a.tiles * (q + 1) / a.split;
   return true;
@@ -363,7 +336,7 @@ __device__ __forceinline__ bool infer_item(const InferArgs& a, int v, int& mt, i
 // a layer, counted through the layers): the CTAs that share a row tile all
 // compute its layers, and take turns in writing them.
 __device__ __forceinline__ bool keeps(const InferArgs& a, int v, int i) {
-  return v < a.whole || i % a.split == ((int)blockIdx.x >> 1) % a.split;
+  return v < a.whole || i % a.split == (int)blockIdx.x / a.part;
 }
 
 // 4 or 16 bytes to shared memory (this thread sees them after cp.async.wait_all).
@@ -429,7 +402,7 @@ __device__ __forceinline__ void store_block(const uint32_t* buf, int lane, char*
 // VB (INFER): the largest of 16, 8 and 4 bytes that divides the address of
 // every row of y
 template <int MODE, int VB>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(INF_THREADS, 1)
+__global__ void __launch_bounds__(INF_THREADS, 1)
     k_chain(const __grid_constant__ InferMaps maps, const __grid_constant__ InferArgs a) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* sRing = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -449,8 +422,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(INF_THREADS, 1)
   if (threadIdx.x == 0) {
     bail = 0;
     issued = 0;
-    // (a stage is free when both CTAs' MMAs have read it: either may write it)
-    for (int s = 0; s < INF_STAGES; ++s) { mbar_init(full0 + 8 * s, 1); mbar_init(empty0 + 8 * s, 2); }
+    for (int s = 0; s < INF_STAGES; ++s) { mbar_init(full0 + 8 * s, 1); mbar_init(empty0 + 8 * s, 1); }
     for (int b = 0; b < INF_GROUPS; ++b) { mbar_init(accf0 + 8 * b, 1); mbar_init(acce0 + 8 * b, MODE == FORWARD ? INF_EPI : 4); }
     mbar_init(hacc, 1);
     mbar_init(hready, INF_EPI);
@@ -466,7 +438,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(INF_THREADS, 1)
   }
   tmem_fence_before();
   __syncthreads();
-  cluster_sync();   // both CTAs' barriers exist before either signals them
   tmem_fence_after();
   const uint32_t tmem = *tmem_slot;
   if constexpr (MODE != INFER) mpcmd::let_next_start();
@@ -474,8 +445,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(INF_THREADS, 1)
 
   if (warp == 0) {
     if (lane == 0) {
-      // weight producer: this CTA's half of every box, to both CTAs
-      const int rank = (int)cluster_rank();
+      // weight producer
       int g = 0, mt, t0, t1;
       // one stage: boxes k..k+nb-1 of a layer, `n` rows of weights from `row` each
       auto fill = [&](const CUtensorMap* m, int k, int nb, int row, int n) -> bool {
@@ -484,11 +454,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(INF_THREADS, 1)
           bail = 1;
           return false;
         }
-        mbar_expect_tx(full0 + 8 * s, (uint32_t)(nb * n * BK * 2));   // (both halves)
-        const int half = rank * (n / 2);
+        mbar_expect_tx(full0 + 8 * s, (uint32_t)(nb * n * BK * 2));
         for (int q = 0; q < nb; ++q)
-          tma_load_2d_pair(smem_u32(sRing + s * INF_STAGE + q * (INF_STAGE / 2) + half * BK * 2), m, full0 + 8 * s,
-                           (k + q) * BK, row + half);
+          tma_load_2d(smem_u32(sRing + s * INF_STAGE + q * (INF_STAGE / 2)), m, full0 + 8 * s, (k + q) * BK, row);
         ++g;
         return true;
       };
@@ -525,7 +493,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(INF_THREADS, 1)
           for (int kk = 0; kk < BK / 16; ++kk)
             mma_bf16_ta(acc, a0 + 8 * kk, sw128_desc(b0 + 32 * kk), idesc, (k + q > 0 || kk > 0) ? 1u : 0u);
         }
-        mma_commit_pair(empty0 + 8 * s);
+        mma_commit(empty0 + 8 * s);
         ++g;
         return true;
       };
@@ -845,7 +813,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(INF_THREADS, 1)
   }
   tmem_fence_before();
   __syncthreads();
-  cluster_sync();   // no CTA leaves while the other may still signal or fill it
   tmem_fence_after();
   if (warp == 1)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
@@ -1331,17 +1298,17 @@ int infer_tail(const mpcmd_mlp* m) { return (m->nout - (infer_tiles(m) - 1) * IN
 
 bool make_infer_maps(mpcmd_mlp* m) {
   for (int l = 0; l < m->L; ++l)
-    if (!make_map(&m->maps.w[l], m->layers[l].wb, m->layers[l].n, m->layers[l].k, m->H / 2)) return false;
+    if (!make_map(&m->maps.w[l], m->layers[l].wb, m->layers[l].n, m->layers[l].k, m->H)) return false;
   const Layer& lo = m->layers[m->L];
-  return make_map(&m->maps.out, lo.wb, lo.n, lo.k, INF_BN / 2) &&
-         make_map(&m->maps.tail, lo.wb, lo.n, lo.k, infer_tail(m) / 2);
+  return make_map(&m->maps.out, lo.wb, lo.n, lo.k, INF_BN) &&
+         make_map(&m->maps.tail, lo.wb, lo.n, lo.k, infer_tail(m));
 }
 
 // Operands and work units of the training step's other launches.
 bool make_train_maps(mpcmd_mlp* m) {
   for (int j = 0; j + 1 < m->L; ++j) {
     const Layer& ly = m->layers[m->L - 1 - j];
-    if (!make_map(&m->back.w[j], ly.wt, ly.k, ly.n, m->H / 2)) return false;
+    if (!make_map(&m->back.w[j], ly.wt, ly.k, ly.n, m->H)) return false;
   }
   const Layer& lo = m->layers[m->L];
   if (!make_map(&m->dx_a, m->dy, m->B, m->npad, BM) || !make_map(&m->dx_b, lo.wt, lo.k, lo.n, 32)) return false;
@@ -1369,14 +1336,14 @@ bool make_train_maps(mpcmd_mlp* m) {
 }
 
 // Row tiles of a chain over the CTAs: whole rounds of one row tile per SM, then
-// the left-over row-tile pairs shared as far as the SMs go.
+// the left-over row tiles shared as far as the SMs go.
 int chain_grid(const mpcmd_mlp* m, int64_t rows, InferArgs& a) {
-  const int pairs = (int)((rows + 2 * BM - 1) / (2 * BM)), cap = std::max(m->sms / 2, 1);
-  a.whole = pairs / cap;
-  a.part = pairs % cap;
+  const int tiles = (int)((rows + BM - 1) / BM);
+  a.whole = tiles / m->sms;
+  a.part = tiles % m->sms;
   const int shares = a.tiles ? a.tiles : a.layers * a.H / 32;   // (BACKWARD: the pieces kept)
-  a.split = a.part ? std::min(shares, cap / a.part) : 1;
-  return 2 * (a.whole ? cap : a.part * a.split);
+  a.split = a.part ? std::min(shares, m->sms / a.part) : 1;
+  return a.whole ? m->sms : a.part * a.split;
 }
 
 // y [rows, nout] = network(x [rows, n_in]) (device, FP32).
@@ -1545,7 +1512,7 @@ int mpcmd_mlp_create(const mpcmd_mlp_config* cfg, mpcmd_mlp** out) {
     delete m;
     return MPCMD_ERR_CUDA;
   }
-  if (m->alloc(m->loss_part, (int64_t)std::max(m->sms, 2) * INF_EPI) != MPCMD_OK) {
+  if (m->alloc(m->loss_part, (int64_t)m->sms * INF_EPI) != MPCMD_OK) {
     delete m;
     return MPCMD_ERR_ALLOC;
   }
