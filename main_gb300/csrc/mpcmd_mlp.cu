@@ -512,6 +512,10 @@ __global__ void __launch_bounds__(INF_THREADS, 1)
           if (ok) mma_commit(hacc);
         }
         if (ok) ok = wait(hready, (uint32_t)hp++ & 1u);
+        // (BACKWARD has no output job: the next input may enter.  The epilogue waits
+        // for this and not for hready itself, whose next phase its own input
+        // completes: this thread must have seen the one before by then.)
+        if (MODE == BACKWARD && ok) mbar_arrive(accf0);
         for (int t = t0; t < t1 && ok; ++t, ++o) {
           const int b = o % 3;
           if (o >= 3 && !(ok = wait(acce0 + 8 * b, ((uint32_t)(o / 3) & 1u) ^ 1u))) break;
@@ -531,13 +535,11 @@ __global__ void __launch_bounds__(INF_THREADS, 1)
     uint32_t* buf = stage_all + ew * 32 * INF_PITCH;
     const uint32_t lanes = tmem + ((uint32_t)(quarter * 32) << 16);
     // A's columns and the reads of the accumulator before it are done
-    int published = 0;
     auto publish = [&]() {
       tmem_wait_st();
       tmem_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(hready);
-      ++published;
     };
     // what enters the chain: the input rows as 64 columns of K (zero-padded),
     // 32 by each of two groups, or the rows of a gradient
@@ -786,9 +788,9 @@ __global__ void __launch_bounds__(INF_THREADS, 1)
         // another group has the last output job
         if (first >= t1) fetch_hidden(0);
         if constexpr (MODE == BACKWARD) {
-          // no output job: the next input may enter when every warp has read the
-          // last accumulator
-          if ((ok = wait(hready, (uint32_t)(published - 1) & 1u))) load_input(nmt, true);
+          // no output job: the next input may enter when the issuer has seen that
+          // every warp has read the last accumulator
+          if ((ok = wait(accf0, (uint32_t)v & 1u))) load_input(nmt, true);
         } else if ((ok = wait(accf0 + 8 * (last % 3), (uint32_t)(last / 3) & 1u))) {
           load_input(nmt, keeps(a, v + 1, a.layers * a.H / 32));
         }
