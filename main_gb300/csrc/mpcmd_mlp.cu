@@ -440,8 +440,8 @@ __global__ void __launch_bounds__(INF_THREADS, 1)
   __syncthreads();
   tmem_fence_after();
   const uint32_t tmem = *tmem_slot;
-  if constexpr (MODE != INFER) mpcmd::let_next_start();
-  if constexpr (MODE == BACKWARD) mpcmd::wait_for_previous();
+  if constexpr (MODE == FORWARD) mpcmd::let_next_start();   // (an ordinary launch: nothing before it still runs)
+  if constexpr (MODE == BACKWARD) mpcmd::after_previous();
 
   if (warp == 0) {
     if (lane == 0) {
@@ -956,8 +956,7 @@ __global__ void __launch_bounds__(DxPipe::THREADS, 1)
   __shared__ int issued;
   DxPipe p;
   p.open(smem_raw, &bail, &issued, a.err);
-  mpcmd::let_next_start();
-  mpcmd::wait_for_previous();
+  mpcmd::after_previous();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int tiles_n = a.H / 32, units = (a.rows / BM) * tiles_n;
   if (warp == 0) {
@@ -1012,7 +1011,9 @@ __global__ void __launch_bounds__(DxPipe::THREADS, 1)
 // refreshes the BF16 copies [n, k] and [k, n].  Work units: the 128 x 64 tiles of
 // every layer, then blocks of 64 biases; 5 of its 8 us are Adam's divisions and
 // root, so 16 warps share a tile (8: 7 us); the parameters and moments (24 bytes a
-// weight, in L2) are fetched before the previous kernel has ended.
+// weight, in L2) are fetched before the previous kernel has ended: only this kernel
+// writes them, in the step before, and every kernel of a step lets the next one
+// start after its own wait.
 struct AdamArgs {
   float lr, b1, b2, eps, c1, c2;
 };

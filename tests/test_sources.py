@@ -2,6 +2,7 @@
 that every rank of a multi-GPU run loads."""
 import glob
 import os
+import re
 
 import pytest
 
@@ -14,3 +15,25 @@ def test_no_tma_multicast(path):
     # a load into several CTAs' shared memory is for code that single-GPU runs alone use
     with open(path) as f:
         assert ".multicast" not in f.read()
+
+
+def kernels(text):
+    """(name, body) of every __global__ function."""
+    for m in re.finditer(r"__global__\s+void\b", text):
+        at = text.index("{", text.index(") {", m.end()))
+        depth, i = 0, at
+        while True:
+            depth += {"{": 1, "}": -1}.get(text[i], 0)
+            i += 1
+            if depth == 0:
+                break
+        yield re.search(r"\b(k_\w+)\s*\(", text[m.end():]).group(1), text[at:i]
+
+
+@pytest.mark.parametrize("path", SOURCES, ids=os.path.basename)
+def test_chained_kernels_wait_before_they_let_the_next_one_start(path):
+    # a kernel may then read, ahead of its own wait, whatever the one right before it does not write
+    with open(path) as f:
+        for name, body in kernels(f.read()):
+            let = body.find("let_next_start()")
+            assert let < 0 or body.find("wait_for_previous()", let) < 0, name
