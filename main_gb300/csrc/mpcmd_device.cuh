@@ -351,14 +351,15 @@ __device__ __forceinline__ double to_f64(double f) { return f; }
 // before it has ended and its writes are visible, and then lets the kernel after
 // it take up the SMs that are free.  What a kernel does before that call may
 // touch only memory that the kernel right before it does not write: everything
-// earlier in the stream has ended by then, because the kernel before it let it
-// start only after its own wait.  An MD step of two
-// short kernels takes 9.6 us instead of 15.4, of which 5 were gaps (one dimer,
-// 30^3 cells, FP32).  A launch through launch_next is only for kernels that call
-// after_previous (or wait_for_previous, when they let nothing start); other
-// kernels, copies and memsets in the stream wait for its end as they always do.
-// The first kernel of a chain, an ordinary launch, may let the next one start at
-// once: nothing before it still runs.
+// earlier in the stream has ended by then and its writes are in L2, because the
+// kernel before it let it start only after its own wait.  Only that wait orders
+// this SM's L1, so what an earlier kernel of the chain wrote is read with __ldcg
+// there.  An MD step of two short kernels takes 9.6 us instead of 15.4, of which 5
+// were gaps (one dimer, 30^3 cells, FP32).  A launch through launch_next is only
+// for kernels that call after_previous (or wait_for_previous, when they let
+// nothing start); other kernels, copies and memsets in the stream wait for its
+// end as they always do.  The first kernel of a chain, an ordinary launch, may let
+// the next one start at once: nothing before it still runs.
 __device__ __forceinline__ void let_next_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void after_previous() {

@@ -1211,7 +1211,7 @@ template <typename T, bool OWN>
 __global__ void __launch_bounds__(TPB, sizeof(T) == 4 ? 5 : 1) k_force(Dev<T> d, KParams<T> kp, StepArgs a) {
   // The entry's state; after the dimer step, which writes none of it, the first
   // entry's arrives while that ends (a period of 64 dimers between walls 1.34 ->
-  // 1.28 ms).
+  // 1.28 ms), from L2 (__ldcg: see after_previous).
   uint32_t cell = 0, idx = 0;
   T ox = 0, oy = 0, oz = 0, vx = 0, vy = 0, vz = 0;
   T msd0 = (T)0;   // loaded with the rest: its use at the end would wait on it
@@ -1222,21 +1222,21 @@ __global__ void __launch_bounds__(TPB, sizeof(T) == 4 ? 5 : 1) k_force(Dev<T> d,
     cell = 0; idx = 0; fl = 0; np = 0;
     ox = oy = oz = vx = vy = vz = msd0 = (T)0;
     if (j >= nin) return;
-    if (a.advance && !a.mpc) msd0 = d.sh.msd[j];
-    cell = d.sh.cell[j];
-    ox = d.sh.ox[j]; oy = d.sh.oy[j]; oz = d.sh.oz[j];
-    vx = d.sh.vx[j]; vy = d.sh.vy[j]; vz = d.sh.vz[j];
-    fl = d.sh.flag[j];
-    np = d.sh.np[j];
+    if (a.advance && !a.mpc) msd0 = __ldcg(&d.sh.msd[j]);
+    cell = __ldcg(&d.sh.cell[j]);
+    ox = __ldcg(&d.sh.ox[j]); oy = __ldcg(&d.sh.oy[j]); oz = __ldcg(&d.sh.oz[j]);
+    vx = __ldcg(&d.sh.vx[j]); vy = __ldcg(&d.sh.vy[j]); vz = __ldcg(&d.sh.vz[j]);
+    fl = __ldcg(&d.sh.flag[j]);
+    np = __ldcg(&d.sh.np[j]);
     // the main index keys the catalysis draws and orders the species lists;
     // without owner tags or the on-exit record nothing here needs the slot,
     // so after a re-sort the entry's main index replaces it
-    idx = (d.lid && !OWN && !d.inc) ? d.sh.mid[j] : d.sh.idx[j];
-    packed = *reinterpret_cast<const uint4*>(d.sh.sph + (size_t)j * PAIRMAX);
+    idx = __ldcg((d.lid && !OWN && !d.inc) ? &d.sh.mid[j] : &d.sh.idx[j]);
+    packed = __ldcg(reinterpret_cast<const uint4*>(d.sh.sph + (size_t)j * PAIRMAX));
   };
   bool loaded = a.after_dimer && (int)blockIdx.x < a.g_force;
   if (loaded) {
-    const unsigned int nin = d.ctr->n_inside;
+    const unsigned int nin = __ldcg(&d.ctr->n_inside);
     load(wave_first(nin, a.g_force), nin);
   }
   after_previous();
@@ -1815,9 +1815,9 @@ __global__ void k_dimer_split(Dev<T> d, KParams<T> kp, StepArgs a, int mode, dou
   const int s1 = 2 * kk, s2 = 2 * kk + 1;
   double X1 = 0, X2 = 0, V1 = 0, V2 = 0, F1 = 0, F2 = 0, Q1 = 0, Q2 = 0;
   if (live && comp) {
-    X1 = d.dpos[3 * s1 + c]; X2 = d.dpos[3 * s2 + c];
-    V1 = d.dvel[3 * s1 + c]; V2 = d.dvel[3 * s2 + c];
-    Q1 = d.dq[3 * s1 + c]; Q2 = d.dq[3 * s2 + c];
+    X1 = __ldcg(&d.dpos[3 * s1 + c]); X2 = __ldcg(&d.dpos[3 * s2 + c]);
+    V1 = __ldcg(&d.dvel[3 * s1 + c]); V2 = __ldcg(&d.dvel[3 * s2 + c]);
+    Q1 = __ldcg(&d.dq[3 * s1 + c]); Q2 = __ldcg(&d.dq[3 * s2 + c]);
   }
   double fw1 = 0., pw1 = 0., fw2 = 0., pw2 = 0.;
   if ((mode & 1) && live && c == 2 && !per) {
@@ -1989,10 +1989,10 @@ __global__ void k_rotor_split(Dev<T> d, KParams<T> kp, StepArgs a, int mode, int
   const int s1 = 2 * kk, s2 = 2 * kk + 1;
   double X1 = 0, X2 = 0, V1 = 0, V2 = 0, F1 = 0, F2 = 0, Q1 = 0, Q2 = 0, A = 0;
   if (live && comp) {
-    X1 = d.dpos[3 * s1 + c]; X2 = d.dpos[3 * s2 + c];
-    V1 = d.dvel[3 * s1 + c]; V2 = d.dvel[3 * s2 + c];
-    Q1 = d.dq[3 * s1 + c]; Q2 = d.dq[3 * s2 + c];
-    A = d.anchor[3 * kk + c];
+    X1 = __ldcg(&d.dpos[3 * s1 + c]); X2 = __ldcg(&d.dpos[3 * s2 + c]);
+    V1 = __ldcg(&d.dvel[3 * s1 + c]); V2 = __ldcg(&d.dvel[3 * s2 + c]);
+    Q1 = __ldcg(&d.dq[3 * s1 + c]); Q2 = __ldcg(&d.dq[3 * s2 + c]);
+    A = __ldcg(&d.anchor[3 * kk + c]);
   }
   // (only the dimer step before wrote the state read so far)
   after_previous();

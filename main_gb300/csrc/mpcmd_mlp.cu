@@ -1011,9 +1011,9 @@ __global__ void __launch_bounds__(DxPipe::THREADS, 1)
 // refreshes the BF16 copies [n, k] and [k, n].  Work units: the 128 x 64 tiles of
 // every layer, then blocks of 64 biases; 5 of its 8 us are Adam's divisions and
 // root, so 16 warps share a tile (8: 7 us); the parameters and moments (24 bytes a
-// weight, in L2) are fetched before the previous kernel has ended: only this kernel
-// writes them, in the step before, and every kernel of a step lets the next one
-// start after its own wait.
+// weight, in L2) are fetched before the previous kernel has ended (__ldcg: see
+// after_previous): only this kernel writes them, in the step before, and every
+// kernel of a step lets the next one start after its own wait.
 struct AdamArgs {
   float lr, b1, b2, eps, c1, c2;
 };
@@ -1103,9 +1103,9 @@ __global__ void __launch_bounds__(DwPipe::THREADS, 1)
         if (UPDATE && real) {
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
-            x[i] = *reinterpret_cast<const float4*>(ly.w + at + i * step);
-            m1[i] = *reinterpret_cast<const float4*>(ly.m + at + i * step);
-            m2[i] = *reinterpret_cast<const float4*>(ly.v + at + i * step);
+            x[i] = __ldcg(reinterpret_cast<const float4*>(ly.w + at + i * step));
+            m1[i] = __ldcg(reinterpret_cast<const float4*>(ly.m + at + i * step));
+            m2[i] = __ldcg(reinterpret_cast<const float4*>(ly.v + at + i * step));
           }
         }
         if (!p.ready(j)) break;
@@ -1160,7 +1160,7 @@ __global__ void __launch_bounds__(DwPipe::THREADS, 1)
         // four rows a warp, their loads in flight together; lane r finishes row r
         const int n0 = (u - ly.first_bias) * 64 + 4 * ew, n = n0 + (lane & 3);
         float b = 0.f, m1 = 0.f, m2 = 0.f;
-        if constexpr (UPDATE) { b = ly.bw[n]; m1 = ly.bm[n]; m2 = ly.bv[n]; }
+        if constexpr (UPDATE) { b = __ldcg(ly.bw + n); m1 = __ldcg(ly.bm + n); m2 = __ldcg(ly.bv + n); }
         mpcmd::wait_for_previous();
         float s[4] = {};
         const __nv_bfloat16* zp = ly.dzt + (size_t)n0 * a.rows + lane;

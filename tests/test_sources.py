@@ -37,3 +37,12 @@ def test_chained_kernels_wait_before_they_let_the_next_one_start(path):
         for name, body in kernels(f.read()):
             let = body.find("let_next_start()")
             assert let < 0 or body.find("wait_for_previous()", let) < 0, name
+
+
+@pytest.mark.parametrize("path", SOURCES, ids=os.path.basename)
+def test_state_read_before_the_wait_comes_from_l2(path):
+    # until a kernel has waited, its SM's L1 may hold lines that an earlier kernel of the chain has changed since
+    with open(path) as f:
+        for name, body in kernels(f.read()):
+            ahead = body[:max(body.find("after_previous()"), body.find("wait_for_previous()"), 0)]
+            assert not re.findall(r"(?<!&)\bd(?:\.\w+)+(?:->|\s*\[)", ahead), name
