@@ -333,13 +333,45 @@ __device__ __forceinline__ void pair_add_prod(PairSum& s, float wh, float wl, fl
   pair_add(s, p);
   s.lo = __fadd_rn(s.lo, __fmaf_rn(wh, xl, __fmaf_rn(wl, xh, e)));
 }
-__device__ __forceinline__ void pair_merge(PairSum& s, float hi, float lo) {
-  pair_add(s, hi);
-  s.lo = __fadd_rn(s.lo, lo);
-}
 __device__ __forceinline__ double pair_value(const PairSum& s) {
   // an infinity or NaN stands in hi; lo is then meaningless
   return isfinite(s.hi) ? widen_f32(s.hi) + widen_f32(s.lo) : widen_f32(s.hi);
+}
+
+// A running sum in three floats, hi + mid + lo: the rounding errors of hi are
+// summed in mid and those of mid in lo, so that what is lost stays below 2^-53
+// of the sum of magnitudes and the value is that of an FP64 sum, or better.
+struct TripleSum {
+  float hi, mid, lo;
+};
+// s = fl(s + x); the rounding error (exact; Knuth's TwoSum).
+__device__ __forceinline__ float add_error(float& s, float x) {
+  const float t = __fadd_rn(s, x);
+  const float b = __fadd_rn(t, -s);
+  const float e = __fadd_rn(__fadd_rn(s, -__fadd_rn(t, -b)), __fadd_rn(x, -b));
+  s = t;
+  return e;
+}
+__device__ __forceinline__ void triple_add(TripleSum& s, float x) {
+  const float e = add_error(s.hi, x);
+  s.lo = __fadd_rn(s.lo, add_error(s.mid, e));
+}
+// s += x^2, exact for the magnitudes that in_triple_range takes.
+__device__ __forceinline__ void triple_add_square(TripleSum& s, float x) {
+  const float p = __fmul_rn(x, x);
+  triple_add(s, p);
+  s.lo = __fadd_rn(s.lo, add_error(s.mid, __fmaf_rn(x, x, -p)));
+}
+__device__ __forceinline__ double triple_value(const TripleSum& s) {
+  // (an infinity or NaN stands in hi; the rest is then meaningless)
+  return isfinite(s.hi) ? widen_f32(s.hi) + (widen_f32(s.mid) + widen_f32(s.lo)) : widen_f32(s.hi);
+}
+// Whether x is zero or between 2^-30 and 2^50 in magnitude: its square and the
+// square's rounding error are then floats, 2^27 of them add up to one, and what a
+// sum's parts lose below the smallest normal number does not count.
+__device__ __forceinline__ bool in_triple_range(float x) {
+  const uint32_t u = __float_as_uint(x) & 0x7FFFFFFFu;
+  return u == 0u || (u >= 0x30800000u && u <= 0x58800000u);
 }
 
 __device__ __forceinline__ double to_f64(float f) { return widen_f32(f); }

@@ -1221,27 +1221,21 @@ __global__ void k_ens_sort_gather(EDev<T> d, int64_t ntot) {
 //
 // FP32 build: bound by the 13 bytes a particle it reads.  In FP64 every
 // particle cost some 25 instructions of the FP64 pipe, which set the time:
-// 3.6 ms for the 133 million particles of 256 replicas.  The four sums run
-// as PairSum (exact terms, about 2^-45 relative error) down to one value per
-// warp, the counts as integers, and only the warps' results are added in FP64,
-// once for a block's part of a replica: 0.51 ms on GB300 (3.4 TB/s; 0.74 with
-// the sums closed after every tile and blocks for the rebuild's registers).
+// 3.6 ms for the 133 million particles of 256 replicas.  The four sums run as
+// TripleSum a thread (exact terms, what is lost below FP64's rounding), the
+// counts as integers, and the threads' results are added in FP64, once for a
+// block's part of a replica.  Speeds outside TripleSum's range and replicas whose
+// species have several masses are summed in FP64 particle by particle.
 constexpr int OBS_UNROLL = 2;   // particles per thread with their loads in flight together
 
 __device__ __forceinline__ void obs_tile_f32(const EDev<float>& d, int64_t lo, int64_t hi, const double* m,
                                              double* out) {
-  __shared__ float s_m[2][4];                       // masses as float pairs
-  __shared__ float s_h[4][MAX_BLOCK / 32], s_l[4][MAX_BLOCK / 32];
+  __shared__ double s_v[4][MAX_BLOCK / 32];
   __shared__ unsigned s_c[4][MAX_BLOCK / 32];
-  if (threadIdx.x < 4) {
-    const float mh = (float)m[threadIdx.x];
-    s_m[0][threadIdx.x] = mh;
-    s_m[1][threadIdx.x] = isfinite(mh) ? (float)(m[threadIdx.x] - (double)mh) : 0.f;
-  }
-  __syncthreads();
   // species of one mass (every input deck's) are weighted once, after the sum
   const bool one_mass = m[0] == m[1] && m[0] == m[2] && m[0] == m[3];
-  PairSum s[4] = {{0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}};   // momentum, twice the kinetic energy
+  TripleSum s[4] = {};                    // momentum, twice the kinetic energy, over the mass
+  double w[4] = {0., 0., 0., 0.};         // the same, weighted, of the particles summed in FP64
   unsigned c[4] = {0u, 0u, 0u, 0u};
   for (int64_t i0 = lo + threadIdx.x; i0 < hi; i0 += (int64_t)blockDim.x * OBS_UNROLL) {
     float v[OBS_UNROLL][3];
@@ -1259,36 +1253,29 @@ __device__ __forceinline__ void obs_tile_f32(const EDev<float>& d, int64_t lo, i
 #pragma unroll
     for (int u = 0; u < OBS_UNROLL; ++u) {
       if (sp[u] < 0) continue;
-      if (one_mass) {
+      if (one_mass && in_triple_range(v[u][0]) && in_triple_range(v[u][1]) && in_triple_range(v[u][2])) {
 #pragma unroll
-        for (int q = 0; q < 3; ++q) { pair_add(s[q], v[u][q]); pair_add_square(s[3], v[u][q]); }
+        for (int q = 0; q < 3; ++q) { triple_add(s[q], v[u][q]); triple_add_square(s[3], v[u][q]); }
       } else {
-        const float mh = s_m[0][sp[u]], ml = s_m[1][sp[u]];
-#pragma unroll
-        for (int q = 0; q < 3; ++q) {
-          const float x = v[u][q], p = __fmul_rn(x, x);
-          pair_add_prod(s[q], mh, ml, x, 0.f);
-          pair_add_prod(s[3], mh, ml, p, __fmaf_rn(x, x, -p));
-        }
+        const double mass = m[sp[u]], x = (double)v[u][0], y = (double)v[u][1], z = (double)v[u][2];
+        w[0] = fma(mass, x, w[0]); w[1] = fma(mass, y, w[1]); w[2] = fma(mass, z, w[2]);
+        w[3] = fma(mass, fma(x, x, fma(y, y, z * z)), w[3]);
       }
       c[0] += sp[u] == 0; c[1] += sp[u] == 1; c[2] += sp[u] == 2; c[3] += sp[u] == 3;
     }
   }
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = (int)(blockDim.x >> 5);
+  const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5, nw = (int)(blockDim.x >> 5);
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
-    for (int o = 16; o > 0; o >>= 1) {
-      const float h2 = __shfl_xor_sync(0xffffffffu, s[k].hi, o), l2 = __shfl_xor_sync(0xffffffffu, s[k].lo, o);
-      pair_merge(s[k], h2, l2);
-    }
+    double t = one_mass ? fma(m[0], triple_value(s[k]), w[k]) : w[k];
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
     const unsigned n = __reduce_add_sync(0xffffffffu, c[k]);
-    if (lane == 0) { s_h[k][w] = s[k].hi; s_l[k][w] = s[k].lo; s_c[k][w] = n; }
+    if (lane == 0) { s_v[k][wi] = t; s_c[k][wi] = n; }
   }
   __syncthreads();
   if (threadIdx.x < 4) {
     double t = 0.;
-    for (int i = 0; i < nw; ++i) t += pair_value(PairSum{s_h[threadIdx.x][i], s_l[threadIdx.x][i]});
-    if (one_mass) t *= m[0];
+    for (int i = 0; i < nw; ++i) t += s_v[threadIdx.x][i];
     atomicAdd(&out[threadIdx.x], threadIdx.x == 3 ? 0.5 * t : t);
   } else if (threadIdx.x < 8) {
     unsigned n = 0u;
