@@ -364,11 +364,10 @@ __device__ __forceinline__ void triple_add_square(TripleSum& s, float x) {
 }
 __device__ __forceinline__ double triple_value(const TripleSum& s) {
   // (an infinity or NaN stands in hi; the rest is then meaningless)
-  return isfinite(s.hi) ? widen_f32(s.hi) + (widen_f32(s.mid) + widen_f32(s.lo)) : widen_f32(s.hi);
+  return isfinite(s.hi) ? (double)s.hi + ((double)s.mid + (double)s.lo) : (double)s.hi;
 }
 // Whether x is zero or between 2^-30 and 2^50 in magnitude: its square and the
-// square's rounding error are then floats, 2^27 of them add up to one, and what a
-// sum's parts lose below the smallest normal number does not count.
+// square's rounding error are then floats, and 2^27 of them add up to one.
 __device__ __forceinline__ bool in_triple_range(float x) {
   const uint32_t u = __float_as_uint(x) & 0x7FFFFFFFu;
   return u == 0u || (u >= 0x30800000u && u <= 0x58800000u);

@@ -49,11 +49,11 @@
 #include <vector>
 
 #include "mpcmd.h"
-#include "mpcmd_device.cuh"   // PairSum
+#include "mpcmd_device.cuh"   // TripleSum, launch chaining
 
 namespace {
 
-using mpcmd::PairSum;
+using mpcmd::TripleSum;
 
 constexpr int BM = 128;        // output rows per tile (the MMA's M)
 constexpr int BK = 64;         // K per stage: one 128-byte swizzle row of BF16
@@ -153,6 +153,11 @@ __device__ __forceinline__ void mma_commit(uint32_t bar) {
 }
 __device__ __forceinline__ void tmem_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tmem_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ float tmem_ld1(uint32_t taddr) {
+  uint32_t r;
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];\n\ttcgen05.wait::ld.sync.aligned;" : "=r"(r) : "r"(taddr));
+  return __uint_as_float(r);
+}
 // A 32 x 32 block of the accumulator (lane = row, values = columns).
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
   uint32_t u[16];
@@ -729,12 +734,13 @@ __global__ void __launch_bounds__(INF_THREADS, 1)
           tmem_ld32(lanes + TM_ACC + (uint32_t)(b * INF_BN + c0), y);
           if constexpr (MODE == FORWARD) {
             // Weighted squared error and its gradient 2 w (y - t) / rows.  The 32
-            // terms of a chunk add up as a float pair, its chunks in FP64 (an FP64
-            // add a term would take 8 us: the pipe has two lanes an SM).
+            // terms of a chunk add up in three floats, without loss against FP64, and
+            // its chunks in FP64 (an FP64 add a term would take 8 us: the pipe has two
+            // lanes an SM).
             const int col = t * INF_BN + c0;
             const float4* tp = reinterpret_cast<const float4*>(buf + lane * INF_PITCH + (c0 < 32 * INF_GROUPS ? 0 : 32));
             const float wl = col + lane < a.n_out ? a.w[col + lane] : 0.f;
-            PairSum part{0.f, 0.f};
+            TripleSum part{};
             uint32_t g[16];
 #pragma unroll
             for (int q = 0; q < 32; q += 4) {
@@ -745,10 +751,12 @@ __global__ void __launch_bounds__(INF_THREADS, 1)
                 const float wt = __shfl_sync(0xffffffffu, wl, q + e);
                 float d = (y[q + e] + bias[c0 + q + e]) - tq[e];
                 d = row < a.rows && col + q + e < a.n_out ? d : 0.f;
-                mpcmd::pair_add(part, __fmul_rn(__fmul_rn(wt, d), d));
+                mpcmd::triple_add(part, __fmul_rn(__fmul_rn(wt, d), d));
                 y[q + e] = 2.f * wt * d;
               }
             }
+            const bool beyond = __any_sync(0xffffffffu, !isfinite(part.hi));
+            if (!beyond) loss += mpcmd::triple_value(part);
             // (a power of two divides exactly as its reciprocal multiplies)
             if (a.inv_rows != 0.f) {
 #pragma unroll
@@ -759,12 +767,21 @@ __global__ void __launch_bounds__(INF_THREADS, 1)
             }
 #pragma unroll
             for (int q = 0; q < 16; ++q) g[q] = pack_bf16(y[2 * q], y[2 * q + 1]);
-            loss += mpcmd::pair_value(part);
             if (row < a.rows) {
               uint4* dst = reinterpret_cast<uint4*>(a.dy + row * a.npad + col);
 #pragma unroll
               for (int q = 0; q < 4; ++q) dst[q] = make_uint4(g[4 * q], g[4 * q + 1], g[4 * q + 2], g[4 * q + 3]);
               put_columns(a.dyt + (size_t)col * a.rows + row, a.rows, g);
+            }
+            if (beyond) {
+              // a sum beyond FP32's largest number: the terms once more, in FP64
+#pragma unroll 1
+              for (int q = 0; q < 32; ++q) {
+                const float wt = __shfl_sync(0xffffffffu, wl, q);
+                float d = tmem_ld1(lanes + TM_ACC + (uint32_t)(b * INF_BN + c0 + q)) + bias[c0 + q];
+                d = row < a.rows && col + q < a.n_out ? d - reinterpret_cast<const float*>(tp)[q] : 0.f;
+                loss += (double)__fmul_rn(__fmul_rn(wt, d), d);
+              }
             }
           } else if (full) {
             stage_chunk(buf, lane, c0 % INF_WIDE, y, bias + c0);
