@@ -28,17 +28,19 @@
 // The arithmetic is the FP64 collision stage of the engine (k_accumulate_main,
 // k_cells and k_rotate_main in mpcmd_kernels.cuh; mpc_rotation_mod.f95:102-228
 // and RMPC_SelkovDimer.f90:15-120 in the reference) in four kernels: clear,
-// accumulate, cells (the affine map of every cell, in place of its sums) and
+// accumulate, cells (the map of every cell, in place of its sums) and
 // rotate.  GB300 issues FP64 at 1/64 of the FP32 rate (two lanes per SM and
 // cycle), so the FP64 instructions per particle set the time, not the 72
 // bytes a particle it moves: the axis (Philox, a sine and a cosine, a square
 // root) is drawn once per cell instead of once per particle, the shifted cell
 // comes from 32.32 fixed-point integers, and the rotation about the centre of
-// mass is one affine map, nine fused multiply-adds a particle.  5.1 million
-// unsorted particles in 80^3 cells: 348 us against 1615 with the axis drawn
+// mass is v_cm + M (v - v_cm), twelve FP64 instructions a particle (as the affine
+// map M v + (v_cm - M v_cm) nine, but then a particle alone in its cell, or at rest
+// in it, would not keep its velocity bit for bit).  5.1 million
+// unsorted particles in 80^3 cells: 342 us against 1615 with the axis drawn
 // and the rotation evaluated per particle (450 with 22 FP64 instructions a
-// particle from the centre of mass and the axis); the atomics take 124 us,
-// the cells 83 (102 with three divisions and unfused products), the rotation 123.
+// particle from the centre of mass and the axis); the atomics take 126 us,
+// the cells 75 (102 with three divisions and unfused products), the rotation 126.
 #include <algorithm>
 #include <cmath>
 #include <mutex>
@@ -59,8 +61,8 @@ constexpr int kThreads = 256;
 constexpr int64_t kOwnMap = 8192;
 
 // per shifted cell, 12 doubles (three whole sectors): first the count (an
-// unsigned int) and the sums of vx, vy, vz, then the map v -> M v + b as rows
-// M[q][0..2], b[q]
+// unsigned int) and the sums of vx, vy, vz, then the map v -> m + M (v - m) as
+// rows M[q][0..2], m[q]
 constexpr int kRec = 12;
 static __device__ __align__(256) double g_collide_scratch[kRec * kMaxCells];
 
@@ -154,14 +156,17 @@ __global__ void __launch_bounds__(kThreads) k_static_accumulate(KParams<double> 
   }
 }
 
-// The collision of a cell as an affine map v -> M v + b: centre of mass and
-// random axis (k_cells), M the rotation by the angle about the axis (both forms
-// of rotate_v; the projection form turns the other way), b = v_cm - M v_cm.
-// a0, a1: the cell's count and velocity sums.  False for an empty cell (no
-// particle reads it).
+// The collision of a cell as a map v -> m + M (v - m): m the centre of mass'
+// velocity, M the rotation by the angle about the random axis (k_cells; both forms
+// of rotate_v, the projection form turns the other way).  a0, a1: the cell's count
+// and velocity sums.  False for an empty cell (no particle reads it).
 struct Map {
-  double M[3][3], b[3];
+  double M[3][3], m[3];
 };
+// One component of the map for d = v - m: m itself where d is zero.
+__device__ __forceinline__ double turned(double M0, double M1, double M2, double m, const double (&d)[3]) {
+  return fma(M0, d[0], fma(M1, d[1], fma(M2, d[2], m)));
+}
 // sum / n for a count n with rn = 1 / n rounded to nearest, rounded as the
 // division (div_const); an infinite or undefined sum stays what it is.
 __device__ __forceinline__ double mean_of(double sum, double n, double rn) {
@@ -176,7 +181,7 @@ __device__ __forceinline__ bool cell_map(const KParams<double>& kp, uint32_t cel
   if (cnt == 0u) return false;
   const double n = (double)cnt;
   const double rn = 1.0 / n;
-  const double m[3] = {mean_of(a0.y, n, rn), mean_of(a1.x, n, rn), mean_of(a1.y, n, rn)};
+  w.m[0] = mean_of(a0.y, n, rn); w.m[1] = mean_of(a1.x, n, rn); w.m[2] = mean_of(a1.y, n, rn);
   double u1, u2, sp, cp;
   contract_pair(kp.seed, TAG_AXIS, cell, 0, step, u1, u2);
   sincos(2.0 * pi * u1, &sp, &cp);
@@ -187,8 +192,6 @@ __device__ __forceinline__ bool cell_map(const KParams<double>& kp, uint32_t cel
   w.M[0][0] = fma(k0, u[0], c); w.M[0][1] = fma(k0, u[1], -su[2]); w.M[0][2] = fma(k0, u[2], su[1]);
   w.M[1][0] = fma(k0, u[1], su[2]); w.M[1][1] = fma(k1, u[1], c); w.M[1][2] = fma(k1, u[2], -su[0]);
   w.M[2][0] = fma(k0, u[2], -su[1]); w.M[2][1] = fma(k1, u[2], su[0]); w.M[2][2] = fma(k2, u[2], c);
-#pragma unroll
-  for (int q = 0; q < 3; ++q) w.b[q] = fma(-w.M[q][2], m[2], fma(-w.M[q][1], m[1], fma(-w.M[q][0], m[0], m[q])));
   return true;
 }
 
@@ -202,7 +205,7 @@ __global__ void __launch_bounds__(kThreads) k_static_cells(KParams<double> kp, u
 #pragma unroll
     for (int q = 0; q < 3; ++q) {
       a[2 * q] = make_double2(w.M[q][0], w.M[q][1]);
-      a[2 * q + 1] = make_double2(w.M[q][2], w.b[q]);
+      a[2 * q + 1] = make_double2(w.M[q][2], w.m[q]);
     }
   }
 }
@@ -224,14 +227,16 @@ __global__ void __launch_bounds__(kThreads) k_static_rotate(KParams<double> kp, 
     if constexpr (OWN_MAP) {
       Map c;
       if (!cell_map(kp, key, step, a[0], a[1], c)) continue;
+      const double d[3] = {v0 - c.m[0], v1 - c.m[1], v2 - c.m[2]};
 #pragma unroll
-      for (int q = 0; q < 3; ++q) w[q] = fma(c.M[q][0], v0, fma(c.M[q][1], v1, fma(c.M[q][2], v2, c.b[q])));
+      for (int q = 0; q < 3; ++q) w[q] = turned(c.M[q][0], c.M[q][1], c.M[q][2], c.m[q], d);
     } else {
+      double2 r[6];
 #pragma unroll
-      for (int q = 0; q < 3; ++q) {
-        const double2 h = a[2 * q], l = a[2 * q + 1];
-        w[q] = fma(h.x, v0, fma(h.y, v1, fma(l.x, v2, l.y)));
-      }
+      for (int q = 0; q < 6; ++q) r[q] = a[q];
+      const double d[3] = {v0 - r[1].y, v1 - r[3].y, v2 - r[5].y};
+#pragma unroll
+      for (int q = 0; q < 3; ++q) w[q] = turned(r[2 * q].x, r[2 * q].y, r[2 * q + 1].x, r[2 * q + 1].y, d);
     }
     vx[i] = w[0]; vy[i] = w[1]; vz[i] = w[2];
   }
