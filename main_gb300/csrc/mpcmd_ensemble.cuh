@@ -136,7 +136,6 @@ struct EDev {
   const int64_t* ct_hi;
   int n_ctiles;
   STile* stile;            // shell tiles of every replica
-  uint32_t* st_prefix;     // [R] first shell tile of each replica
   uint32_t* rt_need;       // [R] rebuild units of each replica (0 when it does not rebuild)
   uint32_t* rt_prefix;     // [R + 1] first rebuild unit of each replica
   // samples
@@ -478,61 +477,88 @@ __device__ __forceinline__ bool last_block(unsigned* counter, unsigned blocks, b
   return last;
 }
 
-// The shell tiles of every replica, from the shell sizes.  One block.
-template <typename T>
-__device__ __forceinline__ void write_shell_tiles(const EDev<T>& d, int shell_block, unsigned* part) {
-  const int nt = blockDim.x;
-  const int chunk = (d.R + nt - 1) / nt;
-  const int lo = min(d.R, (int)threadIdx.x * chunk), hi = min(d.R, lo + chunk);
-  unsigned local = 0;
-  for (int r = lo; r < hi; ++r) local += (__ldcg(&d.dyn[r].n_shell) + shell_block - 1) / shell_block;
-  block_scan(part, local);
-  unsigned run = threadIdx.x ? part[threadIdx.x - 1] : 0u;
-  for (int r = lo; r < hi; ++r) {
-    d.st_prefix[r] = run;
-    run += (__ldcg(&d.dyn[r].n_shell) + shell_block - 1) / shell_block;
-  }
-  if (threadIdx.x == nt - 1) d.g->ntiles_s = part[nt - 1];
-  __threadfence();   // (the prefixes are read back from L2)
-  __syncthreads();
-  // a warp per replica writes its tiles
-  const int lane = threadIdx.x & 31;
-  for (int r = threadIdx.x >> 5; r < d.R; r += nt >> 5) {
-    const unsigned n = __ldcg(&d.dyn[r].n_shell), first = __ldcg(&d.st_prefix[r]);
-    const int64_t e0 = d.rep[r].soff;
-    for (unsigned k = lane; k * shell_block < n; k += 32)
-      d.stile[first + k] =
-          STile{(uint32_t)r, min((unsigned)shell_block, n - k * shell_block), e0 + (int64_t)k * shell_block};
-  }
-}
-
-template <typename T>
-__global__ void k_ens_tiles(EDev<T> d, int shell_block) {
-  __shared__ unsigned part[256];
-  write_shell_tiles(d, shell_block, part);
-}
-
-// After the lists of the rebuilding replicas are complete (the last block of
-// the rebuild): their time_penetrate (main_pattern.f95:187,
-// evolve_mod.f95:555-563) and the shell work tiles.
-template <typename T>
-__device__ __forceinline__ void finish_rebuild(const EDev<T>& d, int shell_block, unsigned* part) {
-  for (int r = threadIdx.x; r < d.R; r += blockDim.x) {
-    Dyn<T>& y = d.dyn[r];
-    const Rep<T>& R = d.rep[r];
-    if (y.rebuild) {
-      const double maxt = __longlong_as_double((long long)__ldcg(&y.maxv2));
-      y.time_penetrate = (int)floor((0.5 * R.skin / sqrt(maxt)) / R.kp.dtd);
+// The shell tiles of every replica, from the shell sizes; FINISH: after the
+// lists of the rebuilding replicas are complete, whose time_penetrate this sets
+// first (main_pattern.f95:187, evolve_mod.f95:555-563).  One block, which every MD
+// step of a large ensemble waits for: a thread per replica with the next one's
+// state on its way, 32 replicas' tiles written by their warp together.  An MD step
+// of 2,048 replicas of 4,096 particles takes 52 us, of 256 of 40,960 particles 36
+// (a warp per replica and three rounds of loads: 92 and 40; a launch of 1,024
+// threads of its own: 70 and 57).
+template <typename T, bool FINISH>
+__device__ __forceinline__ void close_lists(const EDev<T>& d, int shell_block, unsigned* part /* [warps] */) {
+  const int nt = blockDim.x, nw = nt >> 5, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  unsigned n_next = 0u, cap_next = 0u;
+  int rebuild_next = 0;
+  int64_t e_next = 0;
+  double maxt_next = 0., skin_next = 0., dt_next = 0.;
+  auto fetch = [&](int r) {
+    n_next = 0u;
+    rebuild_next = 0;
+    if (r >= d.R) return;
+    n_next = __ldcg(&d.dyn[r].n_shell);
+    e_next = d.rep[r].soff;
+    if (FINISH) {
+      rebuild_next = d.dyn[r].rebuild;
+      maxt_next = __longlong_as_double((long long)__ldcg(&d.dyn[r].maxv2));
+      skin_next = d.rep[r].skin;
+      dt_next = d.rep[r].kp.dtd;
+      cap_next = (unsigned)d.rep[r].scap;
+    }
+  };
+  fetch(threadIdx.x);
+  unsigned run = 0u;
+  for (int r0 = 0; r0 < d.R; r0 += nt) {
+    const int r = r0 + (int)threadIdx.x;
+    const bool rebuilt = FINISH && rebuild_next;
+    const unsigned n = rebuilt ? min(n_next, cap_next) : n_next;
+    const int64_t e0 = e_next;
+    if (rebuilt) {
+      Dyn<T>& y = d.dyn[r];
+      y.time_penetrate = (int)floor((0.5 * skin_next / sqrt(maxt_next)) / dt_next);
       y.time_count = 0;
       y.rebuild = 0;
       y.maxv2 = 0ull;
       y.rebuilds += 1;
-      if (__ldcg(&y.n_shell) > (unsigned)R.scap) y.n_shell = (unsigned)R.scap;
+      if (n < n_next) y.n_shell = n;
     }
+    fetch(r + nt);
+    const unsigned tiles = (n + shell_block - 1) / shell_block;
+    unsigned upto = tiles;   // tiles of the warp's replicas up to this one
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned v = __shfl_up_sync(0xffffffffu, upto, o);
+      if (lane >= o) upto += v;
+    }
+    if (lane == 31) part[w] = upto;
+    __syncthreads();
+    unsigned first = run;
+    for (int q = 0; q < nw; ++q) {
+      if (q < w) first += part[q];
+      run += part[q];
+    }
+    const unsigned count = __shfl_sync(0xffffffffu, upto, 31);
+    for (unsigned base = 0; base < count; base += 32) {
+      const unsigned q = base + lane;
+      int j = 0;   // the lane whose replica has tile q
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1)
+        if (__shfl_sync(0xffffffffu, upto, j + o - 1) <= q) j += o;
+      const unsigned nj = __shfl_sync(0xffffffffu, n, j), k = q - __shfl_sync(0xffffffffu, upto - tiles, j);
+      const int64_t ej = __shfl_sync(0xffffffffu, (long long)e0, j);
+      if (q < count)
+        d.stile[first + q] = STile{(uint32_t)(r0 + 32 * w + j), min((unsigned)shell_block, nj - k * shell_block),
+                                   ej + (int64_t)k * shell_block};
+    }
+    __syncthreads();
   }
-  __threadfence();   // (the clamped sizes are read back from L2)
-  __syncthreads();
-  write_shell_tiles(d, shell_block, part);
+  if (threadIdx.x == 0) d.g->ntiles_s = run;
+}
+
+template <typename T>
+__global__ void k_ens_tiles(EDev<T> d, int shell_block) {
+  __shared__ unsigned part[8];
+  close_lists<T, false>(d, shell_block, part);
 }
 
 // A particle's state, loaded (zeros past the end) ahead of its use: the loops
@@ -556,12 +582,13 @@ struct ParticleIn {
 // replicas out in contiguous parts (tiles of 4,096 in turn left a third wave half
 // empty and cost a search, two barriers and an atomic each), fetch one particle
 // ahead and keep to the registers of four blocks an SM.  256 replicas, 10 of them
-// rebuilding in an MD step: 57 us a step on GB300 (65 before; tiles of 1,024: 90).
+// rebuilding in an MD step: 53 us a step on GB300 (65 in tiles of 4,096, 90 in tiles of
+// 1,024).
 template <typename T>
 __global__ void __launch_bounds__(MAX_BLOCK, sizeof(T) == 4 ? 4 : 0)
     k_ens_rebuild(EDev<T> d, int mode, int shell_block, int advance_step) {
   __shared__ T red[32];
-  __shared__ unsigned part[MAX_BLOCK];
+  __shared__ unsigned part[MAX_BLOCK / 32];
   const unsigned units = d.rt_prefix[d.R];
   if (advance_step && blockIdx.x == 0 && threadIdx.x == 0) d.g->cstep += 1;   // (nothing in this launch reads it)
   unsigned u = (unsigned)((uint64_t)units * blockIdx.x / gridDim.x);
@@ -630,7 +657,7 @@ __global__ void __launch_bounds__(MAX_BLOCK, sizeof(T) == 4 ? 4 : 0)
   // the last of the blocks that had work finishes the rebuild (most MD steps
   // rebuild no replica and end here)
   if ((mode & M_LISTS) && works && last_block(&d.g->arrived[1], min(units, gridDim.x)))
-    finish_rebuild(d, shell_block, part);
+    close_lists<T, true>(d, shell_block, part);
 }
 
 // --------------------------------------------------------------- forces ----

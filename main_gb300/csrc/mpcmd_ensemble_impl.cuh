@@ -189,7 +189,7 @@ struct Ensemble : EnsembleBase {
     s |= alloc(scan_tmp, scan_tmp_words(ctot));
     Rep<T>* drep = nullptr; Dyn<T>* ddyn = nullptr; Glob* dg = nullptr;
     s |= alloc(drep, R); s |= alloc(ddyn, R); s |= alloc(dg, 1);
-    s |= alloc(d.st_prefix, R); s |= alloc(d.rt_need, R);
+    s |= alloc(d.rt_need, R);
     s |= alloc(d.stile, stot / 32 + R);   // (at least 32 entries in every tile but a replica's last)
     s |= alloc(d.rt_prefix, R + 1);
     s |= alloc(d_mass, 4 * (int64_t)R); s |= alloc(d_obs, 8 * (int64_t)R);
