@@ -206,7 +206,8 @@ struct Engine : EngineBase {
   int64_t resort_every = 0, resorts = 0;
   uint32_t *lid_a = nullptr, *lid_b = nullptr, *lpos_buf = nullptr;
   // particles per shifted cell of the last mpc_rotation stage call (k_cells
-  // clears the sums they come from), for mpcmd_get_cell_rotation
+  // clears the sums they come from), for mpcmd_get_cell_rotation; allocated by
+  // the first such call
   uint32_t* cnt_snap = nullptr;
   double w3 = 1.0;
   unsigned int n_inside = 0;
@@ -441,7 +442,6 @@ struct Engine : EngineBase {
     if (c.owner_tags) { r |= alloc(d.owner, n); r |= alloc(d.owner2, n); }
     if (c.catalysis == MPCMD_CAT_ON_EXIT) { r |= alloc(d.inc, n); r |= alloc(d.inc2, n); }
     r |= alloc(lid_a, n); r |= alloc(lid_b, n); r |= alloc(lpos_buf, n);
-    r |= alloc(cnt_snap, kp.ncell_shift);
     if (r) return MPCMD_ERR_ALLOC;
     d.lid = d.lid2 = d.lpos = nullptr;
     // a re-sort every ten collision periods (the cell order of a diffusing
@@ -452,7 +452,6 @@ struct Engine : EngineBase {
     CK(cudaMemsetAsync(d.dcnt, 0, 4 * (size_t)kp.ncell, st));
     CK(cudaMemsetAsync(d.dfirst, 0xFF, 16 * (size_t)kp.ncell, st));
     CK(cudaMemsetAsync(d.affected, 0, (size_t)kp.ncell, st));
-    CK(cudaMemsetAsync(cnt_snap, 0, 4 * (size_t)kp.ncell_shift, st));
     CK(cudaMemsetAsync(d.ctr, 0, sizeof(Counters), st));
     CK(cudaMemsetAsync(d.facc, 0, sizeof(double) * 4 * std::max<int64_t>(ns, 1), st));
     CK(cudaMemsetAsync(d.fmot, 0, sizeof(double) * 4 * std::max<int64_t>(ns, 1), st));
@@ -998,6 +997,7 @@ struct Engine : EngineBase {
 
   int rotation_stage() override {
     if (advanced) return MPCMD_ERR_STATE;
+    if (!cnt_snap && alloc(cnt_snap, kp.ncell_shift)) return MPCMD_ERR_ALLOC;
     flush_shell();
     draw_shift(cstep);
     StepArgs a = args(cstep);
@@ -1338,7 +1338,8 @@ struct Engine : EngineBase {
         if (cm) cm[3 * c + q] = (double)r[(size_t)(6 * c + q)];
         if (axis) axis[3 * c + q] = (double)r[(size_t)(6 * c + 3 + q)];
       }
-    if (count) CK(cudaMemcpy(count, cnt_snap, 4 * (size_t)kp.ncell_shift, cudaMemcpyDeviceToHost));
+    if (count && !cnt_snap) std::memset(count, 0, 4 * (size_t)kp.ncell_shift);
+    else if (count) CK(cudaMemcpy(count, cnt_snap, 4 * (size_t)kp.ncell_shift, cudaMemcpyDeviceToHost));
     return MPCMD_OK;
   }
 
