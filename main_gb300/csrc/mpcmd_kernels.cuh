@@ -2122,7 +2122,7 @@ __global__ void k_rotor_split(Dev<T> d, KParams<T> kp, StepArgs a, int mode, int
   if (live && c == 0 && iters) atomicAdd(&d.ctr->rattle_iters, iters);
 }
 
-constexpr int DIMER_EARLY = 8;   // blocks of eight dimers
+constexpr int DIMER_EARLY = 8;   // blocks of eight dimers, far fewer than SMs
 template <typename T>
 void Launch<T>::dimer(const Dev<T>& d, const KParams<T>& kp, const StepArgs& a, int mode, double w3,
                       int rattle_max, cudaStream_t st) {
@@ -2130,8 +2130,10 @@ void Launch<T>::dimer(const Dev<T>& d, const KParams<T>& kp, const StepArgs& a, 
   // four lanes per dimer, one 32-lane block per eight dimers (spread over the SMs)
   const int blocks = (4 * kp.nd + 31) / 32;
   // Started early, the blocks take the first SMs that have room, and many of
-  // them share an FP64 pipe there: a collision period of 64 dimers is 3 % faster
-  // for it, of 100 dimers 6 % slower, of 256 dimers 16 %.
+  // them share an FP64 pipe there.  A run of collective boxes is faster for it by
+  // 21 % with 1 dimer, 18 % with 16, 13 % with 48, 3 % with 64 and 72, 7 % with 80
+  // (FP64: 10, 7, 3, 2, 0, -0.5 %); with 96 it is 1 % slower, with 256 15 %; of
+  // rotors by 4 % with 9 to 36, equal with 64 to 81, 1 % slower with 100 (FP64 6 %).
   const bool early = blocks <= DIMER_EARLY;
   if (kp.rotor) {
     if (early) launch_next(k_rotor_split<T>, blocks, 32, st, d, kp, a, mode, rattle_max);

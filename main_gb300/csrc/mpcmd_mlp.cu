@@ -207,43 +207,6 @@ __device__ __forceinline__ float dsilu_f(float z) {
   return s * (1.f + z * (1.f - s));
 }
 
-// Row-major store of a warp's 32-row block (thread = row, W 32-bit words
-// per row) through the warp's staging tile (P words per row): the block is
-// written in the thread-per-row layout and read back so that each lane
-// carries VB consecutive bytes of one row and each store instruction writes
-// whole rows (full sectors), rows from `row0` of `base` with pitch `pitch`
-// bytes.
-template <int W, int VB, int P>
-__device__ __forceinline__ void store_rows(uint32_t* buf, const uint32_t (&w)[W], int lane, char* base, int row0,
-                                           size_t pitch, int rows, int wlim = W) {
-  static_assert(W % 4 == 0 && W <= P && P % 4 == 0 && (VB == 16 || VB == 8 || VB == 4), "staged row store shape");
-  constexpr int STAGE_PITCH = P;
-#pragma unroll
-  for (int q = 0; q < W; q += 4)
-    *reinterpret_cast<uint4*>(buf + lane * STAGE_PITCH + q) = make_uint4(w[q], w[q + 1], w[q + 2], w[q + 3]);
-  __syncwarp();
-  constexpr int LPR = W * 4 / VB;    // lanes per row
-  constexpr int RPI = 32 / LPR;      // rows per instruction
-  const int sub = lane / LPR, q = lane % LPR;
-  const int w0 = q * (VB / 4);       // first word of this lane's piece
-#pragma unroll 4
-  for (int it = 0; it < 32 / RPI; ++it) {
-    const int r = it * RPI + sub;
-    if (r < rows && w0 < wlim) {
-      char* dst = base + (size_t)(row0 + r) * pitch + q * VB;
-      const uint32_t* src = buf + r * STAGE_PITCH + w0;
-      if (w0 + VB / 4 <= wlim) {
-        if (VB == 16) *reinterpret_cast<uint4*>(dst) = *reinterpret_cast<const uint4*>(src);
-        else if (VB == 8) *reinterpret_cast<uint2*>(dst) = *reinterpret_cast<const uint2*>(src);
-        else *reinterpret_cast<uint32_t*>(dst) = *src;
-      } else {
-        for (int k = 0; w0 + k < wlim; ++k) reinterpret_cast<uint32_t*>(dst)[k] = src[k];
-      }
-    }
-  }
-  __syncwarp();
-}
-
 __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
   const __nv_bfloat162 p = __floats2bfloat162_rn(lo, hi);
   return *reinterpret_cast<const uint32_t*>(&p);
@@ -274,9 +237,9 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
 //     columns, each repeating the (much cheaper) hidden layers: with fewer row
 //     tiles than SMs all of them, else the last partial wave.
 // Inference: one launch instead of six (one conversion and five GEMMs with the
-// activations through L2): with the call's own cost, 64 points take 43 us against 80, 65,536
-// points 196 against 283.  A hidden layer takes 3 us (1 us of MMAs, then its
-// epilogue, then the next: a chain), 256 output columns of 128 rows 4.4 us.
+// activations through L2): with the call's own cost, 64 points take 39 us against
+// 81, 65,536 points 192 against 284.  A hidden layer takes 3 us (1 us of MMAs, then
+// its epilogue, then the next: a chain), two output tiles of 128 columns 4.4 us.
 constexpr int INF_GROUPS = 3;                      // epilogue groups of four warps
 constexpr int INF_EPI = 4 * INF_GROUPS;
 constexpr int INF_THREADS = 64 + 32 * INF_EPI;
@@ -368,8 +331,8 @@ __device__ __forceinline__ void put_columns(__nv_bfloat16* dst, size_t ld, const
 // complete every instruction writes VB bytes a lane (VB: what the rows'
 // alignment allows) of as few rows as that covers.  L2 takes one request per
 // 128-byte line a piece of a row touches, whole or not, and rows of 2,050
-// values start anywhere in a line: 64-column pieces touch 3 lines for 2 and a
-// 256-column tile of 128 rows takes 4.4 us, 32-column pieces 2 for 1 and 5.7 us
+// values start anywhere in a line: 64-column pieces touch 3 lines for 2 and 256
+// columns of 128 rows take 4.4 us, 32-column pieces 2 for 1 and 5.7 us
 // (aligned rows: 3.1 us).  Measured and not kept: lines assembled whole in the
 // staging tile across chunks (7.6 us, the rotated staging costs more than the
 // requests saved), 128-column pieces of 16 or 8 rows at a time (4.7 and 6.1 us).
@@ -402,6 +365,20 @@ __device__ __forceinline__ void store_block(const uint32_t* buf, int lane, char*
       else *reinterpret_cast<uint32_t*>(d) = *s;
     }
   }
+}
+
+// A ragged piece of it: 32 columns staged a lane per row, of which `rows` rows
+// and `cols` columns are written.
+__device__ __forceinline__ void store_ragged(uint32_t* buf, const uint32_t (&w)[32], int lane, char* base, size_t pitch,
+                                             int rows, int cols) {
+#pragma unroll
+  for (int q = 0; q < 32; q += 4)
+    *reinterpret_cast<uint4*>(buf + lane * INF_PITCH + q) = make_uint4(w[q], w[q + 1], w[q + 2], w[q + 3]);
+  __syncwarp();
+#pragma unroll 4
+  for (int r = 0; r < 32; ++r)
+    if (r < rows && lane < cols) *reinterpret_cast<uint32_t*>(base + r * pitch + 4 * lane) = buf[r * INF_PITCH + lane];
+  __syncwarp();
 }
 
 // VB (INFER): the largest of 16, 8 and 4 bytes that divides the address of
@@ -794,7 +771,7 @@ __global__ void __launch_bounds__(INF_THREADS, 1)
             uint32_t w[32];
 #pragma unroll
             for (int q = 0; q < 32; ++q) w[q] = __float_as_uint(y[q] + bias[c0 + q]);
-            store_rows<32, 4, INF_PITCH>(buf, w, lane, yb + 4 * c0, 0, pitch, rows, cols - c0 < 32 ? cols - c0 : 32);
+            store_ragged(buf, w, lane, yb + 4 * c0, pitch, rows, cols - c0);
           }
         }
         tmem_fence_before();
@@ -1273,7 +1250,7 @@ struct mpcmd_mlp {
   DwMaps dw_maps{};
   DwArgs dw{};
   int64_t step = 0;
-  int sms = 1;             // SMs of the device (one persistent GEMM CTA each)
+  int sms = 1;             // SMs of the device
   cudaStream_t st = nullptr;
 
   ~mpcmd_mlp() {

@@ -57,7 +57,8 @@ constexpr int kMaxDevices = 64;
 constexpr int kThreads = 256;
 // Largest set whose particles each form their cell's map: a map takes some 200
 // FP64 instructions, 2 us for 8,192 particles on 152 SMs, about what the cells
-// kernel's launch costs.
+// kernel's launch costs (calls back to back: 8,192 particles 14.5 us against 15.3
+// with the cells kernel, 20,000 17.4 against 15.2).
 constexpr int64_t kOwnMap = 8192;
 
 // per shifted cell, 12 doubles (three whole sectors): first the count (an
@@ -298,10 +299,12 @@ extern "C" int mpcmd_collide_static(const double* x, const double* y, const doub
   const int grid = (int)std::min<int64_t>(want, (int64_t)nsm * 8);
   const int tgrid = (int)std::min<int64_t>((ncs + kThreads - 1) / kThreads, (int64_t)nsm * 8);
   k_static_clear<<<tgrid, kThreads, 0, st>>>(acc, ncs);
-  // Up to three blocks an SM each kernel starts while the one before it ends (1,536
-  // to 8,192 particles 14.4 us instead of 20.5, 80,000 22 instead of 26.7).
-  // Past that the early blocks crowd the first SMs that fall free, where they
-  // share the FP64 pipe (270,000 particles: 43.7 us instead of 33.7).
+  // Up to three blocks an SM each kernel starts while the one before it ends (calls
+  // back to back: 1,536 to 8,192 particles 14.5 us instead of 18.6, 80,000 20.5
+  // instead of 24.7, the 116,736 at the edge 19.3 instead of 24.8).  Towards eight
+  // blocks an SM, a whole wave, the early blocks crowd the first SMs that fall
+  // free, where they share the FP64 pipe (200,000 particles, 5 blocks: 26.9 instead
+  // of 29.1 us; 270,000, 7 blocks: 34.7 instead of 32.4).
   const bool early = grid <= 3 * nsm;
   auto next = [&](auto kernel, int blocks, auto... args) {
     if (early) launch_next(kernel, blocks, kThreads, st, args...);
