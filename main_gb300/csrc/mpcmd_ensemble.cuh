@@ -1229,7 +1229,8 @@ __global__ void k_ens_sort_gather(EDev<T> d, int64_t ntot) {
 // counts as integers, and the threads' results are added in FP64, once for a
 // block's part of a replica: 0.73 ms on GB300 (0.51 as float pairs, which keep
 // some 2^-45).  Speeds outside TripleSum's range and replicas whose species have
-// several masses are summed in FP64 particle by particle.
+// several masses are summed in FP64 particle by particle (69 million particles of
+// four masses 1.12 ms, of one mass 0.42; converted and multiplied out in FP64 2.02).
 constexpr int OBS_UNROLL = 2;   // particles per thread with their loads in flight together
 
 __device__ __forceinline__ void obs_tile_f32(const EDev<float>& d, int64_t lo, int64_t hi, const double* m,
@@ -1257,11 +1258,14 @@ __device__ __forceinline__ void obs_tile_f32(const EDev<float>& d, int64_t lo, i
 #pragma unroll
     for (int u = 0; u < OBS_UNROLL; ++u) {
       if (sp[u] < 0) continue;
-      if (one_mass && in_triple_range(v[u][0]) && in_triple_range(v[u][1]) && in_triple_range(v[u][2])) {
+      const bool in = in_triple_range(v[u][0]) && in_triple_range(v[u][1]) && in_triple_range(v[u][2]);
+      if (one_mass && in) {
 #pragma unroll
         for (int q = 0; q < 3; ++q) { triple_add(s[q], v[u][q]); triple_add_square(s[3], v[u][q]); }
       } else {
-        const double mass = m[sp[u]], x = (double)v[u][0], y = (double)v[u][1], z = (double)v[u][2];
+        // (widen_f32 leaves the FP64 pipe to the sums, for all but subnormal numbers)
+        const double mass = m[sp[u]], x = in ? widen_f32(v[u][0]) : (double)v[u][0];
+        const double y = in ? widen_f32(v[u][1]) : (double)v[u][1], z = in ? widen_f32(v[u][2]) : (double)v[u][2];
         w[0] = fma(mass, x, w[0]); w[1] = fma(mass, y, w[1]); w[2] = fma(mass, z, w[2]);
         w[3] = fma(mass, fma(x, x, fma(y, y, z * z)), w[3]);
       }
