@@ -206,9 +206,12 @@ struct Engine : EngineBase {
   int64_t resort_every = 0, resorts = 0;
   uint32_t *lid_a = nullptr, *lid_b = nullptr, *lpos_buf = nullptr;
   // particles per shifted cell of the last mpc_rotation stage call (k_cells
-  // clears the sums they come from), for mpcmd_get_cell_rotation; allocated by
-  // the first such call
+  // clears the sums they come from), for mpcmd_get_cell_rotation.  Large tables
+  // are allocated by the first such call, which few contexts make; small ones with
+  // the context (an allocation takes 170 us, a sixth of a call on 2.6 million
+  // particles).
   uint32_t* cnt_snap = nullptr;
+  static constexpr int64_t CNT_AT_CREATE = (int64_t)1 << 22;   // cells (16 MiB)
   double w3 = 1.0;
   unsigned int n_inside = 0;
 
@@ -442,6 +445,7 @@ struct Engine : EngineBase {
     if (c.owner_tags) { r |= alloc(d.owner, n); r |= alloc(d.owner2, n); }
     if (c.catalysis == MPCMD_CAT_ON_EXIT) { r |= alloc(d.inc, n); r |= alloc(d.inc2, n); }
     r |= alloc(lid_a, n); r |= alloc(lid_b, n); r |= alloc(lpos_buf, n);
+    if (kp.ncell_shift <= CNT_AT_CREATE) r |= alloc(cnt_snap, kp.ncell_shift);
     if (r) return MPCMD_ERR_ALLOC;
     d.lid = d.lid2 = d.lpos = nullptr;
     // a re-sort every ten collision periods (the cell order of a diffusing
@@ -452,6 +456,7 @@ struct Engine : EngineBase {
     CK(cudaMemsetAsync(d.dcnt, 0, 4 * (size_t)kp.ncell, st));
     CK(cudaMemsetAsync(d.dfirst, 0xFF, 16 * (size_t)kp.ncell, st));
     CK(cudaMemsetAsync(d.affected, 0, (size_t)kp.ncell, st));
+    if (cnt_snap) CK(cudaMemsetAsync(cnt_snap, 0, 4 * (size_t)kp.ncell_shift, st));
     CK(cudaMemsetAsync(d.ctr, 0, sizeof(Counters), st));
     CK(cudaMemsetAsync(d.facc, 0, sizeof(double) * 4 * std::max<int64_t>(ns, 1), st));
     CK(cudaMemsetAsync(d.fmot, 0, sizeof(double) * 4 * std::max<int64_t>(ns, 1), st));
